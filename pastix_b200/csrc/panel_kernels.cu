@@ -1,4 +1,5 @@
-// Panel factorization of the wide POTRF / LDL^T cblks of one level, in one launch.
+// Panel factorization of the wide cblks of one level, in one launch (LU in the row-block
+// form only, where the level's widest diagonal block fits in shared memory).
 //
 // PaStiX factors a cblk's diagonal block with its blocked kernel and then solves
 // the whole panel below it (cpucblk_zpotrfsp1d_panel, kernels/core_zpotrfsp.c:284-295:
@@ -10,7 +11,7 @@
 // block (block j holds the diagonal tile of step j), the others the rows below it.
 //
 // Items (j, b) with b >= j:
-//   b == j  factor the diagonal tile of step j in shared memory (8-column leaves);
+//   b == j  factor the diagonal tile of step j in registers;
 //   b >  j  solve the step's columns of row block b against that tile by
 //           substitution (x_c = (a_c - sum_{l<c} x_l L_cl) / L_cc; LDL^T: unit L,
 //           then division by D), then update the row block's columns right of the
@@ -41,12 +42,10 @@ namespace b200 {
 namespace {
 
 constexpr int PB = 64;   // tile edge
-constexpr int LP = 65;   // pitch of the diagonal tile (column-major)
 constexpr int XP = 68;   // pitch of the row block's columns (column-major, 16-byte aligned columns)
-constexpr int RP = 64;   // pitch of a resident row block (column-major)
 constexpr int PT = 256;  // threads per CTA
 constexpr long long PANEL_WAIT_CYCLES = 1000000000LL;  // about 0.5 s at the maximum SM clock
-constexpr int PANEL_SMEM_ELEMS = PB * LP + PB * XP + PB * PB + 3 * PB;
+constexpr int PANEL_SMEM_ELEMS = PB * PB + PB * XP + PB * PB + 3 * PB;
 
 __device__ __forceinline__ int ld_acquire(const int *p) {
     int v;
@@ -58,16 +57,18 @@ __device__ __forceinline__ void st_release(int *p, int v) {
     asm volatile("st.release.gpu.global.b32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
 }
 
-// Bounded wait (one thread) until *flag >= target; false on expiry or abort.
-__device__ bool panel_wait(const int *flag, int target, const int *abort_word) {
+// Bounded wait (one thread) until *flag >= target; returns the value seen, below target
+// on expiry or abort.
+__device__ int panel_wait(const int *flag, int target, const int *abort_word) {
     const long long t0 = clock64();
     for (int it = 0;; it++) {
-        if (ld_acquire(flag) >= target) return true;
+        const int v = ld_acquire(flag);
+        if (v >= target) return v;
         if ((it & 15) == 15) {
-            if (ld_acquire(abort_word)) return false;
-            if (clock64() - t0 > PANEL_WAIT_CYCLES) return false;
+            if (ld_acquire(abort_word)) return v;
+            if (clock64() - t0 > PANEL_WAIT_CYCLES) return v;
         }
-        __nanosleep(100);
+        __nanosleep(32);
     }
 }
 
@@ -82,164 +83,299 @@ __device__ __forceinline__ void load4(const T *p, T v[4]) {
     }
 }
 
-// Factor the wd x wd diagonal tile a (pitch LP, lower triangle) in place, by
-// 8-column leaves, right-looking between leaves:
-//   leaf   (warp 0): every lane factors the leaf's 8 x 8 diagonal block in registers
-//          (the same values in every lane, no broadcasts), then its two rows below
-//          it column by column; static pivoting replaces a pivot below thr in
-//          magnitude by +-thr.  The pivot's square root is p * rsqrt(p) (within an
-//          ulp of sqrt(p); rsqrt(p) scales the column).
-//   update (all warps, warp w = trailing columns j = b + 8 + w, b + 16 + w, ...):
-//          a_ij -= l_ik (d_k) l_jk for the leaf's columns k, k ascending.  Every entry
-//          receives the factored columns' terms one by one in ascending k, leaf after
-//          leaf: the same operations in the same order as a left-looking sum over all
-//          earlier columns, spread over the CTA's warps instead of one chain per column.
-// LDL^T keeps D on the diagonal and unit L below.  Called by all PT threads.
-template <typename T, int FACTO, int LP>
-__device__ void factor_tile64(T *a, int wd, double thr, int *s_piv, int *s_err) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
-    for (int b = 0; b < wd; b += 8) {
-        const int bw = min(8, wd - b);
-        if (warp == 0) {
-            T g[36];  // the leaf's diagonal block, lower part: g[r (r + 1) / 2 + c]
-#pragma unroll
-            for (int r = 0; r < 8; r++)
-#pragma unroll
-                for (int c = 0; c <= r; c++) g[r * (r + 1) / 2 + c] = (r < bw) ? a[(b + r) + (b + c) * LP] : (T)0;
-            T dv[8], iv[8];
-            int piv = 0, neg = 0;
-#pragma unroll
-            for (int c = 0; c < 8; c++) {
-                dv[c] = (T)1;
-                iv[c] = (T)1;
-                if (c < bw) {
-                    T p = g[c * (c + 1) / 2 + c];
-                    const bool rep = fabs(p) < (T)thr;
-                    if (rep) p = (FACTO == FACTO_POTRF) ? (T)thr : ((p < (T)0) ? (T)(-thr) : (T)thr);
-                    T d, inv;
-                    if (FACTO == FACTO_POTRF) {
-                        if (p < (T)0) { neg = 1; p = -p; }
-                        inv = rsqrt(p);
-                        d = p * inv;
-                    } else {
-                        d = p;
-                        inv = (T)1 / p;
-                    }
-                    piv += rep;
-                    dv[c] = d;
-                    iv[c] = inv;
-                    g[c * (c + 1) / 2 + c] = d;
-#pragma unroll
-                    for (int r = c + 1; r < 8; r++) g[r * (r + 1) / 2 + c] *= inv;
-#pragma unroll
-                    for (int j = c + 1; j < 8; j++) {
-                        const T ljc = g[j * (j + 1) / 2 + c];
-#pragma unroll
-                        for (int r = j; r < 8; r++) {
-                            const T lrc = g[r * (r + 1) / 2 + c];
-                            if (FACTO == FACTO_SYTRF) g[r * (r + 1) / 2 + j] += (-d * lrc) * ljc;
-                            else g[r * (r + 1) / 2 + j] -= lrc * ljc;
-                        }
-                    }
-                }
-            }
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int i = b + lane + 32 * h;
-                if (i < wd && i >= b + 8) {
-                    T r[8];
-#pragma unroll
-                    for (int j = 0; j < 8; j++) r[j] = (j < bw) ? a[i + (b + j) * LP] : (T)0;
-#pragma unroll
-                    for (int c = 0; c < 8; c++) {
-                        if (c < bw) {
-                            r[c] *= iv[c];
-                            const T m = (FACTO == FACTO_SYTRF) ? -dv[c] * r[c] : r[c];
-#pragma unroll
-                            for (int j = c + 1; j < 8; j++) {
-                                if (j < bw) {
-                                    if (FACTO == FACTO_SYTRF) r[j] += m * g[j * (j + 1) / 2 + c];
-                                    else r[j] -= m * g[j * (j + 1) / 2 + c];
-                                }
-                            }
-                        }
-                    }
-#pragma unroll
-                    for (int j = 0; j < 8; j++)
-                        if (j < bw) a[i + (b + j) * LP] = r[j];
-                }
-            }
-            if (lane < bw) {
-#pragma unroll
-                for (int r = 0; r < 8; r++)
-#pragma unroll
-                    for (int c = 0; c <= r; c++)
-                        if (r == lane) a[(b + r) + (b + c) * LP] = g[r * (r + 1) / 2 + c];
-            }
-            if (lane == 0) {
-                *s_piv += piv;
-                if (neg) *s_err = 1;
-            }
-        }
-        __syncthreads();
-        if (b + 8 < wd) {
-            // rank-bw update of the trailing lower triangle with the leaf's columns
-            T dk[8];
-#pragma unroll
-            for (int c = 0; c < 8; c++) dk[c] = (FACTO == FACTO_SYTRF && c < bw) ? a[(b + c) * (LP + 1)] : (T)1;
-            for (int j = b + 8 + warp; j < wd; j += nwarp) {
-                T ljk[8];
-#pragma unroll
-                for (int c = 0; c < 8; c++) ljk[c] = (c < bw) ? a[j + (b + c) * LP] : (T)0;
-                for (int i = j + lane; i < wd; i += 32) {
-                    T acc = a[i + j * LP];
-#pragma unroll
-                    for (int c = 0; c < 8; c++) {
-                        if (c < bw) {
-                            const T lik = a[i + (b + c) * LP];
-                            if (FACTO == FACTO_SYTRF) acc -= (lik * dk[c]) * ljk[c];
-                            else acc -= lik * ljk[c];
-                        }
-                    }
-                    a[i + j * LP] = acc;
-                }
-            }
-            __syncthreads();
-        }
+template <typename T>
+__device__ __forceinline__ void store4(T *p, T a, T b, T c, T d) {
+    if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<float4 *>(p) = make_float4(a, b, c, d);
+    } else {
+        *reinterpret_cast<double2 *>(p) = make_double2(a, b);
+        *reinterpret_cast<double2 *>(p + 2) = make_double2(c, d);
     }
 }
 
-// Substitution of one row (thread r < 64) of xs (pitch XP) against the unit lower
-// tile lt (pitch LP, identity past the step's width), in 16-column blocks: the
-// block's right-hand sides minus the solved columns to its left, then the
-// triangle inside the block in registers; POTRF scales by rdiag = 1 / L_cc, LDL^T
-// divides by D afterwards (dinv = 1 / D).
-template <typename T, int FACTO, int XP>
-__device__ void trsm_row64(T *xs, const T *lt, const T *rdiag, const T *dinv, int r) {
-    T *xr = xs + r;
+// Factorization of the wd x wd diagonal tile held in the registers of the CTA's 16 x 16
+// threads: thread (tx, ty) has rows 4 tx .. 4 tx + 3 and columns 4 ty .. 4 ty + 3, acc[i][q]
+// (identity past wd).  Step p: the threads of block column p (LU: also of block row p) put
+// their 4 columns (rows) in the strip, and after one barrier every thread factors the 4 x 4
+// diagonal block and solves the strips of its own rows and columns itself, so that a step
+// costs one barrier, one shared-memory round trip and four dependent pivots instead of a
+// one-warp column chain: a 64 x 64 FP32 tile took about 29 K cycles with 8-column leaves.
+// Static pivoting replaces a pivot below thr in magnitude by +-thr.  LDL^T keeps D on the
+// diagonal and unit L below; LU keeps unit L below and U on and above the diagonal.
+//
+// POTRF: the blocks above the diagonal (tx < ty), idle otherwise, carry the inverse W of
+// the tile: they hold W[ty, tx]^T, start from zero and take the same step (their strip is
+// their own raw block, the identity in step tx), and wdiag is the diagonal block of W.
+// strip: 2 x 4 x 64 elements (LU: 2 x 8 x 64).
+template <typename T, int FACTO>
+__device__ void factor_tile_regs(T (&acc)[4][4], T (&wdiag)[4][4], int wd, T *strip, double thr, int *s_piv,
+                                 int *s_err) {
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    constexpr int SB = (FACTO == FACTO_GETRF ? 8 : 4) * PB;
+    int piv = 0, neg = 0;
 #pragma unroll 1
-    for (int cb = 0; cb < PB; cb += 16) {
-        T acc[16];
+    for (int p = 0; 4 * p < wd; p++) {
+        T *cb = strip + (p & 1) * SB, *rb = cb + 4 * PB;  // column strip [k][row], LU row strip [k][column]
+        if (ty == p) {
 #pragma unroll
-        for (int q = 0; q < 16; q++) acc[q] = xr[(cb + q) * XP];
-        for (int l = 0; l < cb; l++) {
-            const T xl = xr[l * XP];
-            const T *lc = lt + cb + l * LP;
-#pragma unroll
-            for (int q = 0; q < 16; q++) acc[q] -= xl * lc[q];
+            for (int q = 0; q < 4; q++) store4(cb + q * PB + 4 * tx, acc[0][q], acc[1][q], acc[2][q], acc[3][q]);
         }
+        if (FACTO == FACTO_GETRF && tx == p && ty > p) {
 #pragma unroll
-        for (int q = 0; q < 16; q++) {
-#pragma unroll
-            for (int p2 = 0; p2 < q; p2++) acc[q] -= acc[p2] * lt[(cb + q) + (cb + p2) * LP];
-            acc[q] *= rdiag[cb + q];
+            for (int i = 0; i < 4; i++) store4(rb + i * PB + 4 * ty, acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
         }
+        __syncthreads();
+        if (ty < p) continue;
+        T g[4][4], P[4][4], Q[4][4];  // diagonal block g[row][col]; strips [row or column][k]
 #pragma unroll
-        for (int q = 0; q < 16; q++) xr[(cb + q) * XP] = acc[q];
+        for (int k = 0; k < 4; k++) {
+            T v[4];
+            load4(cb + k * PB + 4 * p, v);
+#pragma unroll
+            for (int i = 0; i < 4; i++) g[i][k] = v[i];
+            load4(cb + k * PB + 4 * tx, v);
+#pragma unroll
+            for (int i = 0; i < 4; i++) P[i][k] = v[i];
+            load4((FACTO == FACTO_GETRF ? rb : cb) + k * PB + 4 * ty, v);
+#pragma unroll
+            for (int i = 0; i < 4; i++) Q[i][k] = v[i];
+        }
+        if (FACTO == FACTO_POTRF && tx == p) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int k = 0; k < 4; k++) P[i][k] = (i == k) ? (T)1 : (T)0;
+        }
+        T d[4], iv[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            T a = g[c][c];
+            const bool rep = fabs(a) < (T)thr;
+            if (rep) a = (FACTO == FACTO_POTRF) ? (T)thr : ((a < (T)0) ? (T)(-thr) : (T)thr);
+            if (4 * p + c < wd) piv += rep;
+            if (FACTO == FACTO_POTRF) {
+                if (a < (T)0) {
+                    if (4 * p + c < wd) neg = 1;
+                    a = -a;
+                }
+                iv[c] = rsqrt(a);
+                d[c] = a * iv[c];
+            } else {
+                iv[c] = (T)1 / a;
+                d[c] = a;
+            }
+            g[c][c] = d[c];
+#pragma unroll
+            for (int i = c + 1; i < 4; i++) g[i][c] *= iv[c];
+#pragma unroll
+            for (int j = c + 1; j < 4; j++)
+#pragma unroll
+                for (int i = (FACTO == FACTO_GETRF ? c + 1 : j); i < 4; i++) {
+                    if (FACTO == FACTO_GETRF) g[i][j] -= g[i][c] * g[c][j];
+                    else if (FACTO == FACTO_SYTRF) g[i][j] -= (g[i][c] * d[c]) * g[j][c];
+                    else g[i][j] -= g[i][c] * g[j][c];
+                }
+            // the strips' column c, and its terms in the columns after it
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                P[i][c] *= iv[c];
+                if (FACTO != FACTO_GETRF) Q[i][c] *= iv[c];
+#pragma unroll
+                for (int j = c + 1; j < 4; j++) {
+                    if (FACTO == FACTO_GETRF) {
+                        P[i][j] -= P[i][c] * g[c][j];
+                        Q[i][j] -= Q[i][c] * g[j][c];
+                    } else if (FACTO == FACTO_SYTRF) {
+                        P[i][j] -= (P[i][c] * d[c]) * g[j][c];
+                        Q[i][j] -= (Q[i][c] * d[c]) * g[j][c];
+                    } else {
+                        P[i][j] -= P[i][c] * g[j][c];
+                        Q[i][j] -= Q[i][c] * g[j][c];
+                    }
+                }
+            }
+        }
+        if (ty == p) {
+            // final values of block column p (LU: the blocks below the diagonal)
+            if (tx == p) {
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        acc[i][k] = g[i][k];
+                        if (FACTO == FACTO_POTRF) wdiag[i][k] = P[i][k];
+                    }
+            } else if (tx > p || FACTO == FACTO_POTRF) {
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int k = 0; k < 4; k++) acc[i][k] = P[i][k];
+            }
+        } else if (FACTO == FACTO_GETRF && tx == p) {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[k][j] = Q[j][k];
+        } else if (FACTO == FACTO_GETRF ? tx > p : (tx >= ty || (FACTO == FACTO_POTRF && tx <= p))) {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const T m = (FACTO == FACTO_SYTRF) ? P[i][k] * d[k] : P[i][k];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[i][j] -= m * Q[j][k];
+                }
+        }
     }
-    if (FACTO == FACTO_SYTRF) {
-        for (int c = 0; c < PB; c++) xr[c * XP] *= dinv[c];
+    if (tid == PT - 1) {  // active in every step
+        *s_piv += piv;
+        if (neg) *s_err = 1;
     }
+}
+
+// Rows of a tile loaded for factor_tile_regs: a(i, j) for i, j < wd (the lower triangle,
+// LU both), identity past wd and zero above the diagonal.
+template <typename T, int FACTO, typename Load>
+__device__ __forceinline__ void load_tile_regs(T (&acc)[4][4], int wd, Load a) {
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = 4 * tx + i, c = 4 * ty + q;
+            const bool in = r < wd && c < wd && (FACTO == FACTO_GETRF || r >= c);
+            acc[i][q] = in ? a(r, c) : (r == c ? (T)1 : (T)0);
+        }
+}
+
+// Solve of the R rows of xs (64 columns, pitch XP) against the lower triangular tile lt
+// (lt[c + l * 64], l < c; identity past the step's width) by substitution in 4-column
+// blocks over the CTA's threads, thread (tx, ty) rows MR tx .. and columns 4 ty ..: the
+// columns of block p, once final in the left blocks' terms, go through the strip (inside
+// xs, whose values are in registers) and every thread solves its own rows of them against
+// the 4 x 4 diagonal block.  x_c = (a_c - sum_{l<c} x_l t_cl) * rdiag[c]; LDL^T then
+// multiplies by dinv[c] = 1 / D_c.  All PT threads; xs final after the closing barrier.
+template <typename T, int FACTO, int R, int XP>
+__device__ void trsm_tile(T *xs, const T *lt, const T *rdiag, const T *dinv) {
+    constexpr int MR = R / 16;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    T acc[MR][4];
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+        for (int h = 0; h < MR / 4; h++) {
+            T v[4];
+            load4(xs + MR * tx + 4 * h + (4 * ty + q) * XP, v);
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[4 * h + i][q] = v[i];
+        }
+    __syncthreads();
+#pragma unroll 1
+    for (int p = 0; p < 16; p++) {
+        T *st = xs + (p & 1) * 4 * R;
+        if (ty == p) {
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+#pragma unroll
+                for (int h = 0; h < MR / 4; h++)
+                    store4(st + q * R + MR * tx + 4 * h, acc[4 * h][q], acc[4 * h + 1][q], acc[4 * h + 2][q],
+                           acc[4 * h + 3][q]);
+        }
+        T t[4][4], g[4][4], rd[4];  // own columns' rows of the tile [j][k]; the diagonal block [j][k], j > k
+        if (ty >= p) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                T v[4];
+                load4(lt + 4 * p + (4 * p + k) * PB, v);
+#pragma unroll
+                for (int j = 0; j < 4; j++) g[j][k] = v[j];
+                load4(lt + 4 * ty + (4 * p + k) * PB, v);
+#pragma unroll
+                for (int j = 0; j < 4; j++) t[j][k] = v[j];
+            }
+            load4(rdiag + 4 * p, rd);
+        }
+        __syncthreads();
+        if (ty < p) continue;
+#pragma unroll
+        for (int h = 0; h < MR / 4; h++) {
+            T x[4][4];  // [row][k]
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                T v[4];
+                load4(st + k * R + MR * tx + 4 * h, v);
+#pragma unroll
+                for (int i = 0; i < 4; i++) x[i][k] = v[i];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    x[i][k] *= rd[k];
+#pragma unroll
+                    for (int j = k + 1; j < 4; j++) x[i][j] -= x[i][k] * g[j][k];
+                }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    if (ty == p) {
+                        acc[4 * h + i][j] = x[i][j];
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 4; k++) acc[4 * h + i][j] -= x[i][k] * t[j][k];
+                    }
+                }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const T m = (FACTO == FACTO_SYTRF) ? dinv[4 * ty + q] : (T)1;
+#pragma unroll
+        for (int h = 0; h < MR / 4; h++) {
+            if (FACTO == FACTO_SYTRF)
+                store4(xs + MR * tx + 4 * h + (4 * ty + q) * XP, acc[4 * h][q] * m, acc[4 * h + 1][q] * m,
+                       acc[4 * h + 2][q] * m, acc[4 * h + 3][q] * m);
+            else
+                store4(xs + MR * tx + 4 * h + (4 * ty + q) * XP, acc[4 * h][q], acc[4 * h + 1][q], acc[4 * h + 2][q],
+                       acc[4 * h + 3][q]);
+        }
+    }
+    __syncthreads();
+}
+
+// The same solve as the product with the tile's inverse, bs[l * 64 + c] = W[c, l] (POTRF
+// row blocks): no dependent chain, 64 x 64 / 2 multiply-adds per row.
+template <typename T, int R>
+__device__ void trsm_inverse(T *xs, const T *bs) {
+    constexpr int MR = R / 16;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    T acc[MR][4];
+#pragma unroll
+    for (int i = 0; i < MR; i++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[i][q] = 0;
+    const int lend = 4 * ((ty | 1) + 1);  // W[c, l] = 0 for l > c
+#pragma unroll 8
+    for (int l = 0; l < lend; l++) {
+        T av[MR], bv[4];
+#pragma unroll
+        for (int h = 0; h < MR / 4; h++) load4(xs + l * R + MR * tx + 4 * h, av + 4 * h);
+        load4(bs + l * PB + 4 * ty, bv);
+#pragma unroll
+        for (int i = 0; i < MR; i++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) acc[i][q] += av[i] * bv[q];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+        for (int h = 0; h < MR / 4; h++)
+            store4(xs + MR * tx + 4 * h + (4 * ty + q) * R, acc[4 * h][q], acc[4 * h + 1][q], acc[4 * h + 2][q],
+                   acc[4 * h + 3][q]);
+    __syncthreads();
 }
 
 template <typename T, int FACTO>
@@ -249,8 +385,8 @@ __global__ void __launch_bounds__(PT, sizeof(T) == 4 ? 2 : 1) panel_kernel(DevSy
                                                    const double *__restrict__ thr_ptr, unsigned long long *npiv,
                                                    int *err) {
     extern __shared__ __align__(16) unsigned char pn_smem[];
-    T *lt = reinterpret_cast<T *>(pn_smem);  // diagonal tile of the step (pitch LP)
-    T *xs = lt + PB * LP;                    // the row block's columns of the step (pitch XP)
+    T *lt = reinterpret_cast<T *>(pn_smem);  // diagonal tile of the step
+    T *xs = lt + PB * PB;                    // the row block's columns of the step (pitch XP)
     T *bs = xs + PB * XP;                    // update operand L[c, j] (D_j): bs[l * PB + row]
     T *rdiag = bs + PB * PB, *dinv = rdiag + PB, *dd = dinv + PB;
     __shared__ int s_item, s_ok, s_piv, s_err;
@@ -276,8 +412,8 @@ __global__ void __launch_bounds__(PT, sizeof(T) == 4 ? 2 : 1) panel_kernel(DevSy
         int *sol = solved + pc.flag0, *upd = updated + pc.flag0;
         if (tid == 0) {
             // the row block's update of the previous step, and the factored tile of this step
-            if (j > 0 && !panel_wait(upd + b, j, abort_word)) s_ok = 0;
-            if (s_ok && b != j && !panel_wait(sol + j, j + 1, abort_word)) s_ok = 0;
+            if (j > 0 && panel_wait(upd + b, j, abort_word) < j) s_ok = 0;
+            if (s_ok && b != j && panel_wait(sol + j, j + 1, abort_word) < j + 1) s_ok = 0;
         }
         __syncthreads();
         if (!s_ok) {
@@ -287,21 +423,16 @@ __global__ void __launch_bounds__(PT, sizeof(T) == 4 ? 2 : 1) panel_kernel(DevSy
         if (b == j) {
             // ---------------------------------------------- diagonal tile
             T *A = P + c0 + (size_t)c0 * ld;
-            stage_n<PB * PB / PT, T>(
-                [&](int u) {
-                    const int idx = tid + PT * u, i = idx & 63, jj = idx >> 6;
-                    return (i < wd && jj < wd && i >= jj) ? __ldcg(A + i + (size_t)jj * ld) : (T)0;
-                },
-                [&](int u, T v) {
-                    const int idx = tid + PT * u;
-                    lt[(idx & 63) + (idx >> 6) * LP] = v;
-                });
-            __syncthreads();
-            factor_tile64<T, FACTO, LP>(lt, wd, thr, &s_piv, &s_err);
-            for (int idx = tid; idx < PB * PB; idx += PT) {
-                const int i = idx & 63, jj = idx >> 6;
-                if (i < wd && jj < wd && i >= jj) A[i + (size_t)jj * ld] = lt[i + jj * LP];
-            }
+            T acc[4][4], wdiag[4][4];
+            load_tile_regs<T, FACTO>(acc, wd, [&](int r, int c) { return __ldcg(A + r + (size_t)c * ld); });
+            factor_tile_regs<T, FACTO>(acc, wdiag, wd, lt, thr, &s_piv, &s_err);
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int r = 4 * (tid & 15) + i, c = 4 * (tid >> 4) + q;
+                    if (r < wd && c < wd && r >= c) A[r + (size_t)c * ld] = acc[i][q];
+                }
             __syncthreads();
             if (tid == 0) {
                 if (s_piv) atomicAdd(cblk_pivot_counter(s, npiv, k), (unsigned long long)s_piv);
@@ -329,7 +460,7 @@ __global__ void __launch_bounds__(PT, sizeof(T) == 4 ? 2 : 1) panel_kernel(DevSy
             },
             [&](int u, T v) {
                 const int idx = tid + PT * u;
-                lt[(idx & 63) + (idx >> 6) * LP] = v;
+                lt[idx] = v;
             });
         stage_n<PB * PB / PT, T>(
             [&](int u) {
@@ -347,8 +478,7 @@ __global__ void __launch_bounds__(PT, sizeof(T) == 4 ? 2 : 1) panel_kernel(DevSy
             dd[tid] = (FACTO == FACTO_SYTRF) ? dgv : (T)1;
         }
         __syncthreads();
-        if (tid < PB) trsm_row64<T, FACTO, XP>(xs, lt, rdiag, dinv, tid);
-        __syncthreads();
+        trsm_tile<T, FACTO, PB, XP>(xs, lt, rdiag, dinv);
         for (int idx = tid; idx < PB * wd; idx += PT) {
             const int r = idx & 63, c = idx >> 6;
             if (r < nr) X[r + (size_t)c * ld] = xs[r + c * XP];
@@ -362,7 +492,7 @@ __global__ void __launch_bounds__(PT, sizeof(T) == 4 ? 2 : 1) panel_kernel(DevSy
         const int cmax = drows ? b : pc.ns - 1;
         const int tx = tid & 15, ty = tid >> 4;
         for (int c = j + 1; c <= cmax; c++) {
-            if (tid == 0 && c != b && !panel_wait(sol + c, j + 1, abort_word)) s_ok = 0;
+            if (tid == 0 && c != b && panel_wait(sol + c, j + 1, abort_word) < j + 1) s_ok = 0;
             __syncthreads();
             if (!s_ok) break;
             const int wc = min(PB, W - PB * c);
@@ -431,23 +561,60 @@ __global__ void __launch_bounds__(PT, sizeof(T) == 4 ? 2 : 1) panel_kernel(DevSy
 // steps for the rows below the diagonal block) -- and, for b < ns, finally
 // factors its diagonal tile (b, b).  Each solved step of the diagonal block's
 // rows is written back and announced at once (solved[b] = j + 1; b + 1 after the
-// factorization), the only cross-item reads being the factored tiles L[j, j] and
-// the diagonal block's solved tiles L[c, j].  Row blocks: 64 rows in the diagonal
-// block, R rows (64 or 128) below it.  Items: the diagonal blocks' row blocks of
-// every cblk first (b ascending), then the rows below.
+// factorization), the only cross-item reads being the factored tiles L[j, j] (POTRF:
+// their inverses) and the diagonal block's solved tiles L[c, j].  Row blocks: 64 rows in
+// the diagonal block, R rows (64 or 128) below it.  Items: the diagonal blocks' row
+// blocks of every cblk first (b ascending), then the rows below.
+//
+// LU (core_zgetrfsp / core_ztrsmsp, kernels/core_zgetrfsp.c:64-170, without row
+// exchanges) is the same dataflow over two panels, L and V = U^T: a row block of side 0
+// holds rows of L and is updated by L[b, c] -= L[b, j] V[c, j]^T, one of side 1 holds rows
+// of V and is updated by V[b, c] -= V[b, j] L[c, j]^T; side 0 solves against V[j, j]
+// (the stored U^T) and owns the diagonal tiles, side 1 against the unit L[j, j].
+// solved counts side 0, solved_v side 1, whose item of a row block comes first.  The
+// one-CTA diagonal blocks and row-by-row solves this replaces took 56 of the 66 ms of a
+// 64^3 convection-diffusion LU in FP32; the panel launches take 9.3 ms.
+struct RowsCtx {
+    int *sol, *sol_v;     // counters of the cblk's row blocks
+    const int *abort_word;
+    int *known;           // shared: the counters' last values seen, [2][16]
+    int *s_ok, *s_piv, *s_err;
+    double thr;
+};
+
+// Wait until counter c of the given side has reached target, all threads; counters
+// already seen that far cost one shared-memory read.
+__device__ __forceinline__ bool rows_need(const RowsCtx &x, int side, int c, int target) {
+    if (x.known[16 * side + c] < target) {  // the same value in every thread
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const int v = panel_wait((side ? x.sol_v : x.sol) + c, target, x.abort_word);
+            if (v < target) *x.s_ok = 0;
+            x.known[16 * side + c] = v;
+        }
+        __syncthreads();
+    }
+    return *x.s_ok;
+}
+
 template <typename T, int FACTO, int R>
-__device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, T *L, T *lt, T *rdiag, T *dinv, T *dd, T *xs,
-                          int *sol, const int *abort_word, double thr, int *s_ok, int *s_piv, int *s_err) {
+__device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, int side, T *L, T *U, T *Wk, T *lt, T *rdiag,
+                          T *dinv, T *dd, T *xs, const RowsCtx &x) {
     constexpr int MR = R / 16;  // rows of a thread's update tile
+    constexpr bool LU = FACTO == FACTO_GETRF;
     const int tid = threadIdx.x;
     const int k = pc.k, W = s.ncols[k], S = s.stride[k], ld = s.ld[k];
-    T *P = L + s.off[k];
+    T *P = (LU && side ? U : L) + s.off[k];        // this side's panel
+    T *Q = LU ? (side ? L : U) + s.off[k] : P;     // the panel its updates multiply with
+    int *sol = side ? x.sol_v : x.sol;
+    const int qside = LU ? 1 - side : 0;           // counters of Q
     const bool drows = b < pc.ns;
     const int r0 = drows ? PB * b : W + R * (b - pc.ns);
     const int nr = min(R, (drows ? W : S) - r0);
-    const int ncol = drows ? min(W, PB * (b + 1)) : W;  // columns held (lower part for the diagonal block)
+    // columns held (lower part for the diagonal block; V: left of its diagonal tile)
+    const int ncol = drows ? (side ? PB * b : min(W, PB * (b + 1))) : W;
     const int nstep = drows ? b : pc.ns;                 // steps solved in this row block
-    // the row block: rows past nr, the diagonal tile's upper triangle and (below
+    // the row block: rows past nr, the diagonal tile's upper triangle (not LU) and (below
     // the diagonal block) the last step's columns past W as zeros
     const int nzero = drows ? ncol : PB * pc.ns;
     constexpr int CG = PT / R;  // column groups of a load pass
@@ -455,7 +622,7 @@ __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, T *L, T *
         stage_n<4, T>(
             [&](int u) {
                 const int r = tid % R, c = c0s + tid / R + CG * u;
-                const bool keep = r < nr && c < ncol && (!drows || c < PB * b || r >= c - PB * b);
+                const bool keep = r < nr && c < ncol && (LU || !drows || c < PB * b || r >= c - PB * b);
                 return keep ? __ldcg(P + r0 + r + (size_t)c * ld) : (T)0;
             },
             [&](int u, T v) {
@@ -463,79 +630,112 @@ __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, T *L, T *
                 if (c < nzero) xs[r + c * R] = v;
             });
     }
+    if (LU && drows) {
+        // the diagonal block is the sum of L's and the transposed U's (core_zgeadd): 8 rows x
+        // 4 columns of it per warp access
+        const int cfirst = side ? 0 : PB * b, nc = ncol - cfirst;
+        __syncthreads();
+        for (int t = tid >> 5; t < (PB / 8) * ((nc + 3) / 4); t += PT / 32) {
+            const int r = 8 * (t % (PB / 8)) + (tid & 7), c = cfirst + 4 * (t / (PB / 8)) + ((tid & 31) >> 3);
+            if (r < nr && c < ncol) xs[r + c * R] += __ldcg(Q + c + (size_t)(r0 + r) * ld);
+        }
+    }
     __syncthreads();
     const int tx = tid & 15, ty = tid >> 4;
-    for (int j = 0; j < nstep && *s_ok; j++) {
+    T pf[PB * PB / PT];  // tile read ahead: the next update operand, or the next step's diagonal tile
+    auto load_diag = [&](int j) {
         const int c0 = PB * j, wd = min(PB, W - c0);
-        if (tid == 0 && !panel_wait(sol + j, j + 1, abort_word)) *s_ok = 0;
-        __syncthreads();
-        if (!*s_ok) break;
+        // POTRF: the inverse's column l; else the tile the rows are solved against, unit
+        // where it is not scaled by rdiag
+        const T *Dg = FACTO == FACTO_POTRF ? Wk + c0 + (size_t)c0 * W : Q + c0 + (size_t)c0 * ld;
+        const int dl = FACTO == FACTO_POTRF ? W : ld;
+#pragma unroll
+        for (int u = 0; u < PB * PB / PT; u++) {
+            const int idx = tid + PT * u, c = idx & 63, l = idx >> 6;
+            if (FACTO == FACTO_POTRF) pf[u] = (c < wd && l <= c) ? __ldcg(Dg + c + (size_t)l * dl) : (T)0;
+            else pf[u] = (c < wd && l < c) ? __ldcg(Dg + c + (size_t)l * dl) : (c == l ? (T)1 : (T)0);
+        }
+    };
+    auto load_b = [&](int j, int c) {
+        const int wd = min(PB, W - PB * j), wc = min(PB, W - PB * c);
+        const T *B = Q + PB * c + (size_t)(PB * j) * ld;
+#pragma unroll
+        for (int u = 0; u < PB * PB / PT; u++) {
+            const int idx = tid + PT * u, rr = idx & 63, l = idx >> 6;
+            pf[u] = (rr < wc && l < wd) ? __ldcg(B + rr + (size_t)l * ld) : (T)0;
+        }
+    };
+    bool have = false;  // pf holds the tile read next
+    for (int j = 0; j < nstep; j++) {
+        const int c0 = PB * j, wd = min(PB, W - c0);
+        if (!have) {
+            if (!rows_need(x, 0, j, j + 1)) return;
+            load_diag(j);
+        }
+        have = false;
         // ---------------------------------------------- solve of step j's columns
-        const T *Dg = P + c0 + (size_t)c0 * ld;
-        stage_n<PB * PB / PT, T>(
-            [&](int u) {
-                const int idx = tid + PT * u, c = idx & 63, l = idx >> 6;
-                T v = 0;
-                if (c < wd && l < wd) v = (c > l) ? __ldcg(Dg + c + (size_t)l * ld) : (c == l ? (T)1 : (T)0);
-                else if (c == l) v = 1;
-                return v;
-            },
-            [&](int u, T v) {
-                const int idx = tid + PT * u;
-                lt[(idx & 63) + (idx >> 6) * LP] = v;
-            });
-        if (tid < PB) {
-            const T dgv = tid < wd ? __ldcg(Dg + (size_t)tid * (ld + 1)) : (T)1;
-            rdiag[tid] = (FACTO == FACTO_POTRF) ? (T)1 / dgv : (T)1;
+#pragma unroll
+        for (int u = 0; u < PB * PB / PT; u++) lt[tid + PT * u] = pf[u];
+        if (FACTO != FACTO_POTRF && tid < PB) {
+            const T dgv = tid < wd ? __ldcg(Q + (c0 + tid) + (size_t)(c0 + tid) * ld) : (T)1;
+            rdiag[tid] = (LU && side == 0) ? (T)1 / dgv : (T)1;
             dinv[tid] = (FACTO == FACTO_SYTRF) ? (T)1 / dgv : (T)1;
             dd[tid] = (FACTO == FACTO_SYTRF) ? dgv : (T)1;
         }
         __syncthreads();
-        if (tid < R) trsm_row64<T, FACTO, R>(xs + c0 * R, lt, rdiag, dinv, tid);
-        __syncthreads();
+        if (FACTO == FACTO_POTRF) trsm_inverse<T, R>(xs + c0 * R, lt);
+        else trsm_tile<T, FACTO, R, R>(xs + c0 * R, lt, rdiag, dinv);
         for (int idx = tid; idx < R * wd; idx += PT) {
             const int r = idx % R, c = idx / R;
             if (r < nr) P[r0 + r + (size_t)(c0 + c) * ld] = xs[r + (c0 + c) * R];
         }
-        __syncthreads();
-        if (tid == 0 && drows) {
-            __threadfence();
-            st_release(sol + b, j + 1);
+        if (drows) {
+            __syncthreads();
+            if (tid == 0) {
+                __threadfence();
+                st_release(sol + b, j + 1);
+            }
+            if (LU)  // the other panel's diagonal block keeps the transposed factor (core_zgetmo)
+                for (int t = tid >> 5; t < (PB / 8) * ((wd + 3) / 4); t += PT / 32) {
+                    const int r = 8 * (t % (PB / 8)) + (tid & 7), c = c0 + 4 * (t / (PB / 8)) + ((tid & 31) >> 3);
+                    if (r < nr && c < c0 + wd) Q[c + (size_t)(r0 + r) * ld] = xs[r + c * R];
+                }
         }
         // ---------------------------------------------- update of the columns right of the step
-        const int cmax = drows ? b : pc.ns - 1;
+        const int cmax = drows ? (side ? b - 1 : b) : pc.ns - 1;
         for (int c = j + 1; c <= cmax; c++) {
-            if (tid == 0 && c != b && !panel_wait(sol + c, j + 1, abort_word)) *s_ok = 0;
-            __syncthreads();
-            if (!*s_ok) break;
+            const bool own = !LU && drows && c == b;  // this row block's solved columns, in shared memory
+            if (!own && !have) {
+                if (!rows_need(x, qside, c, j + 1)) return;
+                load_b(j, c);
+            }
+            have = false;
             const int wc = min(PB, W - PB * c);
             T *bs = lt;  // bs[l * PB + row]
-            if (drows && c == b) {
-                // this row block's own tile: its solved columns are in shared memory
-                for (int idx = tid; idx < PB * PB; idx += PT) {
-                    const int rr = idx & 63, l = idx >> 6;
-                    const T v = (rr < wc && l < wd) ? xs[rr + (c0 + l) * R] : (T)0;
-                    bs[idx] = (FACTO == FACTO_SYTRF) ? v * dd[l] : v;
-                }
-            } else {
-                const T *B = P + PB * c + (size_t)c0 * ld;
-                stage_n<PB * PB / PT, T>(
-                    [&](int u) {
-                        const int idx = tid + PT * u, rr = idx & 63, l = idx >> 6;
-                        return (rr < wc && l < wd) ? __ldcg(B + rr + (size_t)l * ld) : (T)0;
-                    },
-                    [&](int u, T v) {
-                        const int idx = tid + PT * u;
-                        bs[idx] = (FACTO == FACTO_SYTRF) ? v * dd[idx >> 6] : v;
-                    });
+#pragma unroll
+            for (int u = 0; u < PB * PB / PT; u++) {
+                const int idx = tid + PT * u, rr = idx & 63, l = idx >> 6;
+                const T v = own ? ((rr < wc && l < wd) ? xs[rr + (c0 + l) * R] : (T)0) : pf[u];
+                bs[idx] = (FACTO == FACTO_SYTRF) ? v * dd[l] : v;
             }
             __syncthreads();
+            // read ahead what comes next, when it is known to be there
+            if (c < cmax) {
+                if (!(!LU && drows && c + 1 == b) && x.known[16 * qside + c + 1] >= j + 1) {
+                    load_b(j, c + 1);
+                    have = true;
+                }
+            } else if (j + 1 < nstep && x.known[j + 1] >= j + 2) {
+                load_diag(j + 1);
+                have = true;
+            }
             T acc[MR][4];
 #pragma unroll
             for (int i = 0; i < MR; i++)
 #pragma unroll
                 for (int q = 0; q < 4; q++) acc[i][q] = 0;
             const T *xa = xs + c0 * R + MR * tx;
+#pragma unroll 4
             for (int l = 0; l < wd; l++) {
                 T av[MR], bv[4];
 #pragma unroll
@@ -554,26 +754,61 @@ __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, T *L, T *
 #pragma unroll
                     for (int i = 0; i < MR; i++) {
                         const int r = MR * tx + i;
-                        if (!(drows && c == b) || r >= cc) xc[r + cc * R] -= acc[i][q];
+                        if (!own || r >= cc) xc[r + cc * R] -= acc[i][q];
                     }
                 }
             }
             __syncthreads();
         }
     }
-    if (!*s_ok) return;
-    if (drows) {
+    if (drows && side == 0) {
         // ---------------------------------------------- the row block's diagonal tile
         const int c0 = PB * b, wd = min(PB, W - c0);
-        factor_tile64<T, FACTO, R>(xs + c0 * R, wd, thr, s_piv, s_err);
-        for (int idx = tid; idx < PB * PB; idx += PT) {
-            const int i = idx & 63, jj = idx >> 6;
-            if (i < wd && jj < wd && i >= jj) P[c0 + i + (size_t)(c0 + jj) * ld] = xs[i + (c0 + jj) * R];
+        T *xt = xs + c0 * R;
+        T acc[4][4], wdiag[4][4];
+        load_tile_regs<T, FACTO>(acc, wd, [&](int r, int c) { return xt[r + c * R]; });
+        __syncthreads();
+        factor_tile_regs<T, FACTO>(acc, wdiag, wd, xt, x.thr, x.s_piv, x.s_err);
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (LU || tx >= ty) {
+                store4(xt + 4 * tx + (4 * ty + q) * R, acc[0][q], acc[1][q], acc[2][q], acc[3][q]);
+            } else if (FACTO == FACTO_POTRF) {
+                // W[ty, tx] = acc^T: column 4 tx + q of W, rows 4 ty ..
+                store4(lt + 4 * ty + (4 * tx + q) * PB, acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
+            }
+            if (FACTO == FACTO_POTRF && tx == ty)
+                store4(lt + 4 * tx + (4 * tx + q) * PB, wdiag[q][0], wdiag[q][1], wdiag[q][2], wdiag[q][3]);
+        }
+        __syncthreads();
+        if (FACTO == FACTO_POTRF && b + 1 < pc.ns + (S > W ? 1 : 0)) {
+            for (int idx = tid; idx < PB * PB; idx += PT) {
+                const int c = idx & 63, l = idx >> 6;
+                if (c < wd && l <= c) Wk[(c0 + c) + (size_t)(c0 + l) * W] = lt[idx];
+            }
+        } else {
+            for (int idx = tid; idx < PB * PB; idx += PT) {
+                const int i = idx & 63, jj = idx >> 6;
+                if (i < wd && jj < wd && (LU || i >= jj)) P[c0 + i + (size_t)(c0 + jj) * ld] = xt[i + jj * R];
+            }
+            if (LU)
+                for (int t = tid >> 5; t < (PB / 8) * ((wd + 3) / 4); t += PT / 32) {
+                    const int i = 8 * (t % (PB / 8)) + (tid & 7), jj = 4 * (t / (PB / 8)) + ((tid & 31) >> 3);
+                    if (i < wd && jj < wd) Q[c0 + jj + (size_t)(c0 + i) * ld] = xt[i + jj * R];
+                }
         }
         __syncthreads();
         if (tid == 0) {
             __threadfence();
             st_release(sol + b, b + 1);
+        }
+        if (FACTO == FACTO_POTRF && b + 1 < pc.ns + (S > W ? 1 : 0)) {
+            // the factored tile itself is read by later launches only
+            for (int idx = tid; idx < PB * PB; idx += PT) {
+                const int i = idx & 63, jj = idx >> 6;
+                if (i < wd && jj < wd && i >= jj) P[c0 + i + (size_t)(c0 + jj) * ld] = xt[i + jj * R];
+            }
         }
     }
 }
@@ -581,13 +816,15 @@ __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, T *L, T *
 template <typename T, int FACTO, int RB>
 __global__ void __launch_bounds__(PT, 1)
     panel_rows_kernel(DevSym s, const PanelCblk *__restrict__ pcb, const PanelItem *__restrict__ items, int nitems,
-                      int *ticket, int *solved, int *abort_word, T *L, const double *__restrict__ thr_ptr,
+                      int *ticket, int *solved, int *solved_v, int *abort_word, T *L, T *U, T *WL,
+                      const int64_t *__restrict__ woff, const double *__restrict__ thr_ptr,
                       unsigned long long *npiv, int *err) {
     extern __shared__ __align__(16) unsigned char pn_smem[];
-    T *lt = reinterpret_cast<T *>(pn_smem);  // L[j, j] (pitch LP) for the solve; L[c, j] (D_j) for the update
-    T *rdiag = lt + PB * LP, *dinv = rdiag + PB, *dd = dinv + PB;
+    T *lt = reinterpret_cast<T *>(pn_smem);  // the solve's tile (or its inverse); the update's operand
+    T *rdiag = lt + PB * PB, *dinv = rdiag + PB, *dd = dinv + PB;
     T *xs = dd + PB;                         // the row block, column-major (pitch = its rows)
     __shared__ int s_item, s_ok, s_piv, s_err;
+    __shared__ int s_known[32];
     const int tid = threadIdx.x;
     bool aborted = false;
     for (;;) {
@@ -597,19 +834,17 @@ __global__ void __launch_bounds__(PT, 1)
             s_piv = 0;
             s_err = 0;
         }
+        if (tid < 32) s_known[tid] = 0;
         __syncthreads();
         const int t = s_item;
         if (t >= nitems) break;
         const PanelItem it = items[t];
         const PanelCblk pc = pcb[it.p];
-        int *sol = solved + pc.flag0;
-        const double thr = cblk_threshold(s, thr_ptr, pc.k);
-        if (it.b < pc.ns)
-            rows_item<T, FACTO, PB>(s, pc, it.b, L, lt, rdiag, dinv, dd, xs, sol, abort_word, thr, &s_ok, &s_piv,
-                                    &s_err);
-        else
-            rows_item<T, FACTO, RB>(s, pc, it.b, L, lt, rdiag, dinv, dd, xs, sol, abort_word, thr, &s_ok, &s_piv,
-                                    &s_err);
+        const RowsCtx x{solved + pc.flag0, solved_v + pc.flag0, abort_word, s_known, &s_ok, &s_piv, &s_err,
+                        cblk_threshold(s, thr_ptr, pc.k)};
+        T *Wk = WL + woff[pc.k];
+        if (it.b < pc.ns) rows_item<T, FACTO, PB>(s, pc, it.b, it.j, L, U, Wk, lt, rdiag, dinv, dd, xs, x);
+        else rows_item<T, FACTO, RB>(s, pc, it.b, it.j, L, U, Wk, lt, rdiag, dinv, dd, xs, x);
         __syncthreads();
         if (!s_ok) {
             aborted = true;
@@ -629,8 +864,9 @@ __global__ void __launch_bounds__(PT, 1)
 
 int g_panel_ctas = 0;  // resident CTAs of the panel kernel on the device (all SMs)
 int g_sms = 0, g_smem_optin = 0;
+constexpr int PANEL_STATIC_SMEM = 256;  // room for the kernels' static shared variables
 
-constexpr size_t rows_smem_elems(int nsmax, int rb) { return (size_t)PB * LP + 3 * PB + (size_t)rb * PB * nsmax; }
+constexpr size_t rows_smem_elems(int nsmax, int rb) { return (size_t)PB * PB + 3 * PB + (size_t)rb * PB * nsmax; }
 
 template <typename T, int FACTO>
 int panel_occupancy() {
@@ -651,14 +887,16 @@ int configure_panel_kernels() {
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
     if (cudaDeviceGetAttribute(&g_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return -1;
     g_sms = sms;
-    const int dyn = g_smem_optin - 64;  // room for the kernels' static shared variables
-    if (cudaFuncSetAttribute(panel_rows_kernel<double, FACTO_POTRF, PB>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) ||
-        cudaFuncSetAttribute(panel_rows_kernel<double, FACTO_SYTRF, PB>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) ||
-        cudaFuncSetAttribute(panel_rows_kernel<float, FACTO_POTRF, PB>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) ||
-        cudaFuncSetAttribute(panel_rows_kernel<float, FACTO_SYTRF, PB>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) ||
-        cudaFuncSetAttribute(panel_rows_kernel<float, FACTO_POTRF, 2 * PB>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) ||
-        cudaFuncSetAttribute(panel_rows_kernel<float, FACTO_SYTRF, 2 * PB>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn))
-        return -1;
+    const int dyn = g_smem_optin - PANEL_STATIC_SMEM;
+    const void *rows[] = {
+        (const void *)panel_rows_kernel<double, FACTO_POTRF, PB>, (const void *)panel_rows_kernel<double, FACTO_SYTRF, PB>,
+        (const void *)panel_rows_kernel<double, FACTO_GETRF, PB>, (const void *)panel_rows_kernel<float, FACTO_POTRF, PB>,
+        (const void *)panel_rows_kernel<float, FACTO_SYTRF, PB>, (const void *)panel_rows_kernel<float, FACTO_GETRF, PB>,
+        (const void *)panel_rows_kernel<float, FACTO_POTRF, 2 * PB>,
+        (const void *)panel_rows_kernel<float, FACTO_SYTRF, 2 * PB>,
+        (const void *)panel_rows_kernel<float, FACTO_GETRF, 2 * PB>};
+    for (const void *f : rows)
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn)) return -1;
     int occ = panel_occupancy<double, FACTO_POTRF>();
     occ = std::min(occ, panel_occupancy<double, FACTO_SYTRF>());
     occ = std::min(occ, panel_occupancy<float, FACTO_POTRF>());
@@ -684,51 +922,52 @@ void launch_panel(int facto, const DevSym &s, const PanelCblk *pcb, const PanelI
 }
 
 int panel_rows_block(int nsmax, size_t esz) {
-    const size_t lim = (size_t)g_smem_optin - 64;
+    const size_t lim = (size_t)g_smem_optin - PANEL_STATIC_SMEM;
     if (esz == 4 && rows_smem_elems(nsmax, 2 * PB) * esz <= lim) return 2 * PB;
     return rows_smem_elems(nsmax, PB) * esz <= lim ? PB : 0;
 }
 
-template <typename T, int RB>
-static void launch_rows(int facto, const DevSym &s, const PanelCblk *pcb, const PanelItem *items, int nitems,
-                        int nsmax, int *ticket, int *solved, int *abort_word, T *L, const double *thr,
-                        unsigned long long *npiv, int *err, cudaStream_t st) {
+template <typename T, int FACTO, int RB>
+static void launch_rows(const DevSym &s, const PanelCblk *pcb, const PanelItem *items, int nitems, int nsmax,
+                        int *ticket, int *solved, int *solved_v, int *abort_word, T *L, T *U, T *WL,
+                        const int64_t *woff, const double *thr, unsigned long long *npiv, int *err, cudaStream_t st) {
     const size_t smem = rows_smem_elems(nsmax, RB) * sizeof(T);
     int occ = 0;
-    if (facto == FACTO_POTRF)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, panel_rows_kernel<T, FACTO_POTRF, RB>, PT, smem);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, panel_rows_kernel<T, FACTO_SYTRF, RB>, PT, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, panel_rows_kernel<T, FACTO, RB>, PT, smem);
     const int grid = std::min(nitems, std::max(occ, 1) * g_sms);
-    if (facto == FACTO_POTRF)
-        panel_rows_kernel<T, FACTO_POTRF, RB><<<grid, PT, smem, st>>>(s, pcb, items, nitems, ticket, solved,
-                                                                     abort_word, L, thr, npiv, err);
-    else
-        panel_rows_kernel<T, FACTO_SYTRF, RB><<<grid, PT, smem, st>>>(s, pcb, items, nitems, ticket, solved,
-                                                                     abort_word, L, thr, npiv, err);
+    panel_rows_kernel<T, FACTO, RB><<<grid, PT, smem, st>>>(s, pcb, items, nitems, ticket, solved, solved_v, abort_word,
+                                                           L, U, WL, woff, thr, npiv, err);
 }
 
 template <typename T>
 void launch_panel_rows(int facto, const DevSym &s, const PanelCblk *pcb, const PanelItem *items, int nitems,
-                       int nsmax, int rb, int *ticket, int *solved, int *abort_word, T *L, const double *thr,
-                       unsigned long long *npiv, int *err, cudaStream_t st) {
+                       int nsmax, int rb, int *ticket, int *solved, int *solved_v, int *abort_word, T *L, T *U, T *WL,
+                       const int64_t *woff, const double *thr, unsigned long long *npiv, int *err, cudaStream_t st) {
     if (nitems <= 0) return;
+    auto run = [&](auto f, auto r) {
+        launch_rows<T, decltype(f)::value, decltype(r)::value>(s, pcb, items, nitems, nsmax, ticket, solved, solved_v,
+                                                               abort_word, L, U, WL, woff, thr, npiv, err, st);
+    };
+    auto by_facto = [&](auto r) {
+        if (facto == FACTO_POTRF) run(std::integral_constant<int, FACTO_POTRF>{}, r);
+        else if (facto == FACTO_SYTRF) run(std::integral_constant<int, FACTO_SYTRF>{}, r);
+        else run(std::integral_constant<int, FACTO_GETRF>{}, r);
+    };
     if constexpr (sizeof(T) == 4) {
         if (rb == 2 * PB) {
-            launch_rows<T, 2 * PB>(facto, s, pcb, items, nitems, nsmax, ticket, solved, abort_word, L, thr, npiv, err,
-                                   st);
+            by_facto(std::integral_constant<int, 2 * PB>{});
             return;
         }
     }
-    launch_rows<T, PB>(facto, s, pcb, items, nitems, nsmax, ticket, solved, abort_word, L, thr, npiv, err, st);
+    by_facto(std::integral_constant<int, PB>{});
 }
 
 template void launch_panel_rows<double>(int, const DevSym &, const PanelCblk *, const PanelItem *, int, int, int, int *,
-                                        int *, int *, double *, const double *, unsigned long long *, int *,
-                                        cudaStream_t);
+                                        int *, int *, int *, double *, double *, double *, const int64_t *,
+                                        const double *, unsigned long long *, int *, cudaStream_t);
 template void launch_panel_rows<float>(int, const DevSym &, const PanelCblk *, const PanelItem *, int, int, int, int *,
-                                       int *, int *, float *, const double *, unsigned long long *, int *,
-                                       cudaStream_t);
+                                       int *, int *, int *, float *, float *, float *, const int64_t *,
+                                       const double *, unsigned long long *, int *, cudaStream_t);
 
 template void launch_panel<double>(int, const DevSym &, const PanelCblk *, const PanelItem *, int, int *, int *, int *,
                                    int *, double *, const double *, unsigned long long *, int *, cudaStream_t);

@@ -394,8 +394,13 @@ int build_schedule(b200_solver_t *s) {
     s->lvl_pi1.assign(nlev, 0);
     s->lvl_prows.assign(nlev, 0);
     s->lvl_pns.assign(nlev, 0);
-    const int split_min = 96;  // wider POTRF / LDL^T cblks take the sub-panel path
-    auto is_big = [&](int k) { return s->facto != FACTO_GETRF && s->ncols[k] > split_min; };
+    // wider cblks take the panel launch (LU only in its row-block form, while that fits)
+    const int split_min = 96;
+    auto is_big = [&](int k) {
+        if (s->ncols[k] <= split_min) return false;
+        return s->facto != FACTO_GETRF ||
+               (!s->panel_steps_only && panel_rows_block((s->ncols[k] + 63) / 64, s->esz) > 0);
+    };
     s->lvl_st0.assign(nlev, 0);
     s->lvl_st1.assign(nlev, 0);
     s->lvl_dt0.assign(nlev, 0);
@@ -491,21 +496,24 @@ int build_schedule(b200_solver_t *s) {
                 nrbmax = std::max(nrbmax, pc.nrb);
                 // diagonal factorization, panel solve and the updates inside the panel
                 const double nc = s->ncols[k], m = s->stride[k] - s->ncols[k];
-                s->flops_kind[4] += nc * nc * nc / 3.0 + m * nc * nc;
+                s->flops_kind[4] += (s->facto == FACTO_GETRF ? 2.0 : 1.0) * (nc * nc * nc / 3.0 + m * nc * nc);
             }
             s->lvl_pns[l] = nsmax;
             const int rb = s->panel_steps_only ? 0 : panel_rows_block(nsmax, s->esz);
             s->lvl_prows[l] = rb;
             if (rb) {
                 // row blocks: the diagonal blocks' first (by row block, then cblk), then the
-                // rb-row blocks below them
+                // rb-row blocks below them; LU: U^T's (side 1) before L's, which read them
+                const int sides = s->facto == FACTO_GETRF ? 2 : 1;
                 for (int b = 0; b < nsmax; b++)
-                    for (int p = p0; p < (int)pcbs.size(); p++)
-                        if (b < pcbs[p].ns) pitems.push_back({p, 0, b});
+                    for (int side = sides - 1; side >= 0; side--)
+                        for (int p = p0; p < (int)pcbs.size(); p++)
+                            if (b < pcbs[p].ns && (b > 0 || side == 0)) pitems.push_back({p, side, b});
                 for (int b = 0; b < nrbmax; b++)
                     for (int p = p0; p < (int)pcbs.size(); p++) {
                         const int k = pcbs[p].k, nbelow = (s->stride[k] - s->ncols[k] + rb - 1) / rb;
-                        if (b < nbelow) pitems.push_back({p, 0, pcbs[p].ns + b});
+                        for (int side = 0; side < sides; side++)
+                            if (b < nbelow) pitems.push_back({p, side, pcbs[p].ns + b});
                     }
             } else {
                 for (int j = 0; j < nsmax; j++)
@@ -1076,7 +1084,8 @@ int enqueue_numfact(b200_solver_t *s, cudaStream_t st, Trace *tr = nullptr) {
             if (s->lvl_prows[l])
                 launch_panel_rows<T>(s->facto, s->ds, s->d_pcb, s->d_pitem + s->lvl_pi0[l],
                                      s->lvl_pi1[l] - s->lvl_pi0[l], s->lvl_pns[l], s->lvl_prows[l], tickets + l,
-                                     solved, abort_word, L, s->d_thr, s->d_npiv, s->d_err, st);
+                                     solved, updated, abort_word, L, U, (T *)s->dWL, s->d_woff, s->d_thr, s->d_npiv,
+                                     s->d_err, st);
             else
                 launch_panel<T>(s->facto, s->ds, s->d_pcb, s->d_pitem + s->lvl_pi0[l], s->lvl_pi1[l] - s->lvl_pi0[l],
                                 tickets + l, solved, updated, abort_word, L, s->d_thr, s->d_npiv, s->d_err, st);
