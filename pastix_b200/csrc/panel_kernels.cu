@@ -53,6 +53,7 @@ __device__ __forceinline__ int ld_acquire(const int *p) {
     return v;
 }
 
+// Releases what the CTA wrote before its last barrier.
 __device__ __forceinline__ void st_release(int *p, int v) {
     asm volatile("st.release.gpu.global.b32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
 }
@@ -83,6 +84,16 @@ __device__ __forceinline__ void load4(const T *p, T v[4]) {
     }
 }
 
+// bytes of a B-byte copy (the rest of it zeros) into shared memory
+template <int B>
+__device__ __forceinline__ void cp_async(void *dst, const void *src, int bytes) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if constexpr (B == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(B), "r"(bytes) : "memory");
+}
+
 template <typename T>
 __device__ __forceinline__ void store4(T *p, T a, T b, T c, T d) {
     if constexpr (sizeof(T) == 4) {
@@ -95,115 +106,98 @@ __device__ __forceinline__ void store4(T *p, T a, T b, T c, T d) {
 
 // Factorization of the wd x wd diagonal tile held in the registers of the CTA's 16 x 16
 // threads: thread (tx, ty) has rows 4 tx .. 4 tx + 3 and columns 4 ty .. 4 ty + 3, acc[i][q]
-// (identity past wd).  Step p: the threads of block column p (LU: also of block row p) put
-// their 4 columns (rows) in the strip, and after one barrier every thread factors the 4 x 4
-// diagonal block and solves the strips of its own rows and columns itself, so that a step
-// costs one barrier, one shared-memory round trip and four dependent pivots instead of a
-// one-warp column chain: a 64 x 64 FP32 tile took about 29 K cycles with 8-column leaves.
-// Static pivoting replaces a pivot below thr in magnitude by +-thr.  LDL^T keeps D on the
-// diagonal and unit L below; LU keeps unit L below and U on and above the diagonal.
+// (identity past wd).  Step p: the half-warp of block column p takes the 4 x 4 diagonal
+// block by shuffles, factors it in every lane and solves its own 4 columns with it (four
+// dependent pivots), puts them in the strip, and after one barrier the threads right of
+// it subtract their product.  The strip is double buffered, so the half-warp of the next
+// step goes on as soon as its own columns are up to date.  What bounds a tile is this
+// chain (16 steps of four pivots, a barrier and a strip read), not its multiply-adds;
+// solving the strips in every thread that reads them, with no hand-off to wait for, took
+// 825 cycles a step in FP32 and 2200 in FP64.  Static pivoting replaces a
+// pivot below thr in magnitude by +-thr.  LDL^T keeps D on the diagonal and unit L below;
+// LU keeps unit L below and U on and above the diagonal (its row strip is solved with the
+// unit block by the threads that read it).
 //
 // POTRF: the blocks above the diagonal (tx < ty), idle otherwise, carry the inverse W of
 // the tile: they hold W[ty, tx]^T, start from zero and take the same step (their strip is
 // their own raw block, the identity in step tx), and wdiag is the diagonal block of W.
-// strip: 2 x 4 x 64 elements (LU: 2 x 8 x 64).
+// strip: 2 x STRIP elements.
 template <typename T, int FACTO>
 __device__ void factor_tile_regs(T (&acc)[4][4], T (&wdiag)[4][4], int wd, T *strip, double thr, int *s_piv,
                                  int *s_err) {
+    constexpr int STRIP = 8 * PB;  // 4 solved columns, then LU's 4 raw rows; LDL^T's 4 pivots
+    constexpr bool LU = FACTO == FACTO_GETRF;
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    constexpr int SB = (FACTO == FACTO_GETRF ? 8 : 4) * PB;
     int piv = 0, neg = 0;
 #pragma unroll 1
     for (int p = 0; 4 * p < wd; p++) {
-        T *cb = strip + (p & 1) * SB, *rb = cb + 4 * PB;  // column strip [k][row], LU row strip [k][column]
+        T *cb = strip + (p & 1) * STRIP, *rb = cb + 4 * PB;
         if (ty == p) {
+            const unsigned half = 0xffffu << (16 * (p & 1));
+            T g[4][4], P[4][4], d[4], iv[4];
 #pragma unroll
-            for (int q = 0; q < 4; q++) store4(cb + q * PB + 4 * tx, acc[0][q], acc[1][q], acc[2][q], acc[3][q]);
-        }
-        if (FACTO == FACTO_GETRF && tx == p && ty > p) {
+            for (int k = 0; k < 4; k++)
 #pragma unroll
-            for (int i = 0; i < 4; i++) store4(rb + i * PB + 4 * ty, acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-        }
-        __syncthreads();
-        if (ty < p) continue;
-        T g[4][4], P[4][4], Q[4][4];  // diagonal block g[row][col]; strips [row or column][k]
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            T v[4];
-            load4(cb + k * PB + 4 * p, v);
-#pragma unroll
-            for (int i = 0; i < 4; i++) g[i][k] = v[i];
-            load4(cb + k * PB + 4 * tx, v);
-#pragma unroll
-            for (int i = 0; i < 4; i++) P[i][k] = v[i];
-            load4((FACTO == FACTO_GETRF ? rb : cb) + k * PB + 4 * ty, v);
-#pragma unroll
-            for (int i = 0; i < 4; i++) Q[i][k] = v[i];
-        }
-        if (FACTO == FACTO_POTRF && tx == p) {
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int k = 0; k < 4; k++) P[i][k] = (i == k) ? (T)1 : (T)0;
-        }
-        T d[4], iv[4];
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            T a = g[c][c];
-            const bool rep = fabs(a) < (T)thr;
-            if (rep) a = (FACTO == FACTO_POTRF) ? (T)thr : ((a < (T)0) ? (T)(-thr) : (T)thr);
-            if (4 * p + c < wd) piv += rep;
-            if (FACTO == FACTO_POTRF) {
-                if (a < (T)0) {
-                    if (4 * p + c < wd) neg = 1;
-                    a = -a;
+                for (int i = 0; i < 4; i++) {
+                    if (LU || i >= k) g[i][k] = __shfl_sync(half, acc[i][k], p, 16);
+                    P[i][k] = (FACTO == FACTO_POTRF && tx == p) ? (i == k ? (T)1 : (T)0) : acc[i][k];
                 }
-                iv[c] = rsqrt(a);
-                d[c] = a * iv[c];
-            } else {
-                iv[c] = (T)1 / a;
-                d[c] = a;
-            }
-            g[c][c] = d[c];
 #pragma unroll
-            for (int i = c + 1; i < 4; i++) g[i][c] *= iv[c];
-#pragma unroll
-            for (int j = c + 1; j < 4; j++)
-#pragma unroll
-                for (int i = (FACTO == FACTO_GETRF ? c + 1 : j); i < 4; i++) {
-                    if (FACTO == FACTO_GETRF) g[i][j] -= g[i][c] * g[c][j];
-                    else if (FACTO == FACTO_SYTRF) g[i][j] -= (g[i][c] * d[c]) * g[j][c];
-                    else g[i][j] -= g[i][c] * g[j][c];
+            for (int c = 0; c < 4; c++) {
+                T a = g[c][c];
+                const bool rep = fabs(a) < (T)thr;
+                if (rep) a = (FACTO == FACTO_POTRF) ? (T)thr : ((a < (T)0) ? (T)(-thr) : (T)thr);
+                if (4 * p + c < wd) piv += rep;
+                if (FACTO == FACTO_POTRF) {
+                    if (a < (T)0) {
+                        if (4 * p + c < wd) neg = 1;
+                        a = -a;
+                    }
+                    iv[c] = rsqrt(a);
+                    d[c] = a * iv[c];
+                } else {
+                    iv[c] = (T)1 / a;
+                    d[c] = a;
                 }
-            // the strips' column c, and its terms in the columns after it
+                g[c][c] = d[c];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                P[i][c] *= iv[c];
-                if (FACTO != FACTO_GETRF) Q[i][c] *= iv[c];
+                for (int i = c + 1; i < 4; i++) g[i][c] *= iv[c];
 #pragma unroll
-                for (int j = c + 1; j < 4; j++) {
-                    if (FACTO == FACTO_GETRF) {
-                        P[i][j] -= P[i][c] * g[c][j];
-                        Q[i][j] -= Q[i][c] * g[j][c];
-                    } else if (FACTO == FACTO_SYTRF) {
-                        P[i][j] -= (P[i][c] * d[c]) * g[j][c];
-                        Q[i][j] -= (Q[i][c] * d[c]) * g[j][c];
-                    } else {
-                        P[i][j] -= P[i][c] * g[j][c];
-                        Q[i][j] -= Q[i][c] * g[j][c];
+                for (int j = c + 1; j < 4; j++)
+#pragma unroll
+                    for (int i = (LU ? c + 1 : j); i < 4; i++) {
+                        if (LU) g[i][j] -= g[i][c] * g[c][j];
+                        else if (FACTO == FACTO_SYTRF) g[i][j] -= (g[i][c] * d[c]) * g[j][c];
+                        else g[i][j] -= g[i][c] * g[j][c];
+                    }
+                // this thread's rows: column c, and its terms in the columns after it
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    P[i][c] *= iv[c];
+#pragma unroll
+                    for (int j = c + 1; j < 4; j++) {
+                        if (LU) P[i][j] -= P[i][c] * g[c][j];
+                        else if (FACTO == FACTO_SYTRF) P[i][j] -= (P[i][c] * d[c]) * g[j][c];
+                        else P[i][j] -= P[i][c] * g[j][c];
                     }
                 }
             }
-        }
-        if (ty == p) {
-            // final values of block column p (LU: the blocks below the diagonal)
+            if (LU && tx == p) {
+                // the unit block, for the row strip's readers
+#pragma unroll
+                for (int k = 0; k < 4; k++) store4(cb + k * PB + 4 * p, g[0][k], g[1][k], g[2][k], g[3][k]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; k++) store4(cb + k * PB + 4 * tx, P[0][k], P[1][k], P[2][k], P[3][k]);
+            }
+            if (FACTO == FACTO_SYTRF && tx == p) store4(rb, d[0], d[1], d[2], d[3]);
             if (tx == p) {
 #pragma unroll
                 for (int i = 0; i < 4; i++)
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
-                        acc[i][k] = g[i][k];
                         if (FACTO == FACTO_POTRF) wdiag[i][k] = P[i][k];
+                        if (LU || i >= k) acc[i][k] = g[i][k];
                     }
             } else if (tx > p || FACTO == FACTO_POTRF) {
 #pragma unroll
@@ -211,24 +205,62 @@ __device__ void factor_tile_regs(T (&acc)[4][4], T (&wdiag)[4][4], int wd, T *st
 #pragma unroll
                     for (int k = 0; k < 4; k++) acc[i][k] = P[i][k];
             }
-        } else if (FACTO == FACTO_GETRF && tx == p) {
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[k][j] = Q[j][k];
-        } else if (FACTO == FACTO_GETRF ? tx > p : (tx >= ty || (FACTO == FACTO_POTRF && tx <= p))) {
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const T m = (FACTO == FACTO_SYTRF) ? P[i][k] * d[k] : P[i][k];
-#pragma unroll
-                    for (int j = 0; j < 4; j++) acc[i][j] -= m * Q[j][k];
-                }
         }
+        if (LU && tx == p && ty > p) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) store4(rb + i * PB + 4 * ty, acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        }
+        __syncthreads();
+        if (ty <= p) continue;
+        if (LU ? tx < p : !(tx >= ty || (FACTO == FACTO_POTRF && tx <= p))) continue;
+        T P[4][4], Q[4][4];  // [row][k], [column][k]
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            T v[4];
+            load4(cb + k * PB + 4 * tx, v);
+#pragma unroll
+            for (int i = 0; i < 4; i++) P[i][k] = v[i];
+            load4((LU ? rb : cb) + k * PB + 4 * ty, v);
+#pragma unroll
+            for (int i = 0; i < 4; i++) Q[i][k] = v[i];
+        }
+        if (LU) {
+            // Q = L_pp^{-1} (rows of A), the unit block's entries from the strip
+            T l[4][4];
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                T v[4];
+                load4(cb + k * PB + 4 * p, v);
+#pragma unroll
+                for (int i = k + 1; i < 4; i++) l[i][k] = v[i];
+            }
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+#pragma unroll
+                for (int i = k + 1; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) Q[j][i] -= Q[j][k] * l[i][k];
+            if (tx == p) {
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[k][j] = Q[j][k];
+                continue;
+            }
+        }
+        T d[4] = {(T)1, (T)1, (T)1, (T)1};
+        if (FACTO == FACTO_SYTRF) load4(rb, d);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const T m = (FACTO == FACTO_SYTRF) ? P[i][k] * d[k] : P[i][k];
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] -= m * Q[j][k];
+            }
     }
-    if (tid == PT - 1) {  // active in every step
-        *s_piv += piv;
+    if (tx == 15) {  // one thread of every block column counted its pivots
+        if (piv) atomicAdd(s_piv, piv);
         if (neg) *s_err = 1;
     }
 }
@@ -250,82 +282,77 @@ __device__ __forceinline__ void load_tile_regs(T (&acc)[4][4], int wd, Load a) {
 
 // Solve of the R rows of xs (64 columns, pitch XP) against the lower triangular tile lt
 // (lt[c + l * 64], l < c; identity past the step's width) by substitution in 4-column
-// blocks over the CTA's threads, thread (tx, ty) rows MR tx .. and columns 4 ty ..: the
-// columns of block p, once final in the left blocks' terms, go through the strip (inside
-// xs, whose values are in registers) and every thread solves its own rows of them against
-// the 4 x 4 diagonal block.  x_c = (a_c - sum_{l<c} x_l t_cl) * rdiag[c]; LDL^T then
-// multiplies by dinv[c] = 1 / D_c.  All PT threads; xs final after the closing barrier.
+// blocks over the CTA's threads, thread (tx, ty) rows 4 tx + 64 h .. and columns 4 ty ..:
+// the half-warp of block column p solves its columns against the 4 x 4 diagonal block and
+// puts them in the strip (inside xs, whose values are in registers); after one barrier the
+// threads right of it subtract their product with the tile.  x_c = (a_c - sum_{l<c} x_l
+// t_cl) * rdiag[c]; LDL^T then multiplies by dinv[c] = 1 / D_c.  All PT threads; xs final
+// after the closing barrier.
 template <typename T, int FACTO, int R, int XP>
 __device__ void trsm_tile(T *xs, const T *lt, const T *rdiag, const T *dinv) {
-    constexpr int MR = R / 16;
+    constexpr int G = R / 64;  // groups of 64 rows
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    T acc[MR][4];
+    T acc[G][4][4];  // [group][row][column]
 #pragma unroll
     for (int q = 0; q < 4; q++)
 #pragma unroll
-        for (int h = 0; h < MR / 4; h++) {
+        for (int h = 0; h < G; h++) {
             T v[4];
-            load4(xs + MR * tx + 4 * h + (4 * ty + q) * XP, v);
+            load4(xs + 4 * tx + 64 * h + (4 * ty + q) * XP, v);
 #pragma unroll
-            for (int i = 0; i < 4; i++) acc[4 * h + i][q] = v[i];
+            for (int i = 0; i < 4; i++) acc[h][i][q] = v[i];
         }
     __syncthreads();
 #pragma unroll 1
     for (int p = 0; p < 16; p++) {
         T *st = xs + (p & 1) * 4 * R;
         if (ty == p) {
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-#pragma unroll
-                for (int h = 0; h < MR / 4; h++)
-                    store4(st + q * R + MR * tx + 4 * h, acc[4 * h][q], acc[4 * h + 1][q], acc[4 * h + 2][q],
-                           acc[4 * h + 3][q]);
-        }
-        T t[4][4], g[4][4], rd[4];  // own columns' rows of the tile [j][k]; the diagonal block [j][k], j > k
-        if (ty >= p) {
+            T g[4][4], rd[4];
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 T v[4];
                 load4(lt + 4 * p + (4 * p + k) * PB, v);
 #pragma unroll
                 for (int j = 0; j < 4; j++) g[j][k] = v[j];
+            }
+            load4(rdiag + 4 * p, rd);
+#pragma unroll
+            for (int h = 0; h < G; h++) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        acc[h][i][k] *= rd[k];
+#pragma unroll
+                        for (int j = k + 1; j < 4; j++) acc[h][i][j] -= acc[h][i][k] * g[j][k];
+                    }
+                    store4(st + k * R + 4 * tx + 64 * h, acc[h][0][k], acc[h][1][k], acc[h][2][k], acc[h][3][k]);
+                }
+            }
+        }
+        T t[4][4];  // own columns' rows of the tile [column][k]
+        if (ty > p) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                T v[4];
                 load4(lt + 4 * ty + (4 * p + k) * PB, v);
 #pragma unroll
                 for (int j = 0; j < 4; j++) t[j][k] = v[j];
             }
-            load4(rdiag + 4 * p, rd);
         }
         __syncthreads();
-        if (ty < p) continue;
+        if (ty <= p) continue;
 #pragma unroll
-        for (int h = 0; h < MR / 4; h++) {
-            T x[4][4];  // [row][k]
+        for (int h = 0; h < G; h++) {
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 T v[4];
-                load4(st + k * R + MR * tx + 4 * h, v);
+                load4(st + k * R + 4 * tx + 64 * h, v);
 #pragma unroll
-                for (int i = 0; i < 4; i++) x[i][k] = v[i];
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[h][i][j] -= v[i] * t[j][k];
             }
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    x[i][k] *= rd[k];
-#pragma unroll
-                    for (int j = k + 1; j < 4; j++) x[i][j] -= x[i][k] * g[j][k];
-                }
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    if (ty == p) {
-                        acc[4 * h + i][j] = x[i][j];
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 4; k++) acc[4 * h + i][j] -= x[i][k] * t[j][k];
-                    }
-                }
         }
     }
     __syncthreads();
@@ -333,48 +360,90 @@ __device__ void trsm_tile(T *xs, const T *lt, const T *rdiag, const T *dinv) {
     for (int q = 0; q < 4; q++) {
         const T m = (FACTO == FACTO_SYTRF) ? dinv[4 * ty + q] : (T)1;
 #pragma unroll
-        for (int h = 0; h < MR / 4; h++) {
-            if (FACTO == FACTO_SYTRF)
-                store4(xs + MR * tx + 4 * h + (4 * ty + q) * XP, acc[4 * h][q] * m, acc[4 * h + 1][q] * m,
-                       acc[4 * h + 2][q] * m, acc[4 * h + 3][q] * m);
-            else
-                store4(xs + MR * tx + 4 * h + (4 * ty + q) * XP, acc[4 * h][q], acc[4 * h + 1][q], acc[4 * h + 2][q],
-                       acc[4 * h + 3][q]);
+        for (int h = 0; h < G; h++) {
+            if (FACTO == FACTO_SYTRF) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) acc[h][i][q] *= m;
+            }
+            store4(xs + 4 * tx + 64 * h + (4 * ty + q) * XP, acc[h][0][q], acc[h][1][q], acc[h][2][q], acc[h][3][q]);
         }
     }
     __syncthreads();
 }
 
+template <typename T>
+__device__ __forceinline__ void load_vec(const T *p, T *v) {  // 16 bytes
+    if constexpr (sizeof(T) == 4) {
+        const float4 q = *reinterpret_cast<const float4 *>(p);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+        const double2 q = *reinterpret_cast<const double2 *>(p);
+        v[0] = q.x; v[1] = q.y;
+    }
+}
+template <typename T>
+__device__ __forceinline__ void store_vec(T *p, const T *v) {
+    if constexpr (sizeof(T) == 4) *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+}
+
+// acc = X B over the first nl (a multiple of 8) of 64 K values: X[r, l] = xs[l * R + r],
+// B[l, c] = bs[l * 64 + c].  Thread (tx, ty): columns 4 ty .. 4 ty + 3, rows in groups of
+// 16 bytes, group h at rows EPV (tx + 16 h) .. (a warp's reads of a group are 256
+// contiguous bytes; 8 contiguous rows per thread met every bank twice).  The operands of
+// the next l are read before the products of this one: two warps per SM sub-partition
+// cannot hide a shared-memory read behind 16 or 32 multiply-adds otherwise (a 64 x 64 x 64
+// FP32 product took 6.2 K cycles, three times its multiply-adds).
+template <typename T, int R>
+struct RowTile {
+    static constexpr int MR = R / 16, EPV = 16 / (int)sizeof(T), G = MR / EPV;
+    static __device__ __forceinline__ int row(int i) { return EPV * ((threadIdx.x & 15) + 16 * (i / EPV)) + i % EPV; }
+    static __device__ __forceinline__ void mul(T (&acc)[MR][4], const T *xs, const T *bs, int nl) {
+        const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+        const T *xp = xs + EPV * tx, *bp = bs + 4 * ty;
+#pragma unroll
+        for (int i = 0; i < MR; i++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) acc[i][q] = 0;
+        T av[2][MR], bv[2][4];
+        auto fetch = [&](int l, int s) {
+#pragma unroll
+            for (int h = 0; h < G; h++) load_vec(xp + l * R + 16 * EPV * h, av[s] + EPV * h);
+            load4(bp + l * PB, bv[s]);
+        };
+        fetch(0, 0);
+#pragma unroll 1
+        for (int l0 = 0; l0 < nl; l0 += 8) {
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                if (u < 7 || l0 + 8 < nl) fetch(l0 + u + 1, (u + 1) & 1);
+#pragma unroll
+                for (int i = 0; i < MR; i++)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) acc[i][q] += av[u & 1][i] * bv[u & 1][q];
+            }
+        }
+    }
+};
+
 // The same solve as the product with the tile's inverse, bs[l * 64 + c] = W[c, l] (POTRF
 // row blocks): no dependent chain, 64 x 64 / 2 multiply-adds per row.
 template <typename T, int R>
 __device__ void trsm_inverse(T *xs, const T *bs) {
-    constexpr int MR = R / 16;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    T acc[MR][4];
-#pragma unroll
-    for (int i = 0; i < MR; i++)
-#pragma unroll
-        for (int q = 0; q < 4; q++) acc[i][q] = 0;
-    const int lend = 4 * ((ty | 1) + 1);  // W[c, l] = 0 for l > c
-#pragma unroll 8
-    for (int l = 0; l < lend; l++) {
-        T av[MR], bv[4];
-#pragma unroll
-        for (int h = 0; h < MR / 4; h++) load4(xs + l * R + MR * tx + 4 * h, av + 4 * h);
-        load4(bs + l * PB + 4 * ty, bv);
-#pragma unroll
-        for (int i = 0; i < MR; i++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) acc[i][q] += av[i] * bv[q];
-    }
+    using RT = RowTile<T, R>;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    T acc[RT::MR][4];
+    RT::mul(acc, xs, bs, 8 * (ty / 2 + 1));  // W[c, l] = 0 for l > c
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < 4; q++)
 #pragma unroll
-        for (int h = 0; h < MR / 4; h++)
-            store4(xs + MR * tx + 4 * h + (4 * ty + q) * R, acc[4 * h][q], acc[4 * h + 1][q], acc[4 * h + 2][q],
-                   acc[4 * h + 3][q]);
+        for (int h = 0; h < RT::G; h++) {
+            T v[RT::EPV];
+#pragma unroll
+            for (int i = 0; i < RT::EPV; i++) v[i] = acc[RT::EPV * h + i][q];
+            store_vec(xs + RT::EPV * (tx + 16 * h) + (4 * ty + q) * R, v);
+        }
     __syncthreads();
 }
 
@@ -573,7 +642,7 @@ __global__ void __launch_bounds__(PT, sizeof(T) == 4 ? 2 : 1) panel_kernel(DevSy
 // (the stored U^T) and owns the diagonal tiles, side 1 against the unit L[j, j].
 // solved counts side 0, solved_v side 1, whose item of a row block comes first.  The
 // one-CTA diagonal blocks and row-by-row solves this replaces took 56 of the 66 ms of a
-// 64^3 convection-diffusion LU in FP32; the panel launches take 9.3 ms.
+// 64^3 convection-diffusion LU in FP32; the panel launches take 7.0 ms.
 struct RowsCtx {
     int *sol, *sol_v;     // counters of the cblk's row blocks
     const int *abort_word;
@@ -600,7 +669,6 @@ __device__ __forceinline__ bool rows_need(const RowsCtx &x, int side, int c, int
 template <typename T, int FACTO, int R>
 __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, int side, T *L, T *U, T *Wk, T *lt, T *rdiag,
                           T *dinv, T *dd, T *xs, const RowsCtx &x) {
-    constexpr int MR = R / 16;  // rows of a thread's update tile
     constexpr bool LU = FACTO == FACTO_GETRF;
     const int tid = threadIdx.x;
     const int k = pc.k, W = s.ncols[k], S = s.stride[k], ld = s.ld[k];
@@ -614,22 +682,26 @@ __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, int side,
     // columns held (lower part for the diagonal block; V: left of its diagonal tile)
     const int ncol = drows ? (side ? PB * b : min(W, PB * (b + 1))) : W;
     const int nstep = drows ? b : pc.ns;                 // steps solved in this row block
-    // the row block: rows past nr, the diagonal tile's upper triangle (not LU) and (below
-    // the diagonal block) the last step's columns past W as zeros
+    // the row block: rows past nr and (below the diagonal block) the last step's columns past
+    // W as zeros; the whole of it in flight at once
     const int nzero = drows ? ncol : PB * pc.ns;
-    constexpr int CG = PT / R;  // column groups of a load pass
-    for (int c0s = 0; c0s < nzero; c0s += 4 * CG) {
-        stage_n<4, T>(
-            [&](int u) {
-                const int r = tid % R, c = c0s + tid / R + CG * u;
-                const bool keep = r < nr && c < ncol && (LU || !drows || c < PB * b || r >= c - PB * b);
-                return keep ? __ldcg(P + r0 + r + (size_t)c * ld) : (T)0;
-            },
-            [&](int u, T v) {
-                const int r = tid % R, c = c0s + tid / R + CG * u;
-                if (c < nzero) xs[r + c * R] = v;
-            });
+    constexpr int EPV = 16 / (int)sizeof(T);
+    if (r0 % EPV == 0) {
+        // 16-byte copies (every panel column starts on a 16-byte boundary)
+        constexpr int RV = R / EPV;
+        for (int idx = tid; idx < RV * nzero; idx += PT) {
+            const int r = (idx % RV) * EPV, c = idx / RV;
+            const int bytes = c < ncol && r < nr ? min(EPV, nr - r) * (int)sizeof(T) : 0;
+            cp_async<16>(xs + r + c * R, bytes ? P + r0 + r + (size_t)c * ld : P, bytes);
+        }
+    } else {
+        for (int idx = tid; idx < R * nzero; idx += PT) {
+            const int r = idx % R, c = idx / R;
+            const bool in = c < ncol && r < nr;
+            cp_async<sizeof(T)>(xs + r + c * R, in ? P + r0 + r + (size_t)c * ld : P, in ? (int)sizeof(T) : 0);
+        }
     }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
     if (LU && drows) {
         // the diagonal block is the sum of L's and the transposed U's (core_zgeadd): 8 rows x
         // 4 columns of it per warp access
@@ -685,14 +757,14 @@ __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, int side,
         __syncthreads();
         if (FACTO == FACTO_POTRF) trsm_inverse<T, R>(xs + c0 * R, lt);
         else trsm_tile<T, FACTO, R, R>(xs + c0 * R, lt, rdiag, dinv);
-        for (int idx = tid; idx < R * wd; idx += PT) {
-            const int r = idx % R, c = idx / R;
-            if (r < nr) P[r0 + r + (size_t)(c0 + c) * ld] = xs[r + (c0 + c) * R];
+#pragma unroll 8
+        for (int u = 0; u < R * PB / PT; u++) {
+            const int r = (tid + PT * u) % R, c = (tid + PT * u) / R;
+            if (r < nr && c < wd) P[r0 + r + (size_t)(c0 + c) * ld] = xs[r + (c0 + c) * R];
         }
         if (drows) {
             __syncthreads();
             if (tid == 0) {
-                __threadfence();
                 st_release(sol + b, j + 1);
             }
             if (LU)  // the other panel's diagonal block keeps the transposed factor (core_zgetmo)
@@ -729,34 +801,31 @@ __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, int side,
                 load_diag(j + 1);
                 have = true;
             }
-            T acc[MR][4];
-#pragma unroll
-            for (int i = 0; i < MR; i++)
-#pragma unroll
-                for (int q = 0; q < 4; q++) acc[i][q] = 0;
-            const T *xa = xs + c0 * R + MR * tx;
-#pragma unroll 4
-            for (int l = 0; l < wd; l++) {
-                T av[MR], bv[4];
-#pragma unroll
-                for (int h = 0; h < MR / 4; h++) load4(xa + l * R + 4 * h, av + 4 * h);
-                load4(bs + l * PB + 4 * ty, bv);
-#pragma unroll
-                for (int i = 0; i < MR; i++)
-#pragma unroll
-                    for (int q = 0; q < 4; q++) acc[i][q] += av[i] * bv[q];
-            }
+            using RT = RowTile<T, R>;
+            T acc[RT::MR][4];
+            RT::mul(acc, xs + c0 * R, bs, PB);  // a step with columns right of it is a full one
             T *xc = xs + (PB * c) * R;
+            if (own) {
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int cc = 4 * ty + q;
-                if (cc < wc) {
+                for (int q = 0; q < 4; q++)
 #pragma unroll
-                    for (int i = 0; i < MR; i++) {
-                        const int r = MR * tx + i;
-                        if (!own || r >= cc) xc[r + cc * R] -= acc[i][q];
+                    for (int i = 0; i < RT::MR; i++) {
+                        const int r = RT::row(i), cc = 4 * ty + q;
+                        if (cc < wc && r >= cc) xc[r + cc * R] -= acc[i][q];
                     }
-                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+#pragma unroll
+                    for (int h = 0; h < RT::G; h++) {
+                        if (4 * ty + q >= wc) continue;
+                        T *p = xc + RT::EPV * (tx + 16 * h) + (4 * ty + q) * R;
+                        T v[RT::EPV];
+                        load_vec(p, v);
+#pragma unroll
+                        for (int i = 0; i < RT::EPV; i++) v[i] -= acc[RT::EPV * h + i][q];
+                        store_vec(p, v);
+                    }
             }
             __syncthreads();
         }
@@ -800,7 +869,6 @@ __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, int side,
         }
         __syncthreads();
         if (tid == 0) {
-            __threadfence();
             st_release(sol + b, b + 1);
         }
         if (FACTO == FACTO_POTRF && b + 1 < pc.ns + (S > W ? 1 : 0)) {
