@@ -74,10 +74,14 @@ struct Upd {
     int M, N, K;
     int colbase;  // column in f of block j's first row
     int tiles_m, tiles_n;
-    int tile0;    // first tile index of this update inside its launch
     int flags;
     int nb;       // tensor-core updates: columns per tile (a multiple of 32, at most the launch's tile width)
     int rm0;      // first entry of its row map (M entries: row rowA0 + i of k -> row of f, or -1)
+    // where the operands lie, so that a kernel reads this record only: element offsets in
+    // their arenas (flags) of row rowA0 and of row rowB0 in column colK0, of column
+    // colbase of f, and of D's entry colK0; leading dimensions of k and f
+    int ldk, ldf;
+    int64_t offA, offB, offC, offD;
 };
 
 // Item of the tree-bottom launch, in ticket order: fact = 1 factors cblk k (diagonal
@@ -138,6 +142,7 @@ struct Level {
     int t0, t1;          // row tasks of the off-diagonal panels
     int u0, u1;          // updates
     int ntiles;          // GEMM tiles of the level
+    int64_t m0;          // first of them in the tile map
     int nmax;            // widest cblk of the level
     int64_t flops;
 };

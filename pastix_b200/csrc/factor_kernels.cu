@@ -492,26 +492,6 @@ __global__ void __launch_bounds__(256) panel_trsm_kernel(DevSym s, const RowTask
 
 // ------------------------------------------------------------------ updates
 
-__device__ __forceinline__ int find_update(const Upd *__restrict__ upds, int nupd, int tile) {
-    int lo = 0, hi = nupd - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (upds[mid].tile0 <= tile) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
-
-__device__ __forceinline__ void tile_coords(const Upd &u, int lt, int &mt, int &nt) {
-    if (u.flags & UPD_SYM) {
-        nt = 0;
-        while (lt >= u.tiles_m - nt) { lt -= u.tiles_m - nt; nt++; }
-        mt = nt + lt;
-    } else {
-        mt = lt % u.tiles_m;
-        nt = lt / u.tiles_m;
-    }
-}
-
 __device__ __forceinline__ void dmma_16x8x4(double (&c)[4], const double (&a)[2], double b) {
     asm volatile(
         "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
@@ -521,129 +501,207 @@ __device__ __forceinline__ void dmma_16x8x4(double (&c)[4], const double (&a)[2]
 
 constexpr int UT_M = 64, UT_N = 64, UT_K = 16, UT_STAGES = 3, UT_LDS = UT_M + 4;
 constexpr int UPD_F64_SMEM = 2 * UT_STAGES * UT_K * UT_LDS * sizeof(double);
+constexpr int UPD_F64_CTAS = 4;  // per SM: 128 registers per thread, 52 KB of shared memory each
 
-// 64x64 output tile per CTA, 4 warps (2x2) of 32x32, DMMA m16n8k4, 3-stage
-// cp.async pipeline over K in chunks of 16 columns.
-__global__ void __launch_bounds__(128) update_f64_kernel(DevSym s, const Upd *__restrict__ upds, int nupd,
-                                                         double *L, double *U) {
+// 64x64 output tiles, 4 warps (2x2) of 32x32, DMMA m16n8k4, 3-stage cp.async pipeline over
+// K in chunks of 16 columns.  The grid is persistent (UPD_F64_CTAS per SM) and the pipeline
+// runs over the chunks of a CTA's tiles one after the other: while a tile's last chunks
+// are multiplied and its sums go out, the first chunks of the next tile are already on
+// their way, and its record (read two tiles ahead through the ring su) costs no wait.  A
+// launch of one CTA per tile spent a fifth of each 64 x 64 x 320 tile on finding its
+// update (a binary search), filling the pipeline and draining it.  Warps skip the 8-column
+// and 16-row groups past the update's edge and the 32 x 32 quarters above the diagonal of
+// a symmetric update (17 % of the issued products at 80^3); which quarter a warp takes
+// turns with the CTA, so that the skipped ones do not all idle the same SM sub-partition.
+__global__ void __launch_bounds__(128, UPD_F64_CTAS)
+    update_f64_kernel(DevSym s, const Upd *__restrict__ upds, const int2 *__restrict__ tmap, int ntiles, double *L,
+                      double *U) {
     extern __shared__ __align__(16) unsigned char upd_smem[];
     double(*As)[UT_K][UT_LDS] = reinterpret_cast<double(*)[UT_K][UT_LDS]>(upd_smem);
     double(*Bs)[UT_K][UT_LDS] = reinterpret_cast<double(*)[UT_K][UT_LDS]>(upd_smem + sizeof(double) * UT_STAGES * UT_K * UT_LDS);
     __shared__ double Ds[UT_STAGES][UT_K];
-    __shared__ int drow[UT_M];
-    const int tile = blockIdx.x;
-    const Upd u = upds[find_update(upds, nupd, tile)];
-    int mt, nt;
-    tile_coords(u, tile - u.tile0, mt, nt);
-    const int m0 = mt * UT_M, n0 = nt * UT_N;
-    const int k = u.k, ldk = s.ld[k];
-    const double *Ap = ((u.flags & UPD_A_U) ? U : L) + s.off[k] + u.rowA0 + m0 + (size_t)u.colK0 * ldk;
-    const double *Bp = ((u.flags & UPD_B_U) ? U : L) + s.off[k] + u.rowB0 + n0 + (size_t)u.colK0 * ldk;
-    const double *Dp = L + s.off[k] + (size_t)u.colK0 * (ldk + 1);
-    const bool scale = (u.flags & UPD_SCALE_D) != 0;
-    const int mrem = u.M - m0, nrem = u.N - n0;
+    constexpr int UW = sizeof(Upd) / 4;
+    static_assert(UW <= 31 && sizeof(Upd) % 8 == 0, "one warp reads a record and its tile");
+    __shared__ __align__(8) int su[8][32];  // records of the tiles from the one being summed to the next to load
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp & 1, wn = warp >> 1;
+    const int quarter = (warp + blockIdx.x) & 3, wm = quarter & 1, wn = quarter >> 1;
     const int g = lane >> 2, tg = lane & 3;
-
-    auto load_stage = [&](int st, int kc) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int idx = tid + i * 128;
-            const int r = idx & 63, c = idx >> 6;
-            const int kk = kc + c;
-            const bool okA = (r < mrem) && (kk < u.K);
-            const bool okB = (r < nrem) && (kk < u.K);
-            cp_async8(&As[st][c][r], okA ? Ap + r + (size_t)kk * ldk : Ap, okA);
-            cp_async8(&Bs[st][c][r], okB ? Bp + r + (size_t)kk * ldk : Bp, okB);
-        }
-        if (scale && tid < UT_K) {
-            const int kk = kc + tid;
-            Ds[st][tid] = (kk < u.K) ? Dp[(size_t)kk * (ldk + 1)] : 0.0;
-        }
+    const int nmine = (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;  // tiles of this CTA
+    auto tile_of = [&](int q) { return tmap[blockIdx.x + q * gridDim.x]; };
+    // record of tile q: words of its update, then the tile's coordinates
+    int word = 0;
+    auto read_record = [&](int2 t) {
+        if (warp == 0) word = lane < UW ? reinterpret_cast<const int *>(upds + t.x)[lane] : t.y;
+    };
+    auto keep_record = [&](int q) {
+        if (warp == 0) su[q & 7][lane] = word;
     };
 
-    double acc[2][4][4];
+    // loads: tile lq, chunk at column lk
+    int lq = 0, lk = 0, lK = 0, lld = 0;
+    const double *lA = nullptr, *lB = nullptr, *lD = nullptr;  // this thread's first element of each operand
+    bool lokA = false, lokB = false;
+    int2 ahead = make_int2(0, 0);  // tile lq + 2
+    auto open_tile = [&]() {       // record lq is in su
+        const Upd &u = *reinterpret_cast<const Upd *>(su[lq & 7]);
+        const int m0 = (su[lq & 7][31] & 0xffff) * UT_M, n0 = (su[lq & 7][31] >> 16) * UT_N;
+        const int r = tid & 63, c = tid >> 6;
+        lK = u.K;
+        lld = u.ldk;
+        lokA = r < u.M - m0;
+        lokB = r < u.N - n0;
+        lA = ((u.flags & UPD_A_U) ? U : L) + u.offA + (lokA ? m0 + r : 0) + (size_t)c * lld;
+        lB = ((u.flags & UPD_B_U) ? U : L) + u.offB + (lokB ? n0 + r : 0) + (size_t)c * lld;
+        lD = (u.flags & UPD_SCALE_D) ? L + u.offD + (size_t)(tid & (UT_K - 1)) * (lld + 1) : nullptr;
+        lk = 0;
+    };
+    auto load_stage = [&](int st) {
+        const int r = tid & 63, c = tid >> 6;
 #pragma unroll
-    for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) acc[a][b][e] = 0.0;
+        for (int i = 0; i < UT_K / 2; i++) {
+            const bool ok = lk + c + 2 * i < lK;
+            cp_async8(&As[st][c + 2 * i][r], ok ? lA + (size_t)(2 * i) * lld : lA, ok && lokA);
+            cp_async8(&Bs[st][c + 2 * i][r], ok ? lB + (size_t)(2 * i) * lld : lB, ok && lokB);
+        }
+        if (tid < UT_K && lD) {
+            const bool ok = lk + tid < lK;
+            cp_async8(&Ds[st][tid], ok ? lD : L, ok);
+            lD += (size_t)UT_K * (lld + 1);
+        }
+        lA += (size_t)UT_K * lld;
+        lB += (size_t)UT_K * lld;
+        lk += UT_K;
+    };
+    // the next chunk into stage st, if there is one; the record of the tile after a newly
+    // opened one is then on its way in `word` (returns true: keep_record(lq + 1) later)
+    auto load_next = [&](int st) -> bool {
+        if (lq >= nmine) return false;
+        load_stage(st);
+        if (lk < lK) return false;
+        lq++;
+        if (lq >= nmine) return false;
+        open_tile();
+        if (lq + 1 < nmine) {
+            read_record(ahead);
+            if (lq + 2 < nmine) ahead = tile_of(lq + 2);
+            return true;
+        }
+        return false;
+    };
+    if (nmine <= 0) return;
+    read_record(tile_of(0));
+    keep_record(0);
+    if (nmine > 1) {
+        read_record(tile_of(1));
+        keep_record(1);
+    }
+    if (nmine > 2) ahead = tile_of(2);
+    __syncthreads();
+    open_tile();
 
-    const int nk = (u.K + UT_K - 1) / UT_K;
+    // the first two chunks; records they read ahead are kept at once
 #pragma unroll
     for (int st = 0; st < UT_STAGES - 1; st++) {
-        if (st < nk) load_stage(st, st * UT_K);
+        if (load_next(st)) keep_record(lq + 1);
         cp_async_commit();
-    }
-    for (int kt = 0; kt < nk; kt++) {
-        cp_async_wait<UT_STAGES - 2>();
         __syncthreads();
-        const int st = kt % UT_STAGES;
-        const int nxt = kt + UT_STAGES - 1;
-        if (nxt < nk) load_stage(nxt % UT_STAGES, nxt * UT_K);
-        cp_async_commit();
+    }
+    int st = 0;
+    for (int q = 0; q < nmine; q++) {
+        double acc[2][4][4];
 #pragma unroll
-        for (int k4 = 0; k4 < UT_K; k4 += 4) {
-            double a[2][2], b[4];
-            const double dsc = scale ? Ds[st][k4 + tg] : 1.0;
+        for (int a = 0; a < 2; a++)
 #pragma unroll
-            for (int mi = 0; mi < 2; mi++) {
-                const int row = wm * 32 + mi * 16 + g;
-                a[mi][0] = As[st][k4 + tg][row] * dsc;
-                a[mi][1] = As[st][k4 + tg][row + 8] * dsc;
+            for (int b = 0; b < 4; b++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) acc[a][b][e] = 0.0;
+        const Upd &u = *reinterpret_cast<const Upd *>(su[q & 7]);
+        const int m0 = (su[q & 7][31] & 0xffff) * UT_M + wm * 32, n0 = (su[q & 7][31] >> 16) * UT_N + wn * 32;
+        const int flags = u.flags, nk = (u.K + UT_K - 1) / UT_K;
+        const bool scale = (flags & UPD_SCALE_D) != 0, sym = (flags & UPD_SYM) != 0;
+        const bool skip = sym && m0 + 31 < n0;
+        const int mrem = skip ? 0 : u.M - m0, nrem = skip ? 0 : u.N - n0;  // of this warp's quarter
+        const int nmi = (mrem + 15) >> 4, nni = mrem > 0 ? (nrem + 7) >> 3 : 0;
+        int drow[2][2];
+        for (int kt = 0; kt < nk; kt++) {
+            cp_async_wait<UT_STAGES - 2>();
+            __syncthreads();
+            const int nxt = st + UT_STAGES - 1 >= UT_STAGES ? st - 1 : st + UT_STAGES - 1;
+            const bool keep = load_next(nxt);
+            cp_async_commit();
+            if (kt == nk - 1) {
+                // destination rows, used after the last products
+#pragma unroll
+                for (int mi = 0; mi < 2; mi++)
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int row = mi * 16 + h * 8 + g;
+                        drow[mi][h] = row < mrem ? __ldg(s.rmap + u.rm0 + m0 + row) : -1;
+                    }
             }
+            if (nni > 0) {
 #pragma unroll
-            for (int ni = 0; ni < 4; ni++) b[ni] = Bs[st][k4 + tg][wn * 32 + ni * 8 + g];
+                for (int k4 = 0; k4 < UT_K; k4 += 4) {
+                    double a[2][2], b[4];
+                    const double dsc = scale ? Ds[st][k4 + tg] : 1.0;
 #pragma unroll
-            for (int mi = 0; mi < 2; mi++)
+                    for (int mi = 0; mi < 2; mi++) {
+                        const int row = wm * 32 + mi * 16 + g;
+                        a[mi][0] = As[st][k4 + tg][row];
+                        a[mi][1] = As[st][k4 + tg][row + 8];
+                        if (scale) {
+                            a[mi][0] *= dsc;
+                            a[mi][1] *= dsc;
+                        }
+                    }
 #pragma unroll
-                for (int ni = 0; ni < 4; ni++) dmma_16x8x4(acc[mi][ni], a[mi], b[ni]);
+                    for (int ni = 0; ni < 4; ni++) b[ni] = Bs[st][k4 + tg][wn * 32 + ni * 8 + g];
+#pragma unroll
+                    for (int ni = 0; ni < 4; ni++)
+                        if (ni < nni) {
+                            dmma_16x8x4(acc[0][ni], a[0], b[ni]);
+                            if (nmi > 1) dmma_16x8x4(acc[1][ni], a[1], b[ni]);
+                        }
+                }
+            }
+            if (keep) keep_record(lq + 1);
+            st = st + 1 == UT_STAGES ? 0 : st + 1;
+        }
+        double *C = ((flags & UPD_C_U) ? U : L) + u.offC;
+        const int ldf = u.ldf;
+        const bool atomic = (flags & UPD_ATOMIC) != 0;
+#pragma unroll
+        for (int mi = 0; mi < 2; mi++) {
+#pragma unroll
+            for (int ni = 0; ni < 4; ni++) {
+                if (ni >= nni) continue;
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int row = mi * 16 + g + (e >> 1) * 8, col = ni * 8 + 2 * tg + (e & 1);
+                    const int d = drow[mi][e >> 1];
+                    if (d < 0 || col >= nrem || (sym && m0 + row < n0 + col)) continue;
+                    double *p = C + d + (size_t)(n0 + col) * ldf;
+                    if (atomic) atomicAdd(p, -acc[mi][ni][e]);
+                    else *p -= acc[mi][ni][e];
+                }
+            }
         }
     }
     cp_async_wait<0>();
-    if (tid < UT_M) drow[tid] = (m0 + tid < u.M) ? __ldg(s.rmap + u.rm0 + m0 + tid) : -1;
-    __syncthreads();
-    double *C = ((u.flags & UPD_C_U) ? U : L) + s.off[u.f];
-    const int ldf = s.ld[u.f];
-    const bool atomic = (u.flags & UPD_ATOMIC) != 0;
-    const bool sym = (u.flags & UPD_SYM) != 0;
-#pragma unroll
-    for (int mi = 0; mi < 2; mi++) {
-#pragma unroll
-        for (int ni = 0; ni < 4; ni++) {
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int row = wm * 32 + mi * 16 + g + (e >> 1) * 8;
-                const int col = wn * 32 + ni * 8 + 2 * tg + (e & 1);
-                if (n0 + col >= u.N) continue;
-                if (sym && m0 + row < n0 + col) continue;
-                const int d = drow[row];
-                if (d < 0) continue;
-                double *p = C + d + (size_t)(u.colbase + n0 + col) * ldf;
-                if (atomic) atomicAdd(p, -acc[mi][ni][e]);
-                else *p -= acc[mi][ni][e];
-            }
-        }
-    }
 }
 
 // FP32 factor update on CUDA cores: 64x64 tile, 256 threads (4x4 each), K chunks of 16.
-__global__ void __launch_bounds__(256) update_simt_f32_kernel(DevSym s, const Upd *__restrict__ upds, int nupd,
-                                                              float *L, float *U) {
+__global__ void __launch_bounds__(256) update_simt_f32_kernel(DevSym s, const Upd *__restrict__ upds,
+                                                              const int2 *__restrict__ tmap, float *L, float *U) {
     __shared__ __align__(16) float As[2][UT_K][UT_M + 4];
     __shared__ __align__(16) float Bs[2][UT_K][UT_N + 4];
     __shared__ int drow[UT_M];
-    const int tile = blockIdx.x;
-    const Upd u = upds[find_update(upds, nupd, tile)];
-    int mt, nt;
-    tile_coords(u, tile - u.tile0, mt, nt);
-    const int m0 = mt * UT_M, n0 = nt * UT_N;
-    const int k = u.k, ldk = s.ld[k];
-    const float *Ap = ((u.flags & UPD_A_U) ? U : L) + s.off[k] + u.rowA0 + m0 + (size_t)u.colK0 * ldk;
-    const float *Bp = ((u.flags & UPD_B_U) ? U : L) + s.off[k] + u.rowB0 + n0 + (size_t)u.colK0 * ldk;
-    const float *Dp = L + s.off[k] + (size_t)u.colK0 * (ldk + 1);
+    const int2 tc2 = tmap[blockIdx.x];
+    const Upd u = upds[tc2.x];
+    const int m0 = (tc2.y & 0xffff) * UT_M, n0 = (tc2.y >> 16) * UT_N, ldk = u.ldk;
+    const float *Ap = ((u.flags & UPD_A_U) ? U : L) + u.offA + m0;
+    const float *Bp = ((u.flags & UPD_B_U) ? U : L) + u.offB + n0;
+    const float *Dp = L + u.offD;
     const bool scale = (u.flags & UPD_SCALE_D) != 0;
     const int mrem = u.M - m0, nrem = u.N - n0;
     const int tid = threadIdx.x;
@@ -688,8 +746,8 @@ __global__ void __launch_bounds__(256) update_simt_f32_kernel(DevSym s, const Up
     }
     if (tid < UT_M) drow[tid] = (m0 + tid < u.M) ? __ldg(s.rmap + u.rm0 + m0 + tid) : -1;
     __syncthreads();
-    float *C = ((u.flags & UPD_C_U) ? U : L) + s.off[u.f];
-    const int ldf = s.ld[u.f];
+    float *C = ((u.flags & UPD_C_U) ? U : L) + u.offC;
+    const int ldf = u.ldf;
     const bool atomic = (u.flags & UPD_ATOMIC) != 0;
     const bool sym = (u.flags & UPD_SYM) != 0;
 #pragma unroll
@@ -701,7 +759,7 @@ __global__ void __launch_bounds__(256) update_simt_f32_kernel(DevSym s, const Up
             if (sym && m0 + row < n0 + col) continue;
             const int d = drow[row];
             if (d < 0) continue;
-            float *p = C + d + (size_t)(u.colbase + n0 + col) * ldf;
+            float *p = C + d + (size_t)(n0 + col) * ldf;
             if (atomic) atomicAdd(p, -acc[a][b]);
             else *p -= acc[a][b];
         }
@@ -1198,20 +1256,20 @@ void launch_trsm(const DevSym &s, const RowTask *tasks, int ntasks, int TR, int 
     panel_trsm_kernel<T><<<ntasks, 256, smem, st>>>(s, tasks, TR, P, D, mode, tinv, tinv_off, which, getrf, scale_d);
 }
 
-void launch_update_f64(const DevSym &s, const Upd *upds, int nupd, int ntiles, double *L, double *U,
+static int g_f64_grid = 0;  // resident CTAs of update_f64_kernel on the device
+
+void launch_update_f64(const DevSym &s, const Upd *upds, const int2 *tmap, int ntiles, double *L, double *U,
                        cudaStream_t st) {
     if (ntiles <= 0) return;
-    update_f64_kernel<<<ntiles, 128, UPD_F64_SMEM, st>>>(s, upds, nupd, L, U);
+    update_f64_kernel<<<std::min(ntiles, g_f64_grid), 128, UPD_F64_SMEM, st>>>(s, upds, tmap, ntiles, L, U);
 }
 
-void launch_update_f32(const DevSym &s, const Upd *upds, int nupd, int ntiles, float *L, float *U,
+void launch_update_f32(const DevSym &s, const Upd *upds, const int2 *tmap, int ntiles, float *L, float *U,
                        cudaStream_t st) {
     if (ntiles <= 0) return;
-    update_simt_f32_kernel<<<ntiles, 256, 0, st>>>(s, upds, nupd, L, U);
+    update_simt_f32_kernel<<<ntiles, 256, 0, st>>>(s, upds, tmap, L, U);
 }
 
-// Raise the dynamic shared-memory limit of a kernel to what the device allows
-// beyond its static shared memory; returns that limit (bytes) or -1.
 template <typename K>
 static int raise_smem(K kernel) {
     int dev = 0, optin = 0;
@@ -1242,6 +1300,15 @@ int configure_factor_kernels() {
     int lim = 1 << 30;
     int v;
     if ((v = raise_smem(update_f64_kernel)) < UPD_F64_SMEM) return -1;
+    {
+        int dev = 0, sms = 0, occ = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, update_f64_kernel, 128, UPD_F64_SMEM) != cudaSuccess ||
+            occ < 1)
+            return -1;
+        g_f64_grid = occ * sms;
+    }
     if (raise_diag_small_smem<8>() < 0 || raise_diag_small_smem<16>() < 0 || raise_diag_small_smem<32>() < 0)
         return -1;
     if (raise_smem(dag_bottom_kernel<double, FACTO_POTRF>) < 0 || raise_smem(dag_bottom_kernel<double, FACTO_SYTRF>) < 0 ||

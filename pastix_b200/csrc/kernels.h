@@ -52,9 +52,10 @@ void launch_get_diag(const DevSym &s, const T *L, double *out, cudaStream_t st);
 // updates with K <= 16 and N <= 32, one warp each
 template <typename T>
 void launch_update_small(const DevSym &s, const Upd *upds, int nupd, T *L, T *U, cudaStream_t st);
-void launch_update_f64(const DevSym &s, const Upd *upds, int nupd, int ntiles, double *L, double *U,
+// 64 x 64 tiles listed by tmap ({update, row tile | column tile << 16})
+void launch_update_f64(const DevSym &s, const Upd *upds, const int2 *tmap, int ntiles, double *L, double *U,
                        cudaStream_t st);
-void launch_update_f32(const DevSym &s, const Upd *upds, int nupd, int ntiles, float *L, float *U,
+void launch_update_f32(const DevSym &s, const Upd *upds, const int2 *tmap, int ntiles, float *L, float *U,
                        cudaStream_t st);
 // the bottom levels of the tree in one launch (cblks of at most 32 columns): items
 // (factor items, then update items, level by level) taken by warps from *ticket; a

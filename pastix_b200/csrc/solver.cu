@@ -121,6 +121,7 @@ struct b200_solver_s {
     void *dTinv = nullptr;
     void *dWL = nullptr, *dWU = nullptr;
     Upd *d_upd = nullptr;
+    int2 *d_updmap = nullptr;           // 64 x 64 tiles of the d_upd launches, level by level
     std::vector<Level> levels;
     // cblks of each level that go through the one-CTA diagonal kernel (the others take the sub-panel path)
     int *d_diag_list = nullptr;
@@ -324,6 +325,7 @@ int build_schedule(b200_solver_t *s) {
         }
         return true;
     };
+    std::vector<int2> updmap;         // tiles of the 64 x 64 update launches: {update of the level, row | col << 16}
     std::vector<int2> tcmap, tcmapw;  // tile maps of the 64- and 128-column tensor-core launches
     std::vector<Upd> smallupds;
     s->lvl_us0.assign(nlev, 0);
@@ -437,6 +439,12 @@ int build_schedule(b200_solver_t *s) {
         u.N = s->lrow[j] - s->frow[j] + 1;
         u.K = s->ncols[k];
         u.colbase = s->frow[j] - s->fcol[u.f];
+        u.ldk = s->ld[k];
+        u.ldf = s->ld[u.f];
+        u.offA = s->off[k] + u.rowA0;
+        u.offB = s->off[k] + u.rowB0;
+        u.offC = s->off[u.f] + (int64_t)u.colbase * u.ldf;
+        u.offD = s->off[k];
         return true;
     };
     const size_t trsm_smem = (size_t)s->trsm_smem;
@@ -561,6 +569,7 @@ int build_schedule(b200_solver_t *s) {
             }
         }
         L.u0 = (int)upds.size();
+        L.m0 = (int64_t)updmap.size();
         s->lvl_us0[l] = (int)smallupds.size();
         s->lvl_tc_u0[l] = (int)tcupds.size();
         s->lvl_tc_m0[l] = (int)tcmap.size();
@@ -598,10 +607,12 @@ int build_schedule(b200_solver_t *s) {
                     }
                     u.tiles_m = (u.M + 63) / 64;
                     u.tiles_n = (u.N + 63) / 64;
-                    const int nt = (u.flags & UPD_SYM) ? u.tiles_n * u.tiles_m - u.tiles_n * (u.tiles_n - 1) / 2
-                                                       : u.tiles_n * u.tiles_m;
-                    u.tile0 = tile0;
-                    tile0 += nt;
+                    const int ui = (int)upds.size() - L.u0;
+                    for (int nt = 0; nt < u.tiles_n; nt++)
+                        for (int mt = (u.flags & UPD_SYM) ? nt : 0; mt < u.tiles_m; mt++) {
+                            updmap.push_back(make_int2(ui, mt | (nt << 16)));
+                            tile0++;
+                        }
                     s->flops_kind[3] += upd_flops(u);
                     upds.push_back(u);
                 }
@@ -853,6 +864,7 @@ int build_schedule(b200_solver_t *s) {
     s->tinv_elems = tpos;
     RET(s->dupload(&s->d_toff, toff));
     RET(s->dupload(&s->d_upd, upds));
+    RET(s->dupload(&s->d_updmap, updmap));
     RET(s->dupload(&s->d_tcupd, tcupds));
     RET(s->dupload(&s->d_tcmap, tcmap));
     RET(s->dupload(&s->d_tcmapw, tcmapw));
@@ -1099,9 +1111,9 @@ int enqueue_numfact(b200_solver_t *s, cudaStream_t st, Trace *tr = nullptr) {
         }
         if (Lv.ntiles > 0) {
             if (sizeof(T) == 8)
-                launch_update_f64(s->ds, s->d_upd + Lv.u0, Lv.u1 - Lv.u0, Lv.ntiles, (double *)L, (double *)U, st);
+                launch_update_f64(s->ds, s->d_upd + Lv.u0, s->d_updmap + Lv.m0, Lv.ntiles, (double *)L, (double *)U, st);
             else
-                launch_update_f32(s->ds, s->d_upd + Lv.u0, Lv.u1 - Lv.u0, Lv.ntiles, (float *)L, (float *)U, st);
+                launch_update_f32(s->ds, s->d_upd + Lv.u0, s->d_updmap + Lv.m0, Lv.ntiles, (float *)L, (float *)U, st);
             launches++;
         }
         if (tr) tr->end(3, st);
