@@ -898,56 +898,56 @@ __global__ void __launch_bounds__(32 * DS_WARPS) diag_small_kernel(DevSym s, con
     small_trsm_warp<T, FACTO, NB>(s, k, L, U, tile, wl, lane);
 }
 
-// Small GEMM-scatter updates (K <= 16, N <= 32: the bottom levels of the tree,
+// Small GEMM-scatter updates (K <= KB = 8 or 16, N <= 32: the bottom levels of the tree,
 // far below a 64 x 64 tile), one warp each: lane = row of the M-range (32 rows per
 // pass), C[d(i)][colbase + c] -= sum_k A[i][k] (D[k]) B[c][k] for c < N (c <= i when
 // symmetric).  Same operation as the tile kernels (core_zgemmsp_2d2d,
-// kernels/core_zgemmsp.c:396-465).  Each warp waits mostly on its loads, so the
-// launch bounds ask for 4 (FP32) / 3 (FP64) CTAs per SM: 64 / 80 registers, a few
-// bytes of spill, a third to a half more warps in flight.
+// kernels/core_zgemmsp.c:396-465).  Each warp waits mostly on its loads: the update's
+// record carries the operands' places, so that two reads (record, operands) depend on
+// one another and not three, the K <= 8 instance holds half the registers, and the launch
+// bounds ask for 4 (FP32) / 3 (FP64) CTAs per SM (a few bytes of spill at K <= 16).  The
+// 512-system 2D forest's updates: 2.57 -> 1.53 ms; 80^3 27-point, FP32: 2.89 -> 2.11 ms.
 constexpr int US_WARPS = 8;
 
-template <typename T>
-__global__ void __launch_bounds__(32 * US_WARPS, sizeof(T) == 4 ? 4 : 3) update_small_kernel(DevSym s, const Upd *__restrict__ upds, int nupd,
-                                                                     T *L, T *U) {
+template <typename T, int KB>
+__global__ void __launch_bounds__(32 * US_WARPS, KB == 8 ? 5 : sizeof(T) == 4 ? 4 : 3)
+    update_small_kernel(DevSym s, const Upd *__restrict__ upds, int nupd, T *L, T *U) {
     const int lane = threadIdx.x & 31;
     const int ui = blockIdx.x * US_WARPS + (threadIdx.x >> 5);
     if (ui >= nupd) return;
     const Upd u = upds[ui];
-    const int k = u.k, ldk = s.ld[k];
-    const T *Ap = ((u.flags & UPD_A_U) ? U : L) + s.off[k] + u.rowA0 + (size_t)u.colK0 * ldk;
-    const T *Bp = ((u.flags & UPD_B_U) ? U : L) + s.off[k] + u.rowB0 + (size_t)u.colK0 * ldk;
-    const T *Dp = L + s.off[k] + (size_t)u.colK0 * (ldk + 1);
+    const int ldk = u.ldk, ldf = u.ldf;
+    const T *Ap = ((u.flags & UPD_A_U) ? U : L) + u.offA;
+    const T *Bp = ((u.flags & UPD_B_U) ? U : L) + u.offB;
     const bool scale = (u.flags & UPD_SCALE_D) != 0;
     const bool atomic = (u.flags & UPD_ATOMIC) != 0;
     const bool sym = (u.flags & UPD_SYM) != 0;
-    T *C = ((u.flags & UPD_C_U) ? U : L) + s.off[u.f];
-    const int ldf = s.ld[u.f];
-    // B (N x K, N <= 32, K <= 16) with D folded into A: bs[c][q] = B[c][q] in shared
+    T *C = ((u.flags & UPD_C_U) ? U : L) + u.offC;
+    // B (N x K, N <= 32, K <= KB) with D folded into A: bs[c][q] = B[c][q] in shared
     // memory, read by every lane as 128-bit broadcasts
-    __shared__ __align__(16) T bsm[US_WARPS][32][16];
-    T(*bs)[16] = bsm[threadIdx.x >> 5];
+    __shared__ __align__(16) T bsm[US_WARPS][32][KB];
+    T(*bs)[KB] = bsm[threadIdx.x >> 5];
 #pragma unroll
-    for (int q = 0; q < 16; q++) bs[lane][q] = (lane < u.N && q < u.K) ? Bp[lane + (size_t)q * ldk] : (T)0;
-    T dk = (scale && lane < u.K) ? Dp[(size_t)lane * (ldk + 1)] : (T)1;
+    for (int q = 0; q < KB; q++) bs[lane][q] = (lane < u.N && q < u.K) ? Bp[lane + (size_t)q * ldk] : (T)0;
+    T dk = (scale && lane < u.K) ? L[u.offD + (size_t)lane * (ldk + 1)] : (T)1;
     __syncwarp();
     for (int r0 = 0; r0 < u.M; r0 += 32) {
         const int i = r0 + lane;
         const bool in = i < u.M;
-        T a[16];
+        const int d = in ? __ldg(s.rmap + u.rm0 + i) : -1;
+        T a[KB];
 #pragma unroll
-        for (int q = 0; q < 16; q++) {
+        for (int q = 0; q < KB; q++) {
             const T dq = __shfl_sync(0xffffffffu, dk, q);
             a[q] = (in && q < u.K) ? Ap[i + (size_t)q * ldk] * dq : (T)0;
         }
-        const int d = in ? __ldg(s.rmap + u.rm0 + i) : -1;
-        T *crow = C + d + (size_t)u.colbase * ldf;
+        T *crow = C + d;
         for (int c = 0; c < u.N; c++) {
             T acc = 0;
             if constexpr (sizeof(T) == 4) {
                 const float4 *b4 = reinterpret_cast<const float4 *>(bs[c]);
 #pragma unroll
-                for (int h = 0; h < 4; h++) {
+                for (int h = 0; h < KB / 4; h++) {
                     const float4 bq = b4[h];
                     acc += a[4 * h] * bq.x;
                     acc += a[4 * h + 1] * bq.y;
@@ -957,7 +957,7 @@ __global__ void __launch_bounds__(32 * US_WARPS, sizeof(T) == 4 ? 4 : 3) update_
             } else {
                 const double2 *b2 = reinterpret_cast<const double2 *>(bs[c]);
 #pragma unroll
-                for (int h = 0; h < 8; h++) {
+                for (int h = 0; h < KB / 2; h++) {
                     const double2 bq = b2[h];
                     acc += a[2 * h] * bq.x;
                     acc += a[2 * h + 1] * bq.y;
@@ -1146,12 +1146,13 @@ template void launch_get_diag<double>(const DevSym &, const double *, double *, 
 template void launch_get_diag<float>(const DevSym &, const float *, double *, cudaStream_t);
 
 template <typename T>
-void launch_update_small(const DevSym &s, const Upd *upds, int nupd, T *L, T *U, cudaStream_t st) {
-    if (nupd <= 0) return;
-    update_small_kernel<T><<<(nupd + US_WARPS - 1) / US_WARPS, 32 * US_WARPS, 0, st>>>(s, upds, nupd, L, U);
+void launch_update_small(const DevSym &s, const Upd *upds, int n8, int nupd, T *L, T *U, cudaStream_t st) {
+    auto grid = [](int n) { return (unsigned)((n + US_WARPS - 1) / US_WARPS); };
+    if (n8 > 0) update_small_kernel<T, 8><<<grid(n8), 32 * US_WARPS, 0, st>>>(s, upds, n8, L, U);
+    if (nupd > n8) update_small_kernel<T, 16><<<grid(nupd - n8), 32 * US_WARPS, 0, st>>>(s, upds + n8, nupd - n8, L, U);
 }
-template void launch_update_small<double>(const DevSym &, const Upd *, int, double *, double *, cudaStream_t);
-template void launch_update_small<float>(const DevSym &, const Upd *, int, float *, float *, cudaStream_t);
+template void launch_update_small<double>(const DevSym &, const Upd *, int, int, double *, double *, cudaStream_t);
+template void launch_update_small<float>(const DevSym &, const Upd *, int, int, float *, float *, cudaStream_t);
 
 template <typename T, int NB>
 static void launch_diag_small_nb(int facto, const DevSym &s, const int *cblks, int ncblk, T *L, T *U, T *tinv,

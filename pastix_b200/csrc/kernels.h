@@ -49,9 +49,9 @@ int configure_panel_kernels();
 // the diagonal of the factor's diagonal blocks, in the permuted numbering (n doubles)
 template <typename T>
 void launch_get_diag(const DevSym &s, const T *L, double *out, cudaStream_t st);
-// updates with K <= 16 and N <= 32, one warp each
+// updates with K <= 16 and N <= 32, one warp each, the first n8 of them with K <= 8
 template <typename T>
-void launch_update_small(const DevSym &s, const Upd *upds, int nupd, T *L, T *U, cudaStream_t st);
+void launch_update_small(const DevSym &s, const Upd *upds, int n8, int nupd, T *L, T *U, cudaStream_t st);
 // 64 x 64 tiles listed by tmap ({update, row tile | column tile << 16})
 void launch_update_f64(const DevSym &s, const Upd *upds, const int2 *tmap, int ntiles, double *L, double *U,
                        cudaStream_t st);

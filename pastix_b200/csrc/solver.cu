@@ -177,7 +177,7 @@ struct b200_solver_s {
     int2 *d_tcmapw = nullptr;             // 128-column tiles
     int2 *d_tcmap = nullptr;              // tiles of each tensor-core launch: {update, row | col << 16}
     Upd *d_smallupd = nullptr;            // updates with K <= 16, N <= 32 (one warp each)
-    std::vector<int> lvl_us0, lvl_us1;
+    std::vector<int> lvl_us0, lvl_us8, lvl_us1;  // of each level: K <= 8, then the others
     std::vector<char> tc_wanted;          // cblks whose panels the tensor-core updates read
     std::vector<int64_t> toff;            // operand copy of cblk k: row-major, pitch ncols rounded up to 16 bytes
     int64_t tsize = 0;                    // elements of one operand arena
@@ -329,7 +329,9 @@ int build_schedule(b200_solver_t *s) {
     std::vector<int2> tcmap, tcmapw;  // tile maps of the 64- and 128-column tensor-core launches
     std::vector<Upd> smallupds;
     s->lvl_us0.assign(nlev, 0);
+    s->lvl_us8.assign(nlev, 0);
     s->lvl_us1.assign(nlev, 0);
+    std::vector<Upd> small16;  // the level's K > 8
     std::vector<SplitTask> splits;
     std::vector<char> ext_wanted(N, 0);   // cblks with external tensor-core updates
     s->lvl_sp0.assign(nlev, 0);
@@ -602,7 +604,7 @@ int build_schedule(b200_solver_t *s) {
                     if (!map_rows(u)) return ERR_NOTIMPL;
                     if (u.K <= 16 && u.N <= 32) {
                         s->flops_kind[3] += upd_flops(u);
-                        smallupds.push_back(u);
+                        (u.K <= 8 ? smallupds : small16).push_back(u);
                         continue;
                     }
                     u.tiles_m = (u.M + 63) / 64;
@@ -620,6 +622,9 @@ int build_schedule(b200_solver_t *s) {
         }
         L.u1 = (int)upds.size();
         L.ntiles = tile0;
+        s->lvl_us8[l] = (int)smallupds.size();
+        smallupds.insert(smallupds.end(), small16.begin(), small16.end());
+        small16.clear();
         s->lvl_us1[l] = (int)smallupds.size();
         s->lvl_tc_u1[l] = (int)tcupds.size();
         s->lvl_tc_tiles[l] = tc_tile0;
@@ -1106,8 +1111,9 @@ int enqueue_numfact(b200_solver_t *s, cudaStream_t st, Trace *tr = nullptr) {
         }
         if (tr) tr->begin(st);
         if (s->lvl_us1[l] > s->lvl_us0[l]) {
-            launch_update_small<T>(s->ds, s->d_smallupd + s->lvl_us0[l], s->lvl_us1[l] - s->lvl_us0[l], L, U, st);
-            launches++;
+            const int n8 = s->lvl_us8[l] - s->lvl_us0[l], nu = s->lvl_us1[l] - s->lvl_us0[l];
+            launch_update_small<T>(s->ds, s->d_smallupd + s->lvl_us0[l], n8, nu, L, U, st);
+            launches += (n8 > 0) + (nu > n8);
         }
         if (Lv.ntiles > 0) {
             if (sizeof(T) == 8)
