@@ -21,16 +21,23 @@ __device__ __forceinline__ int panel_row_to_global(const DevSym &s, int k, int p
     return s.prow[s.rbase[k] + prow];
 }
 
+// one warp per cblk, lane = row (a CTA per cblk took 0.19 ms for the 232 K cblks of a
+// 512-system forest, most of them 4 to 8 columns wide; this, 0.09)
+constexpr int SCALE_WARPS = 8;
+
 template <typename T, typename V>
-__global__ void solve_scale_diag_kernel(DevSym s, const int *__restrict__ cblks, const T *__restrict__ L, V *x,
-                                        int64_t ldx, int nrhs) {
-    const int k = cblks[blockIdx.x];
+__global__ void __launch_bounds__(32 * SCALE_WARPS) solve_scale_diag_kernel(DevSym s, const int *__restrict__ cblks,
+                                                                            int ncblk, const T *__restrict__ L, V *x,
+                                                                            int64_t ldx, int nrhs) {
+    const int ci = blockIdx.x * SCALE_WARPS + (threadIdx.x >> 5);
+    if (ci >= ncblk) return;
+    const int k = cblks[ci];
     const int n = s.ncols[k], ld = s.ld[k];
     const T *D = L + s.off[k];
     V *xk = x + s.fcol[k];
-    for (int idx = threadIdx.x; idx < n * nrhs; idx += blockDim.x) {
-        const int i = idx % n, r = idx / n;
-        xk[i + (size_t)r * ldx] /= (V)D[(size_t)i * (ld + 1)];
+    for (int i = threadIdx.x & 31; i < n; i += 32) {
+        const V d = (V)D[(size_t)i * (ld + 1)];
+        for (int r = 0; r < nrhs; r++) xk[i + (size_t)r * ldx] /= d;
     }
 }
 
@@ -56,7 +63,8 @@ template <typename T, typename V>
 void launch_solve_scale_diag(const DevSym &s, const int *cblks, int ncblk, const T *L, V *x, int64_t ldx, int nrhs,
                              cudaStream_t st) {
     if (ncblk <= 0) return;
-    solve_scale_diag_kernel<T, V><<<ncblk, 128, 0, st>>>(s, cblks, L, x, ldx, nrhs);
+    solve_scale_diag_kernel<T, V>
+        <<<(ncblk + SCALE_WARPS - 1) / SCALE_WARPS, 32 * SCALE_WARPS, 0, st>>>(s, cblks, ncblk, L, x, ldx, nrhs);
 }
 
 void launch_permute(int n, int nrhs, const int *peri, const double *src, int64_t lds, double *dst, int64_t ldd,
@@ -362,13 +370,13 @@ __global__ void __launch_bounds__(128) solve_mm_kernel(DevSym s, const SolveTile
 // W_k is the inverse of the diagonal block (n x n, column-major), P the cblk panel.
 constexpr int LEAF_R = 16;  // right-hand sides per pass
 
-template <typename T, typename V>
+template <typename T, typename V, int LR>
 __global__ void __launch_bounds__(128) solve_leaf_kernel(DevSym s, const int *__restrict__ cblks, int ncblk,
                                                          const T *__restrict__ P, const T *__restrict__ W,
                                                          const int64_t *__restrict__ woff, V *x, V *aux,
                                                          int64_t ldx, int nrhs, int backward) {
-    __shared__ V ys[4][32][LEAF_R + 1];
-    __shared__ V xr[4][32][LEAF_R + 1];
+    __shared__ V ys[4][32][LR + 1];
+    __shared__ V xr[4][32][LR + 1];
     __shared__ int gr[4][32];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ci = blockIdx.x * 4 + w;
@@ -377,28 +385,28 @@ __global__ void __launch_bounds__(128) solve_leaf_kernel(DevSym s, const int *__
     const int n = s.ncols[k], ld = s.ld[k], stride = s.stride[k], f0 = s.fcol[k];
     const T *Pk = P + s.off[k];
     const T *Wk = W + woff[k];
-    for (int q0 = 0; q0 < nrhs; q0 += LEAF_R) {
-        const int R = min(LEAF_R, nrhs - q0);
+    for (int q0 = 0; q0 < nrhs; q0 += LR) {
+        const int R = min(LR, nrhs - q0);
         if (!backward) {
 #pragma unroll
-            for (int j = 0; j < LEAF_R; j++)
+            for (int j = 0; j < LR; j++)
                 ys[w][lane][j] = (lane < n && j < R) ? x[f0 + lane + (size_t)(q0 + j) * ldx] : (V)0;
             __syncwarp();
-            V y[LEAF_R];
+            V y[LR];
 #pragma unroll
-            for (int j = 0; j < LEAF_R; j++) y[j] = 0;
+            for (int j = 0; j < LR; j++) y[j] = 0;
             if (lane < n) {
 #pragma unroll 4
                 for (int c = 0; c <= lane; c++) {
                     const V wv = (V)Wk[lane + (size_t)c * n];
 #pragma unroll
-                    for (int j = 0; j < LEAF_R; j++) y[j] += wv * ys[w][c][j];
+                    for (int j = 0; j < LR; j++) y[j] += wv * ys[w][c][j];
                 }
             }
             __syncwarp();
             if (lane < n) {
 #pragma unroll
-                for (int j = 0; j < LEAF_R; j++) {
+                for (int j = 0; j < LR; j++) {
                     ys[w][lane][j] = y[j];
                     if (j < R) aux[f0 + lane + (size_t)(q0 + j) * ldx] = y[j];
                 }
@@ -406,31 +414,31 @@ __global__ void __launch_bounds__(128) solve_leaf_kernel(DevSym s, const int *__
             __syncwarp();
             for (int r = n + lane; r < stride; r += 32) {
                 const int g = panel_row_to_global(s, k, r);
-                V acc[LEAF_R];
+                V acc[LR];
 #pragma unroll
-                for (int j = 0; j < LEAF_R; j++) acc[j] = 0;
+                for (int j = 0; j < LR; j++) acc[j] = 0;
 #pragma unroll 4
                 for (int c = 0; c < n; c++) {
                     const V pv = (V)Pk[r + (size_t)c * ld];
 #pragma unroll
-                    for (int j = 0; j < LEAF_R; j++) acc[j] += pv * ys[w][c][j];
+                    for (int j = 0; j < LR; j++) acc[j] += pv * ys[w][c][j];
                 }
 #pragma unroll
-                for (int j = 0; j < LEAF_R; j++)
+                for (int j = 0; j < LR; j++)
                     if (j < R) atomicAdd(&x[g + (size_t)(q0 + j) * ldx], -acc[j]);
             }
             __syncwarp();
         } else {
-            V t[LEAF_R];
+            V t[LR];
 #pragma unroll
-            for (int j = 0; j < LEAF_R; j++) t[j] = (lane < n && j < R) ? aux[f0 + lane + (size_t)(q0 + j) * ldx] : (V)0;
+            for (int j = 0; j < LR; j++) t[j] = (lane < n && j < R) ? aux[f0 + lane + (size_t)(q0 + j) * ldx] : (V)0;
             for (int r0 = n; r0 < stride; r0 += 32) {
                 const int nr = min(32, stride - r0);
                 gr[w][lane] = (lane < nr) ? panel_row_to_global(s, k, r0 + lane) : 0;
                 __syncwarp();
                 // stage x of the 32 rows: xr[i][j] = x[grow(r0 + i)][q0 + j]
-                for (int idx = lane; idx < 32 * LEAF_R; idx += 32) {
-                    const int i = idx / LEAF_R, j = idx % LEAF_R;
+                for (int idx = lane; idx < 32 * LR; idx += 32) {
+                    const int i = idx / LR, j = idx % LR;
                     xr[w][i][j] = (i < nr && j < R) ? x[gr[w][i] + (size_t)(q0 + j) * ldx] : (V)0;
                 }
                 __syncwarp();
@@ -439,27 +447,27 @@ __global__ void __launch_bounds__(128) solve_leaf_kernel(DevSym s, const int *__
                     for (int i = 0; i < nr; i++) {
                         const V pv = (V)Pk[r0 + i + (size_t)lane * ld];
 #pragma unroll
-                        for (int j = 0; j < LEAF_R; j++) t[j] -= pv * xr[w][i][j];
+                        for (int j = 0; j < LR; j++) t[j] -= pv * xr[w][i][j];
                     }
                 }
                 __syncwarp();
             }
             if (lane < n) {
 #pragma unroll
-                for (int j = 0; j < LEAF_R; j++) ys[w][lane][j] = t[j];
+                for (int j = 0; j < LR; j++) ys[w][lane][j] = t[j];
             }
             __syncwarp();
             if (lane < n) {
-                V o[LEAF_R];
+                V o[LR];
 #pragma unroll
-                for (int j = 0; j < LEAF_R; j++) o[j] = 0;
+                for (int j = 0; j < LR; j++) o[j] = 0;
                 for (int r = lane; r < n; r++) {
                     const V wv = (V)Wk[r + (size_t)lane * n];
 #pragma unroll
-                    for (int j = 0; j < LEAF_R; j++) o[j] += wv * ys[w][r][j];
+                    for (int j = 0; j < LR; j++) o[j] += wv * ys[w][r][j];
                 }
 #pragma unroll
-                for (int j = 0; j < LEAF_R; j++)
+                for (int j = 0; j < LR; j++)
                     if (j < R) x[f0 + lane + (size_t)(q0 + j) * ldx] = o[j];
             }
             __syncwarp();
@@ -467,11 +475,101 @@ __global__ void __launch_bounds__(128) solve_leaf_kernel(DevSym s, const int *__
     }
 }
 
+// One right-hand side: the same products with everything in registers.  Forward, lane =
+// row; backward the column sums of 32 panel rows at a time, lane = row, met by a
+// reduction over the warp (column c in lane c).  The kernel above spent the padding of
+// 16 right-hand sides and its shared memory on one: 0.33 ms for the 103 K leaves of a
+// 512-system forest.
+constexpr int LEAF1_WARPS = 8;
+
+// v[c] summed over the warp, returned in lane c (c < NB, NB a power of two)
+template <int NB, typename V>
+__device__ __forceinline__ V reduce_columns(V (&v)[NB], int lane) {
+#pragma unroll
+    for (int h = NB / 2; h > 0; h >>= 1) {
+        const bool up = lane & h;
+#pragma unroll
+        for (int i = 0; i < h; i++) {
+            const V send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+        }
+    }
+    V r = v[0];
+#pragma unroll
+    for (int h = NB; h < 32; h <<= 1) r += __shfl_xor_sync(0xffffffffu, r, h);
+    return r;
+}
+
+template <int NB, typename T, typename V>
+__device__ __forceinline__ V leaf1_columns(const DevSym &s, int k, int n, int ld, int stride, const T *Pk, const V *x,
+                                           int lane) {
+    V acc[NB];
+#pragma unroll
+    for (int c = 0; c < NB; c++) acc[c] = 0;
+    for (int r = n + lane; r < stride; r += 32) {
+        const V xv = x[panel_row_to_global(s, k, r)];
+#pragma unroll
+        for (int c = 0; c < NB; c++)
+            if (c < n) acc[c] += (V)Pk[r + (size_t)c * ld] * xv;
+    }
+    return reduce_columns<NB>(acc, lane);
+}
+
+template <typename T, typename V>
+__global__ void __launch_bounds__(32 * LEAF1_WARPS) solve_leaf1_kernel(DevSym s, const int *__restrict__ cblks,
+                                                                       int ncblk, const T *__restrict__ P,
+                                                                       const T *__restrict__ W,
+                                                                       const int64_t *__restrict__ woff, V *x, V *aux,
+                                                                       int backward) {
+    const int lane = threadIdx.x & 31, ci = blockIdx.x * LEAF1_WARPS + (threadIdx.x >> 5);
+    if (ci >= ncblk) return;
+    const int k = cblks[ci];
+    const int n = s.ncols[k], ld = s.ld[k], stride = s.stride[k], f0 = s.fcol[k];
+    const T *Pk = P + s.off[k], *Wk = W + woff[k];
+    if (!backward) {
+        const V xv = lane < n ? x[f0 + lane] : (V)0;
+        V y = 0;
+        for (int c = 0; c < n; c++) {
+            const V xc = __shfl_sync(0xffffffffu, xv, c);
+            if (lane < n && c <= lane) y += (V)Wk[lane + (size_t)c * n] * xc;
+        }
+        if (lane < n) aux[f0 + lane] = y;
+        for (int r0 = n; r0 < stride; r0 += 32) {
+            const int r = r0 + lane;
+            V acc = 0;
+#pragma unroll 4
+            for (int c = 0; c < n; c++) {
+                const V yc = __shfl_sync(0xffffffffu, y, c);
+                if (r < stride) acc += (V)Pk[r + (size_t)c * ld] * yc;
+            }
+            if (r < stride) atomicAdd(x + panel_row_to_global(s, k, r), -acc);
+        }
+    } else {
+        V t = lane < n ? aux[f0 + lane] : (V)0;
+        t -= n <= 8 ? leaf1_columns<8>(s, k, n, ld, stride, Pk, x, lane)
+                    : n <= 16 ? leaf1_columns<16>(s, k, n, ld, stride, Pk, x, lane)
+                              : leaf1_columns<32>(s, k, n, ld, stride, Pk, x, lane);
+        V o = 0;
+        for (int r = 0; r < n; r++) {
+            const V tr = __shfl_sync(0xffffffffu, t, r);
+            if (lane <= r) o += (V)Wk[r + (size_t)lane * n] * tr;
+        }
+        if (lane < n) x[f0 + lane] = o;
+    }
+}
+
 template <typename T, typename V>
 void launch_solve_leaf(const DevSym &s, const int *cblks, int ncblk, const T *P, const T *W, const int64_t *woff,
                        V *x, V *aux, int64_t ldx, int nrhs, int backward, cudaStream_t st) {
     if (ncblk <= 0) return;
-    solve_leaf_kernel<T, V><<<(ncblk + 3) / 4, 128, 0, st>>>(s, cblks, ncblk, P, W, woff, x, aux, ldx, nrhs, backward);
+    const int grid = (ncblk + 3) / 4;
+    if (nrhs == 1)
+        solve_leaf1_kernel<T, V><<<(ncblk + LEAF1_WARPS - 1) / LEAF1_WARPS, 32 * LEAF1_WARPS, 0, st>>>(
+            s, cblks, ncblk, P, W, woff, x, aux, backward);
+    else if (nrhs <= 4)
+        solve_leaf_kernel<T, V, 4><<<grid, 128, 0, st>>>(s, cblks, ncblk, P, W, woff, x, aux, ldx, nrhs, backward);
+    else
+        solve_leaf_kernel<T, V, LEAF_R><<<grid, 128, 0, st>>>(s, cblks, ncblk, P, W, woff, x, aux, ldx, nrhs, backward);
 }
 template void launch_solve_leaf<double, double>(const DevSym &, const int *, int, const double *, const double *,
                                                 const int64_t *, double *, double *, int64_t, int, int, cudaStream_t);
