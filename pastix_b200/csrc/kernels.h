@@ -99,10 +99,14 @@ void launch_solve_tiles(const DevSym &s, const SolveTile *tasks, int ntasks, con
 template <typename T, typename V>
 void launch_solve_leaf(const DevSym &s, const int *cblks, int ncblk, const T *P, const T *W, const int64_t *woff,
                        V *x, V *aux, int64_t ldx, int nrhs, int backward, cudaStream_t st);
-// W_k = inverse of the lower-triangular diagonal block of every listed cblk (W: n x n per cblk)
+// W_k = inverse of the lower-triangular diagonal block of cblks of more than 32 columns
+// (W: n x n per cblk), for LU (U, WU given) of both sides: tiles lists their 32-column
+// diagonal blocks {k, first column}, strips their 16-column strips that have blocks below
+// the diagonal one; nmax: the widest; unit: the L side has a unit diagonal
 template <typename T>
-void launch_diag_inverse(const DevSym &s, const int *cblks, int ncblk, const T *L, T *W, const int64_t *woff,
-                         int unit, cudaStream_t st);
+void launch_diag_inverse(const DevSym &s, const RowTask *tiles, int ntiles, const RowTask *strips, int nstrips,
+                         int nmax, const T *L, const T *U, T *WL, T *WU, const int64_t *woff, int unit,
+                         cudaStream_t st);
 // W_k of cblks with at most 32 columns, copied from the diagonal kernel's tile inverses (which: 0 L, 1 U^T)
 template <typename T>
 void launch_copy_tile_inverse(const DevSym &s, const int *cblks, int ncblk, const T *tinv, const int64_t *toff, T *W,

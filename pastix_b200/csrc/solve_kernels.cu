@@ -979,120 +979,165 @@ template void launch_solve_flow<float, float>(const DevSym &, const FlowItem *, 
 
 // ====================================================================== diagonal-block inverses
 //
-// W_k = T_k^{-1} for the lower-triangular diagonal block T_k of every cblk
-// (L_kk, unit for LDL^T and LU; for the backward sweep of LU the stored U_kk^T).
-// With W the diagonal solves of both sweeps are plain products, computed on
-// tensor cores like the off-diagonal tiles, instead of a chain of dependent
-// 32-column steps per cblk.  One CTA per cblk, 8 warps:
-//   phase 1: every 32x32 diagonal tile inverted by one warp (row per lane);
-//   phase 2: block column j of W by one warp: W_ij = -W_ii sum_{j<=m<i} T_im W_mj.
+// W_k = T_k^{-1} for the lower-triangular diagonal block T_k of every cblk of more than
+// 32 columns (L_kk, unit for LDL^T and LU; for the backward sweep of LU the stored
+// U_kk^T).  With W the diagonal solves of both sweeps are plain products, computed on
+// tensor cores like the off-diagonal tiles, instead of a chain of dependent 32-column
+// steps per cblk.  Two launches over 32 x 32 blocks, in double whatever the factor's type:
+//   inverse_tiles_kernel : every diagonal block inverted by one warp, the blocks above it
+//                          zeroed;
+//   inverse_strips_kernel: 16 columns of W per CTA, block row by block row, W_i = -W_ii
+//                          sum_{j <= m < i} T_im W_m on the FP64 tensor cores, the strip
+//                          so far in shared memory.
+// The strips are independent, so a single wide cblk keeps 2 CTAs per block column busy
+// and a level's many run side by side: one CTA per cblk took 0.15 ms for the five wide
+// cblks of a 20^3 tree and 1.6 ms for the two sides of a 64^3 LU.
 namespace b200 {
 
 constexpr int INV_WARPS = 4;
 constexpr int DIAG_INV_SMEM = INV_WARPS * 2 * 32 * TP * sizeof(double);
 
-// W_k = T_k^{-1} for the lower-triangular diagonal block T_k of every listed cblk
-// (L_kk, unit for LDL^T and LU; for the backward sweep of LU the stored U_kk^T).
-// With W the diagonal solves of both sweeps are plain products on tensor cores.
-// One CTA of 4 warps per cblk, 32 x 32 blocks:
-//   phase 1: every diagonal block inverted by one warp (invert_lower_tile);
-//   phase 2: block rows in order, the blocks of a row in parallel over the warps:
-//            W_ij = -W_ii sum_{j <= m < i} T_im W_mj, each product from shared-memory
-//            copies of T_im and W_mj staged with all loads in flight.
 template <typename T>
-__global__ void __launch_bounds__(128, 3) diag_inverse_kernel(DevSym s, const int *__restrict__ cblks,
-                                                           const T *__restrict__ Lsrc, T *W,
-                                                           const int64_t *__restrict__ woff, int unit) {
+__global__ void __launch_bounds__(32 * INV_WARPS) inverse_tiles_kernel(DevSym s, const RowTask *__restrict__ tasks,
+                                                                      int ntasks, const T *__restrict__ L,
+                                                                      const T *__restrict__ U, T *WL, T *WU,
+                                                                      const int64_t *__restrict__ woff, int unit) {
     extern __shared__ __align__(16) double inv_smem[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double *ta = inv_smem + warp * 2 * 32 * TP;
     double *tb = ta + 32 * TP;
-    const int k = cblks[blockIdx.x];
-    const int n = s.ncols[k], ld = s.ld[k];
-    const T *Tk = Lsrc + s.off[k];
-    T *Wk = W + woff[k];
-    const int nb = (n + 31) / 32;
-    // phase 1: diagonal blocks; the blocks above them are zero
-    for (int b = warp; b < nb; b += INV_WARPS) {
-        const int b0 = b * 32, bw = min(32, n - b0);
-        stage_n<32, double>(
-            [&](int j) {
-                return (lane < bw && j < bw && lane >= j) ? (double)Tk[(b0 + lane) + (size_t)(b0 + j) * ld] : 0.0;
-            },
-            [&](int j, double v) { ta[lane + j * TP] = v; });
-        __syncwarp();
-        invert_lower_tile<double>(ta, tb, bw, lane, unit, 0);
-        for (int idx = lane; idx < 32 * bw; idx += 32) {
-            const int i = idx & 31, j = idx >> 5;
-            if (i < bw) Wk[(b0 + i) + (size_t)(b0 + j) * n] = (T)tb[i + j * TP];
-        }
-        for (int idx = lane; idx < b0 * bw; idx += 32) {
-            const int i = idx % b0, j = idx / b0;
-            Wk[i + (size_t)(b0 + j) * n] = (T)0;
-        }
-        __syncwarp();
+    const int ti = blockIdx.x * INV_WARPS + warp;
+    if (ti >= ntasks) return;
+    const int k = tasks[ti].k, b0 = tasks[ti].row0, side = blockIdx.y;
+    const int n = s.ncols[k], ld = s.ld[k], bw = min(32, n - b0);
+    const T *Tk = (side ? U : L) + s.off[k];
+    T *Wk = (side ? WU : WL) + woff[k];
+    stage_n<32, double>(
+        [&](int j) {
+            return (lane < bw && j < bw && lane >= j) ? (double)Tk[(b0 + lane) + (size_t)(b0 + j) * ld] : 0.0;
+        },
+        [&](int j, double v) { ta[lane + j * TP] = v; });
+    __syncwarp();
+    invert_lower_tile<double>(ta, tb, bw, lane, unit && side == 0, 0);
+    for (int idx = lane; idx < 32 * bw; idx += 32) {
+        const int i = idx & 31, j = idx >> 5;
+        if (i < bw) Wk[(b0 + i) + (size_t)(b0 + j) * n] = (T)tb[i + j * TP];
     }
-    __syncthreads();
-    // phase 2
-    for (int bi = 1; bi < nb; bi++) {
-        const int i0 = bi * 32, iw = min(32, n - i0);
-        for (int bj = warp; bj < bi; bj += INV_WARPS) {
-            const int j0 = bj * 32, jw = min(32, n - j0);
-            double acc[32];
-#pragma unroll
-            for (int j = 0; j < 32; j++) acc[j] = 0.0;
-            for (int bm = bj; bm < bi; bm++) {
-                const int m0 = bm * 32, mw = min(32, n - m0);
-                stage_n<32, double>(
-                    [&](int j) {
-                        return (lane < iw && j < mw) ? (double)Tk[(i0 + lane) + (size_t)(m0 + j) * ld] : 0.0;
-                    },
-                    [&](int j, double v) { ta[lane + j * TP] = v; });
-                stage_n<32, double>(
-                    [&](int j) { return (lane < mw && j < jw) ? (double)Wk[(m0 + lane) + (size_t)(j0 + j) * n] : 0.0; },
-                    [&](int j, double v) { tb[lane + j * TP] = v; });
-                __syncwarp();
-#pragma unroll 4
-                for (int m = 0; m < 32; m++) {
-                    const double tv = ta[lane + m * TP];
-#pragma unroll
-                    for (int j = 0; j < 32; j++) acc[j] += tv * tb[m + j * TP];
-                }
-                __syncwarp();
-            }
-            // W_ij = -W_ii acc (W_ii written in phase 1)
-            stage_n<32, double>(
-                [&](int j) {
-                    return (lane < iw && j < iw && lane >= j) ? (double)Wk[(i0 + lane) + (size_t)(i0 + j) * n] : 0.0;
-                },
-                [&](int j, double v) { tb[lane + j * TP] = v; });
-#pragma unroll
-            for (int j = 0; j < 32; j++) ta[lane + j * TP] = acc[j];
-            __syncwarp();
-            if (lane < iw) {
-                double out[32];
-#pragma unroll
-                for (int j = 0; j < 32; j++) out[j] = 0.0;
-                for (int l = 0; l <= lane; l++) {
-                    const double wv = tb[lane + l * TP];
-#pragma unroll
-                    for (int j = 0; j < 32; j++) out[j] -= wv * ta[l + j * TP];
-                }
-#pragma unroll
-                for (int j = 0; j < 32; j++)
-                    if (j < jw) Wk[(i0 + lane) + (size_t)(j0 + j) * n] = (T)out[j];
-            }
-            __syncwarp();
-        }
-        __syncthreads();
+    for (int j = 0; j < bw; j++)
+        for (int i = lane; i < b0; i += 32) Wk[i + (size_t)(b0 + j) * n] = (T)0;
+}
+
+constexpr int IS_COLS = 16;    // columns of a strip
+constexpr int IS_PITCH = 36;   // pitch of a staged 32 x 32 block (column-major)
+constexpr int IS_WP = 20;      // pitch of the strip's rows: conflict-free B fragments
+constexpr int IS_STAGES = 3;
+constexpr int is_smem(int rows, int esz) {
+    return (rows + 32) * IS_WP * (int)sizeof(double) + IS_STAGES * 32 * IS_PITCH * esz;
+}
+
+// Task {k, first column of the strip}.  Steps: for every block row i below the strip's own,
+// the products with blocks T_ij .. T_i,i-1, then with W_ii; their blocks come through a
+// 3-stage cp.async pipeline.  Warp (wr, wc): rows 16 wr .., columns 8 wc .. of a product.
+template <typename T>
+__global__ void __launch_bounds__(128) inverse_strips_kernel(DevSym s, const RowTask *__restrict__ tasks,
+                                                             const T *__restrict__ L, const T *__restrict__ U, T *WL,
+                                                             T *WU, const int64_t *__restrict__ woff, int rows_max) {
+    extern __shared__ __align__(16) double is_mem[];
+    double *ws = is_mem;                          // the strip's rows from its own block row on
+    double *ss = ws + (size_t)rows_max * IS_WP;   // the sum of a block row
+    T *st = reinterpret_cast<T *>(ss + 32 * IS_WP);
+    const int k = tasks[blockIdx.x].k, j0 = tasks[blockIdx.x].row0, side = blockIdx.y;
+    const int n = s.ncols[k], ld = s.ld[k], nb = (n + 31) / 32, bd = j0 / 32, jw = min(IS_COLS, n - j0);
+    const T *Tk = (side ? U : L) + s.off[k];
+    T *Wk = (side ? WU : WL) + woff[k];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wr = warp & 1, wc = warp >> 1, g = lane >> 2, tg = lane & 3;
+    // own block row: the columns of W_dd
+    const int dw = min(32, n - 32 * bd);
+    for (int idx = tid; idx < 32 * IS_COLS; idx += 128) {
+        const int r = idx & 31, c = idx >> 5;
+        ws[r * IS_WP + c] = (r < dw && c < jw) ? (double)Wk[32 * bd + r + (size_t)(j0 + c) * n] : 0.0;
     }
+    // blocks in step order: block row li, block column lm (lm == li: W_ii)
+    int li = bd + 1, lm = bd;
+    auto load = [&](int q) {
+        if (li < nb) {
+            const int iw = min(32, n - 32 * li);
+            const bool wii = lm == li;
+            const T *src = wii ? Wk + 32 * li + (size_t)(32 * li) * n : Tk + 32 * li + (size_t)(32 * lm) * ld;
+            const size_t lds = wii ? n : ld;
+            T *dst = st + q * 32 * IS_PITCH;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int r = lane, c = warp + 4 * u;
+                const bool ok = r < iw && (!wii || (c < iw && r >= c));
+                cp_async_el(dst + c * IS_PITCH + r, ok ? src + r + (size_t)c * lds : Tk, ok);
+            }
+            if (++lm > li) {
+                li++;
+                lm = bd;
+            }
+        }
+        cp_commit();
+    };
+    load(0);
+    load(1);
+    int q = 0;
+    for (int bi = bd + 1; bi < nb; bi++) {
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int m = bd; m <= bi; m++) {
+            cp_wait<1>();
+            if (m == bi) {
+                // the block row's sum, for the product with W_ii
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    ss[(wr * 16 + g + (e >> 1) * 8) * IS_WP + wc * 8 + 2 * tg + (e & 1)] = acc[e];
+                    acc[e] = 0.0;
+                }
+            }
+            __syncthreads();
+            load(q + 2 >= IS_STAGES ? q + 2 - IS_STAGES : q + 2);
+            const T *a = st + q * 32 * IS_PITCH;
+            const double *bsrc = m == bi ? ss : ws + (size_t)(32 * (m - bd)) * IS_WP;
+#pragma unroll
+            for (int kk = 0; kk < 32; kk += 16) {
+                double av[8], bv[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int kq = kk + 4 * j + tg;
+                    av[2 * j] = (double)a[kq * IS_PITCH + wr * 16 + g];
+                    av[2 * j + 1] = (double)a[kq * IS_PITCH + wr * 16 + g + 8];
+                    bv[j] = bsrc[kq * IS_WP + wc * 8 + g];
+                }
+                dmma16x8x16(acc, av, bv);
+            }
+            q = q + 1 == IS_STAGES ? 0 : q + 1;
+        }
+        double *wrow = ws + (size_t)(32 * (bi - bd)) * IS_WP;
+        const int iw = min(32, n - 32 * bi);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int r = wr * 16 + g + (e >> 1) * 8, c = wc * 8 + 2 * tg + (e & 1);
+            wrow[r * IS_WP + c] = -acc[e];
+            if (r < iw && c < jw) Wk[32 * bi + r + (size_t)(j0 + c) * n] = (T)-acc[e];
+        }
+        // (the next block row's first barrier covers wrow)
+    }
+    cp_wait<0>();
 }
 
 template <typename T>
-void launch_diag_inverse(const DevSym &s, const int *cblks, int ncblk, const T *L, T *W, const int64_t *woff,
-                         int unit, cudaStream_t st) {
-    if (ncblk <= 0) return;
-    diag_inverse_kernel<T><<<ncblk, 32 * INV_WARPS, DIAG_INV_SMEM, st>>>(s, cblks, L, W, woff, unit);
+void launch_diag_inverse(const DevSym &s, const RowTask *tiles, int ntiles, const RowTask *strips, int nstrips,
+                         int nmax, const T *L, const T *U, T *WL, T *WU, const int64_t *woff, int unit,
+                         cudaStream_t st) {
+    if (ntiles <= 0) return;
+    const unsigned sides = U ? 2 : 1;
+    inverse_tiles_kernel<T><<<dim3((ntiles + INV_WARPS - 1) / INV_WARPS, sides), 32 * INV_WARPS, DIAG_INV_SMEM, st>>>(
+        s, tiles, ntiles, L, U, WL, WU, woff, unit);
+    if (nstrips <= 0) return;
+    const int rows = (nmax + 31) / 32 * 32;
+    inverse_strips_kernel<T><<<dim3(nstrips, sides), 128, is_smem(rows, sizeof(T)), st>>>(s, strips, L, U, WL, WU, woff,
+                                                                                        rows);
 }
 
 template <typename T, typename V>
@@ -1105,17 +1150,23 @@ void launch_solve_diag_inv(const DevSym &s, const SolveTile *tasks, int ntasks, 
 
 int configure_inverse_kernels() {
     int rc = configure_solve_mm<double, double>() | configure_solve_mm<float, float>();
-    rc |= (int)cudaFuncSetAttribute(diag_inverse_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    rc |= (int)cudaFuncSetAttribute(inverse_tiles_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     DIAG_INV_SMEM);
-    rc |= (int)cudaFuncSetAttribute(diag_inverse_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    rc |= (int)cudaFuncSetAttribute(inverse_tiles_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     DIAG_INV_SMEM);
+    // the widest cblk the library takes: 1024 columns
+    rc |= (int)cudaFuncSetAttribute(inverse_strips_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    is_smem(1024, sizeof(double)));
+    rc |= (int)cudaFuncSetAttribute(inverse_strips_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    is_smem(1024, sizeof(float)));
     return rc == 0 ? 0 : -1;
 }
 
-template void launch_diag_inverse<double>(const DevSym &, const int *, int, const double *, double *, const int64_t *,
-                                          int, cudaStream_t);
-template void launch_diag_inverse<float>(const DevSym &, const int *, int, const float *, float *, const int64_t *,
-                                         int, cudaStream_t);
+template void launch_diag_inverse<double>(const DevSym &, const RowTask *, int, const RowTask *, int, int,
+                                          const double *, const double *, double *, double *, const int64_t *, int,
+                                          cudaStream_t);
+template void launch_diag_inverse<float>(const DevSym &, const RowTask *, int, const RowTask *, int, int, const float *,
+                                         const float *, float *, float *, const int64_t *, int, cudaStream_t);
 template void launch_solve_diag_inv<double, double>(const DevSym &, const SolveTile *, int, const double *,
                                                     const int64_t *, const double *, double *, int64_t, int, int,
                                                     cudaStream_t);

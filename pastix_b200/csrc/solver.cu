@@ -125,8 +125,9 @@ struct b200_solver_s {
     std::vector<Level> levels;
     // cblks of each level that go through the one-CTA diagonal kernel (the others take the sub-panel path)
     int *d_diag_list = nullptr;
-    int *d_inv_small = nullptr, *d_inv_big = nullptr;  // cblks of <= 32 / > 32 columns
-    int n_inv_small = 0, n_inv_big = 0;
+    int *d_inv_small = nullptr;                        // cblks of <= 32 columns
+    RowTask *d_inv_tile = nullptr, *d_inv_strip = nullptr;  // diagonal blocks and strips of the wider ones
+    int n_inv_small = 0, n_inv_tile = 0, n_inv_strip = 0, inv_nmax = 0;
     std::vector<int> lvl_ds0, lvl_ds1;
     std::vector<int> lvl_dsm0, lvl_dsm1;  // cblks of <= 32 columns (one warp each)
     std::vector<int> lvl_dsm8, lvl_dsm16; // ends of their <= 8 and <= 16 column classes
@@ -836,14 +837,24 @@ int build_schedule(b200_solver_t *s) {
     RET(s->dupload(&s->d_diag_list, diag_list));
     {
         std::vector<int> small, big;
-        for (int k = 0; k < cs; k++) (s->ncols[k] <= 32 && !is_big(k) ? small : big).push_back(k);
-        // widest first: their inverses take the longest, so they start before the many
-        // narrow ones instead of forming the launch's tail
-        std::stable_sort(big.begin(), big.end(), [&](int a, int b) { return s->ncols[a] > s->ncols[b]; });
+        for (int k = 0; k < cs; k++) (s->ncols[k] <= 32 ? small : big).push_back(k);
+        // the strips with the most blocks below them first, so that they do not form the
+        // launch's tail
+        std::vector<RowTask> tiles, strips;
+        for (int k : big) {
+            s->inv_nmax = std::max(s->inv_nmax, s->ncols[k]);
+            for (int c = 0; c < s->ncols[k]; c += 32) tiles.push_back({k, c});
+            for (int c = 0; c < (s->ncols[k] - 1) / 32 * 32; c += 16) strips.push_back({k, c});
+        }
+        auto below = [&](const RowTask &t) { return (s->ncols[t.k] + 31) / 32 - t.row0 / 32; };
+        std::stable_sort(strips.begin(), strips.end(),
+                         [&](const RowTask &x, const RowTask &y) { return below(x) > below(y); });
         s->n_inv_small = (int)small.size();
-        s->n_inv_big = (int)big.size();
+        s->n_inv_tile = (int)tiles.size();
+        s->n_inv_strip = (int)strips.size();
         RET(s->dupload(&s->d_inv_small, small));
-        RET(s->dupload(&s->d_inv_big, big));
+        RET(s->dupload(&s->d_inv_tile, tiles));
+        RET(s->dupload(&s->d_inv_strip, strips));
     }
     RET(s->dupload(&s->d_pcb, pcbs));
     RET(s->dupload(&s->d_pitem, pitems));
@@ -1142,13 +1153,13 @@ int enqueue_numfact(b200_solver_t *s, cudaStream_t st, Trace *tr = nullptr) {
     if (tr) tr->begin(st);
     launch_copy_tile_inverse<T>(s->ds, s->d_inv_small, s->n_inv_small, (const T *)s->dTinv, s->d_toff, (T *)s->dWL,
                                 s->d_woff, 0, st);
-    launch_diag_inverse<T>(s->ds, s->d_inv_big, s->n_inv_big, L, (T *)s->dWL, s->d_woff, s->facto != FACTO_POTRF, st);
-    launches += 2;
+    launch_diag_inverse<T>(s->ds, s->d_inv_tile, s->n_inv_tile, s->d_inv_strip, s->n_inv_strip, s->inv_nmax, L, U,
+                           (T *)s->dWL, (T *)s->dWU, s->d_woff, s->facto != FACTO_POTRF, st);
+    launches += (s->n_inv_small > 0) + (s->n_inv_tile > 0) + (s->n_inv_strip > 0);
     if (s->facto == FACTO_GETRF) {
         launch_copy_tile_inverse<T>(s->ds, s->d_inv_small, s->n_inv_small, (const T *)s->dTinv, s->d_toff,
                                     (T *)s->dWU, s->d_woff, 1, st);
-        launch_diag_inverse<T>(s->ds, s->d_inv_big, s->n_inv_big, U, (T *)s->dWU, s->d_woff, 0, st);
-        launches += 2;
+        launches += s->n_inv_small > 0;
     }
     if (tr) tr->end(5, st);
     CU(cudaGetLastError());
