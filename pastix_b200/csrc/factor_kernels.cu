@@ -1,9 +1,9 @@
 // Numerical factorization kernels (sm_100a).
 //
 //  scatter_kernel      bcsc -> panel arena (cpucblk_zfillin_fr, kernels/cpucblk_zinit.c:229-309)
-//  diag_factor_kernel  per-cblk diagonal-block POTRF / GETRF / SYTRF with static pivoting
+//  diag_lu_kernel      diagonal block of a wide LU cblk that the panel launch does not take
 //                      (core_z{potrf,getrf,sytrf}sp, kernels/core_z*trfsp.c)
-//  panel_trsm_kernel   off-diagonal panel solve (core_ztrsmsp_2d, kernels/core_ztrsmsp.c:147-181)
+//  lu_trsm_kernel      its off-diagonal panel solve (core_ztrsmsp_2d, kernels/core_ztrsmsp.c:147-181)
 //  update_f64_kernel   GEMM + scatter-add into the facing cblk on FP64 tensor cores (DMMA)
 //                      (core_zgemmsp_2d2d, kernels/core_zgemmsp.c:396-465)
 //  update_simt_kernel  the same update for FP32 factors on CUDA cores
@@ -130,9 +130,8 @@ __device__ void factor_tile(T *t, int pb, int lane, double thr, int *piv, int *e
     __syncwarp();
 }
 
-// 32x32 output tile of a trailing update, computed by one warp:
-// C[i][j] -= sum_c X[i][c] * B(j, c) for c < pb, where X(i, c) = A[(r0+i) + (p+c) ld]
-// and B(j, c) = A[(c0+j) + (p+c) ld] (btrans = 0) or A[(p+c) + (c0+j) ld] (btrans = 1).
+// 32x32 output tile of a trailing LU update, computed by one warp:
+// A[r0 + i][c0 + j] -= sum_c A[r0 + i][p + c] A[p + c][c0 + j] for c < pb.
 __device__ __forceinline__ void dmma_tile(double (&c)[4], double a0, double a1, double b) {
     asm volatile(
         "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
@@ -140,8 +139,7 @@ __device__ __forceinline__ void dmma_tile(double (&c)[4], double a0, double a1, 
         : "d"(a0), "d"(a1), "d"(b));
 }
 
-__device__ void warp_tile_update(double *A, int ld, int n, int p, int pb, int r0, int c0, int btrans, int lower_only,
-                                 int lane, double *) {
+__device__ void warp_tile_update(double *A, int ld, int n, int p, int pb, int r0, int c0, int lane, double *) {
     const int g = lane >> 2, tg = lane & 3;
     double acc[2][4][4];
 #pragma unroll
@@ -163,7 +161,7 @@ __device__ void warp_tile_update(double *A, int ld, int n, int p, int pb, int r0
 #pragma unroll
         for (int ni = 0; ni < 4; ni++) {
             const int j = c0 + ni * 8 + g;
-            b[ni] = (okc && j < n) ? (btrans ? A[(p + c) + (size_t)j * ld] : A[j + (size_t)(p + c) * ld]) : 0.0;
+            b[ni] = (okc && j < n) ? A[(p + c) + (size_t)j * ld] : 0.0;
         }
 #pragma unroll
         for (int mi = 0; mi < 2; mi++)
@@ -178,17 +176,16 @@ __device__ void warp_tile_update(double *A, int ld, int n, int p, int pb, int r0
             for (int e = 0; e < 4; e++) {
                 const int i = r0 + mi * 16 + g + (e >> 1) * 8;
                 const int j = c0 + ni * 8 + 2 * tg + (e & 1);
-                if (i < n && j < n && (!lower_only || i >= j)) A[i + (size_t)j * ld] -= acc[mi][ni][e];
+                if (i < n && j < n) A[i + (size_t)j * ld] -= acc[mi][ni][e];
             }
 }
 
 // FP32 version: lane i owns row r0+i of the tile; B staged in per-warp shared memory.
-__device__ void warp_tile_update(float *A, int ld, int n, int p, int pb, int r0, int c0, int btrans, int lower_only,
-                                 int lane, float *bs) {
+__device__ void warp_tile_update(float *A, int ld, int n, int p, int pb, int r0, int c0, int lane, float *bs) {
     for (int idx = lane; idx < 32 * 32; idx += 32) {
         const int j = idx & 31, c = idx >> 5;
         float v = 0.0f;
-        if (c < pb && c0 + j < n) v = btrans ? A[(p + c) + (size_t)(c0 + j) * ld] : A[(c0 + j) + (size_t)(p + c) * ld];
+        if (c < pb && c0 + j < n) v = A[(p + c) + (size_t)(c0 + j) * ld];
         bs[c * 33 + j] = v;
     }
     __syncwarp();
@@ -205,50 +202,39 @@ __device__ void warp_tile_update(float *A, int ld, int n, int p, int pb, int r0,
 #pragma unroll
         for (int j = 0; j < 32; j++) {
             const int jj = c0 + j;
-            if (jj < n && (!lower_only || i >= jj)) A[i + (size_t)jj * ld] -= acc[j];
+            if (jj < n) A[i + (size_t)jj * ld] -= acc[j];
         }
     }
     __syncwarp();
 }
 
-// One CTA (256 threads) factors the diagonal block of one cblk, blocked by 32
-// columns.  Per panel: warp 0 factors the 32x32 diagonal tile in registers and then
-// inverts it (warp 1 inverts the upper triangle for LU); the rows (and, for LU,
-// columns) below the tile inside the diagonal block are solved as products with
-// those inverses; every warp then updates its own 32x32 tiles of the trailing
-// block (FP64 tensor cores for double).  The tile inverses are also stored in
-// tinv for the panel TRSM.  For LU the diagonal block of the U arena is first
-// added transposed into L (core_zgeadd) and afterwards receives the transposed
-// factor (core_zgetmo).  At most 128 registers per thread, so that two CTAs share an
-// SM: the levels of many 33-96 column cblks are latency-bound, and the second CTA's
-// warps cover the first one's single-warp tile steps (the spills this costs are
-// cheaper than the idle SMs).
-template <typename T, int FACTO>
-__global__ void __launch_bounds__(256, 2) diag_factor_kernel(DevSym s, const int *__restrict__ cblks, T *L,
-                                                          T *U, T *tinv, const int64_t *__restrict__ tinv_off,
-                                                          const double *__restrict__ thr_ptr,
-                                                          unsigned long long *npiv, int *err) {
+// Wide LU cblks whose row blocks do not fit in the shared memory of the panel launch:
+// one CTA (256 threads) factors the diagonal block of one cblk, blocked by 32 columns.
+// Per panel: warp 0 factors the 32x32 diagonal tile in registers; the rows and columns
+// beside the tile inside the diagonal block are solved by substitution in the
+// reference's order; every warp then updates its own 32x32 tiles of the trailing block
+// (FP64 tensor cores for double).  The diagonal block of the U arena is first added
+// transposed into L (core_zgeadd) and afterwards receives the transposed factor
+// (core_zgetmo).
+template <typename T>
+__global__ void __launch_bounds__(256, 2) diag_lu_kernel(DevSym s, const int *__restrict__ cblks, T *L, T *U,
+                                                         const double *__restrict__ thr_ptr,
+                                                         unsigned long long *npiv, int *err) {
     __shared__ T tile[32 * TP];
-    __shared__ T wl[32 * TP];
-    __shared__ T wu[32 * TP];
     extern __shared__ __align__(16) float diag_wbuf[];  // FP32 only: per-warp 32x33 staging
     __shared__ int s_piv, s_err;
     const int k = cblks[blockIdx.x];
     const int n = s.ncols[k], ld = s.ld[k];
     const double thr = cblk_threshold(s, thr_ptr, k);
-    T *A = L + s.off[k];
-    T *ti = tinv + tinv_off[k];
+    T *A = L + s.off[k], *Au = U + s.off[k];
     const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) { s_piv = 0; s_err = 0; }
-    if (FACTO == FACTO_GETRF) {
-        const T *Au = U + s.off[k];
-        for (int idx = tid; idx < n * n; idx += nth) {
-            const int i = idx % n, j = idx / n;
-            A[i + (size_t)j * ld] += Au[j + (size_t)i * ld];
-        }
+    for (int idx = tid; idx < n * n; idx += nth) {
+        const int i = idx % n, j = idx / n;
+        A[i + (size_t)j * ld] += Au[j + (size_t)i * ld];
     }
     __syncthreads();
-    for (int p = 0, pi = 0; p < n; p += 32, pi++) {
+    for (int p = 0; p < n; p += 32) {
         const int pb = min(32, n - p);
         T *Ap = A + p + (size_t)p * ld;
         for (int idx = tid; idx < 32 * 32; idx += nth) {
@@ -256,112 +242,61 @@ __global__ void __launch_bounds__(256, 2) diag_factor_kernel(DevSym s, const int
             tile[i + j * TP] = (i < pb && j < pb) ? Ap[i + (size_t)j * ld] : (T)0;
         }
         __syncthreads();
-        if (warp == 0) factor_tile<T, FACTO>(tile, pb, lane, thr, &s_piv, &s_err);
+        if (warp == 0) factor_tile<T, FACTO_GETRF>(tile, pb, lane, thr, &s_piv, &s_err);
         __syncthreads();
-        if (warp == 0) invert_lower_tile<T>(tile, wl, pb, lane, FACTO != FACTO_POTRF, 0);
-        if (FACTO == FACTO_GETRF && warp == 1) invert_lower_tile<T>(tile, wu, pb, lane, 0, 1);  // inv(U^T)
-        __syncthreads();
-        // store the factored tile and its inverse(s)
         for (int idx = tid; idx < 32 * 32; idx += nth) {
             const int i = idx & 31, j = idx >> 5;
-            if (i < pb && j < pb && (FACTO != FACTO_POTRF || i >= j)) Ap[i + (size_t)j * ld] = tile[i + j * TP];
-            // panel pi of the tile-inverse store: 32 x pb, after pi full panels (two per panel for LU)
-            if (j < pb) {
-                T *tp = ti + (size_t)pi * 1024 * (FACTO == FACTO_GETRF ? 2 : 1);
-                tp[i + j * 32] = wl[i + j * TP];
-                if (FACTO == FACTO_GETRF) tp[32 * pb + i + j * 32] = wu[i + j * TP];
-            }
+            if (i < pb && j < pb) Ap[i + (size_t)j * ld] = tile[i + j * TP];
         }
         const int rest = n - p - pb;
         if (rest > 0) {
-            // rows below the tile: X = A op(T)^{-1}; Cholesky with the tile inverse,
-            // LU / LDL^T by substitution in the reference's order (indefinite or
-            // badly scaled tiles)
+            // rows below the tile: X U = A
             for (int r = tid; r < rest; r += nth) {
                 T *row = A + (p + pb + r) + (size_t)p * ld;
                 T a[32];
 #pragma unroll
                 for (int c = 0; c < 32; c++) a[c] = (c < pb) ? row[(size_t)c * ld] : (T)0;
-                if (FACTO == FACTO_POTRF) {
 #pragma unroll
-                    for (int c = 0; c < 32; c++) {
-                        if (c < pb) {
-                            // X = A L^{-T}: (L^{-T})[l][c] = inv(L)[c][l]
-                            T v = 0;
+                for (int c = 0; c < 32; c++) {
+                    if (c < pb) {
+                        T v = a[c];
 #pragma unroll
-                            for (int l = 0; l <= c; l++) v += a[l] * wl[c + l * TP];
-                            row[(size_t)c * ld] = v;
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 32; c++) {
-                        if (c < pb) {
-                            T v = a[c];
-#pragma unroll
-                            for (int l = 0; l < c; l++) {
-                                // GETRF: X U = A with U = the upper part; LDL^T: V L^T = A, unit L
-                                const T u = (FACTO == FACTO_GETRF) ? tile[l + c * TP] : tile[c + l * TP];
-                                v -= a[l] * u;
-                            }
-                            if (FACTO == FACTO_GETRF) v /= tile[c * (TP + 1)];
-                            a[c] = v;
-                            if (FACTO == FACTO_SYTRF) {
-                                A[(p + c) + (size_t)(p + pb + r) * ld] = v;          // (L D)^T in the upper part
-                                row[(size_t)c * ld] = v * ((T)1 / tile[c * (TP + 1)]);  // L
-                            } else {
-                                row[(size_t)c * ld] = v;
-                            }
-                        }
+                        for (int l = 0; l < c; l++) v -= a[l] * tile[l + c * TP];
+                        v /= tile[c * (TP + 1)];
+                        a[c] = v;
+                        row[(size_t)c * ld] = v;
                     }
                 }
             }
-            if (FACTO == FACTO_GETRF) {
-                // columns right of the tile: Y = L_tile^{-1} A (unit lower), by substitution
-                for (int cc = tid; cc < rest; cc += nth) {
-                    T *col = A + p + (size_t)(p + pb + cc) * ld;
-                    T a[32];
+            // columns right of the tile: Y = L_tile^{-1} A (unit lower)
+            for (int cc = tid; cc < rest; cc += nth) {
+                T *col = A + p + (size_t)(p + pb + cc) * ld;
+                T a[32];
 #pragma unroll
-                    for (int l = 0; l < 32; l++) a[l] = (l < pb) ? col[l] : (T)0;
+                for (int l = 0; l < 32; l++) a[l] = (l < pb) ? col[l] : (T)0;
 #pragma unroll
-                    for (int l = 0; l < 32; l++) {
-                        if (l < pb) {
-                            T v = a[l];
+                for (int l = 0; l < 32; l++) {
+                    if (l < pb) {
+                        T v = a[l];
 #pragma unroll
-                            for (int m = 0; m < l; m++) v -= tile[l + m * TP] * a[m];
-                            a[l] = v;
-                            col[l] = v;
-                        }
+                        for (int m = 0; m < l; m++) v -= tile[l + m * TP] * a[m];
+                        a[l] = v;
+                        col[l] = v;
                     }
                 }
             }
             __syncthreads();
             // trailing update, one 32x32 tile per warp at a time
             const int nt = (rest + 31) / 32;
-            const int ntiles = (FACTO == FACTO_GETRF) ? nt * nt : nt * (nt + 1) / 2;
-            for (int t = warp; t < ntiles; t += 8) {
-                int ti_, tj_;
-                if (FACTO == FACTO_GETRF) {
-                    ti_ = t % nt;
-                    tj_ = t / nt;
-                } else {
-                    tj_ = 0;
-                    int rem = t;
-                    while (rem >= nt - tj_) { rem -= nt - tj_; tj_++; }
-                    ti_ = tj_ + rem;
-                }
-                warp_tile_update(A, ld, n, p, pb, p + pb + ti_ * 32, p + pb + tj_ * 32, FACTO != FACTO_POTRF,
-                                 FACTO != FACTO_GETRF, lane, reinterpret_cast<T *>(diag_wbuf) + warp * 32 * 33);
-            }
+            for (int t = warp; t < nt * nt; t += 8)
+                warp_tile_update(A, ld, n, p, pb, p + pb + t % nt * 32, p + pb + t / nt * 32, lane,
+                                 reinterpret_cast<T *>(diag_wbuf) + warp * 32 * 33);
         }
         __syncthreads();
     }
-    if (FACTO == FACTO_GETRF) {
-        T *Au = U + s.off[k];
-        for (int idx = tid; idx < n * n; idx += nth) {
-            const int i = idx % n, j = idx / n;
-            Au[j + (size_t)i * ld] = A[i + (size_t)j * ld];
-        }
+    for (int idx = tid; idx < n * n; idx += nth) {
+        const int i = idx % n, j = idx / n;
+        Au[j + (size_t)i * ld] = A[i + (size_t)j * ld];
     }
     if (tid == 0) {
         if (s_piv) atomicAdd(cblk_pivot_counter(s, npiv, k), (unsigned long long)s_piv);
@@ -371,15 +306,13 @@ __global__ void __launch_bounds__(256, 2) diag_factor_kernel(DevSym s, const int
 
 // ------------------------------------------------------------------ panel TRSM
 
-// X op(T) = B for a tile of TR off-diagonal rows of cblk k, the whole tile held
-// in shared memory.  op(T) is upper triangular:
-//   mode 0: op(T)[l][c] = D[l + c*ld]  (upper part of the diagonal block)
-//   mode 1: op(T)[l][c] = D[c + l*ld]  (lower part, transposed)
+// X op(T) = B for a tile of TR off-diagonal rows of a wide LU cblk (diag_lu_kernel's), the
+// whole tile held in shared memory, by substitution in the order of PaStiX's TRSM.  op(T)
+// is the upper triangle of the diagonal block (side 0, rows of L) or the transposed unit
+// lower one (side 1, rows of the stored U^T).
 template <typename T>
-__global__ void __launch_bounds__(256) panel_trsm_kernel(DevSym s, const RowTask *__restrict__ tasks, int TR,
-                                                         T *P, const T *Dsrc, int mode, const T *__restrict__ tinv,
-                                                         const int64_t *__restrict__ tinv_off, int which, int getrf,
-                                                         int scale_d) {
+__global__ void __launch_bounds__(256) lu_trsm_kernel(DevSym s, const RowTask *__restrict__ tasks, int TR, T *P,
+                                                      const T *Dsrc, int side) {
     extern __shared__ __align__(16) unsigned char smraw[];
     T *xs = reinterpret_cast<T *>(smraw);  // TR x n, column-major
     __shared__ T ts[64 * TP];
@@ -408,7 +341,7 @@ __global__ void __launch_bounds__(256) panel_trsm_kernel(DevSym s, const RowTask
             for (int idx = tid; idx < 64 * 32; idx += nth) {
                 const int l = idx >> 5, c = idx & 31;
                 T v = 0;
-                if (l < lw && c < w) v = mode == 0 ? D[(l0 + l) + (size_t)(cb + c) * ld] : D[(cb + c) + (size_t)(l0 + l) * ld];
+                if (l < lw && c < w) v = side == 0 ? D[(l0 + l) + (size_t)(cb + c) * ld] : D[(cb + c) + (size_t)(l0 + l) * ld];
                 ts[l * TP + c] = v;
             }
             __syncthreads();
@@ -425,58 +358,19 @@ __global__ void __launch_bounds__(256) panel_trsm_kernel(DevSym s, const RowTask
             const int c = cg * CPG + q;
             if (q < CPG && c < w) xs[r + (cb + c) * TR] -= acc[q];
         }
-        if (!getrf && !scale_d) {
-        // multiplier of this column block: M(l, c) = W[c][l] (W = the stored tile
-        // inverse of the Cholesky factor)
-        {
-            const T *W = tinv + tinv_off[k] + (size_t)(cb >> 5) * 1024 * (getrf ? 2 : 1) + (which ? 32 * w : 0);
-            for (int idx = tid; idx < 32 * 32; idx += nth) {
-                const int l = idx >> 5, c = idx & 31;
-                T v = 0;
-                if (l < w && c < w && c >= l) {
-                    v = W[c + l * 32];
-                    if (scale_d) v = v / D[(size_t)(cb + c) * (ld + 1)];
-                }
-                tt[l * TP + c] = v;
-            }
+        for (int idx = tid; idx < 32 * 32; idx += nth) {
+            const int l = idx >> 5, c = idx & 31;
+            T v = 0;
+            if (l < w && c < w && c >= l)
+                v = side == 0 ? D[(cb + l) + (size_t)(cb + c) * ld] : D[(cb + c) + (size_t)(cb + l) * ld];
+            tt[l * TP + c] = v;
         }
         __syncthreads();
-        {
-            T out[8];
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                out[q] = 0;
-                const int c = cg * CPG + q;
-                if (q < CPG && c < w)
-                    for (int l = 0; l <= c; l++) out[q] += xs[r + (cb + l) * TR] * tt[l * TP + c];
-            }
-            __syncthreads();
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const int c = cg * CPG + q;
-                if (q < CPG && c < w) xs[r + (cb + c) * TR] = out[q];
-            }
-        }
-        } else {
-            // LU and LDL^T: substitution against the upper triangular block
-            // U(l, c) = op(T)[cb + l][cb + c] (LDL^T: D L^T; the U-side LU panel has a
-            // unit diagonal), the order of PaStiX's TRSM, which keeps indefinite or
-            // badly scaled diagonal blocks as accurate as the reference
-            for (int idx = tid; idx < 32 * 32; idx += nth) {
-                const int l = idx >> 5, c = idx & 31;
-                T v = 0;
-                if (l < w && c < w && c >= l)
-                    v = mode == 0 ? D[(cb + l) + (size_t)(cb + c) * ld] : D[(cb + c) + (size_t)(cb + l) * ld];
-                tt[l * TP + c] = v;
-            }
-            __syncthreads();
-            const bool unit = getrf && which == 0;
-            if (tid < TR) {
-                for (int c = 0; c < w; c++) {
-                    T x = xs[tid + (cb + c) * TR];
-                    for (int l = 0; l < c; l++) x -= xs[tid + (cb + l) * TR] * tt[l * TP + c];
-                    xs[tid + (cb + c) * TR] = unit ? x : x / tt[c * TP + c];
-                }
+        if (tid < TR) {
+            for (int c = 0; c < w; c++) {
+                T x = xs[tid + (cb + c) * TR];
+                for (int l = 0; l < c; l++) x -= xs[tid + (cb + l) * TR] * tt[l * TP + c];
+                xs[tid + (cb + c) * TR] = side ? x : x / tt[c * TP + c];
             }
         }
         __syncthreads();
@@ -486,9 +380,6 @@ __global__ void __launch_bounds__(256) panel_trsm_kernel(DevSym s, const RowTask
         if (rr < rows) X[rr + (size_t)c * ld] = xs[idx];
     }
 }
-
-
-
 
 // ------------------------------------------------------------------ updates
 
@@ -871,7 +762,7 @@ __device__ __forceinline__ void small_diag_warp(const DevSym &s, int k, T *L, T 
 }
 
 // Cblks with at most 32 columns, one warp per cblk (the bottom levels of the tree
-// hold tens of thousands): the single-panel case of diag_factor_kernel -- geadd of
+// hold tens of thousands): static pivoting, geadd of
 // U^T for LU, factor_tile, the tile inverse(s), write-back (and U^T for LU) -- and
 // the panel solve of the rows below (small_trsm_warp), so that these cblks need no
 // TRSM launch.  One instance per width class NB (8, 16, 32 columns): the narrow
@@ -1237,24 +1128,20 @@ int dag_bottom_grid(int facto, bool f32, int ncblk) {
 }
 
 template <typename T>
-void launch_diag(int facto, const DevSym &s, const int *cblks, int ncblk, T *L, T *U, T *tinv,
-                 const int64_t *tinv_off, const double *thr, unsigned long long *npiv, int *err, cudaStream_t st) {
+void launch_diag_lu(const DevSym &s, const int *cblks, int ncblk, T *L, T *U, const double *thr,
+                    unsigned long long *npiv, int *err, cudaStream_t st) {
     if (ncblk <= 0) return;
     const size_t smem = (sizeof(T) == 4) ? 8 * 32 * 33 * sizeof(float) : 0;
-    if (facto == FACTO_POTRF)
-        diag_factor_kernel<T, FACTO_POTRF><<<ncblk, 256, smem, st>>>(s, cblks, L, U, tinv, tinv_off, thr, npiv, err);
-    else if (facto == FACTO_GETRF)
-        diag_factor_kernel<T, FACTO_GETRF><<<ncblk, 256, smem, st>>>(s, cblks, L, U, tinv, tinv_off, thr, npiv, err);
-    else
-        diag_factor_kernel<T, FACTO_SYTRF><<<ncblk, 256, smem, st>>>(s, cblks, L, U, tinv, tinv_off, thr, npiv, err);
+    diag_lu_kernel<T><<<ncblk, 256, smem, st>>>(s, cblks, L, U, thr, npiv, err);
 }
 
 template <typename T>
-void launch_trsm(const DevSym &s, const RowTask *tasks, int ntasks, int TR, int nmax, T *P, const T *D, int mode,
-                 const T *tinv, const int64_t *tinv_off, int which, int getrf, int scale_d, cudaStream_t st) {
+void launch_lu_trsm(const DevSym &s, const RowTask *tasks, int ntasks, int TR, int nmax, T *L, T *U,
+                    cudaStream_t st) {
     if (ntasks <= 0) return;
     const size_t smem = (size_t)TR * nmax * sizeof(T);
-    panel_trsm_kernel<T><<<ntasks, 256, smem, st>>>(s, tasks, TR, P, D, mode, tinv, tinv_off, which, getrf, scale_d);
+    lu_trsm_kernel<T><<<ntasks, 256, smem, st>>>(s, tasks, TR, L, L, 0);
+    lu_trsm_kernel<T><<<ntasks, 256, smem, st>>>(s, tasks, TR, U, L, 1);
 }
 
 static int g_f64_grid = 0;  // resident CTAs of update_f64_kernel on the device
@@ -1316,9 +1203,9 @@ int configure_factor_kernels() {
         raise_smem(dag_bottom_kernel<double, FACTO_GETRF>) < 0 || raise_smem(dag_bottom_kernel<float, FACTO_POTRF>) < 0 ||
         raise_smem(dag_bottom_kernel<float, FACTO_SYTRF>) < 0 || raise_smem(dag_bottom_kernel<float, FACTO_GETRF>) < 0)
         return -1;
-    if ((v = raise_smem(panel_trsm_kernel<double>)) < 0) return -1;
+    if ((v = raise_smem(lu_trsm_kernel<double>)) < 0) return -1;
     lim = std::min(lim, v);
-    if ((v = raise_smem(panel_trsm_kernel<float>)) < 0) return -1;
+    if ((v = raise_smem(lu_trsm_kernel<float>)) < 0) return -1;
     lim = std::min(lim, v);
     return lim;
 }
@@ -1327,13 +1214,11 @@ template void launch_scatter<double>(int64_t, const int64_t *, const double *, c
                                      cudaStream_t);
 template void launch_scatter<float>(int64_t, const int64_t *, const double *, const double *, float *, float *,
                                     cudaStream_t);
-template void launch_diag<double>(int, const DevSym &, const int *, int, double *, double *, double *,
-                                  const int64_t *, const double *, unsigned long long *, int *, cudaStream_t);
-template void launch_diag<float>(int, const DevSym &, const int *, int, float *, float *, float *, const int64_t *,
-                                 const double *, unsigned long long *, int *, cudaStream_t);
-template void launch_trsm<double>(const DevSym &, const RowTask *, int, int, int, double *, const double *, int,
-                                  const double *, const int64_t *, int, int, int, cudaStream_t);
-template void launch_trsm<float>(const DevSym &, const RowTask *, int, int, int, float *, const float *, int,
-                                 const float *, const int64_t *, int, int, int, cudaStream_t);
+template void launch_diag_lu<double>(const DevSym &, const int *, int, double *, double *, const double *,
+                                     unsigned long long *, int *, cudaStream_t);
+template void launch_diag_lu<float>(const DevSym &, const int *, int, float *, float *, const double *,
+                                    unsigned long long *, int *, cudaStream_t);
+template void launch_lu_trsm<double>(const DevSym &, const RowTask *, int, int, int, double *, double *, cudaStream_t);
+template void launch_lu_trsm<float>(const DevSym &, const RowTask *, int, int, int, float *, float *, cudaStream_t);
 
 }  // namespace b200

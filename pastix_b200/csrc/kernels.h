@@ -11,22 +11,23 @@ namespace b200 {
 template <typename T>
 void launch_scatter(int64_t nnz, const int64_t *dest, const double *Lv, const double *Uv, T *L, T *U,
                     cudaStream_t st);
-// tinv: per cblk 32 x ncols (x2 for LU) tile inverses written by the diagonal kernel, read by the TRSM
+// wide LU cblks that the panel launch does not take: diagonal blocks, then the rows below
+// (both sides), TR rows per task
 template <typename T>
-void launch_diag(int facto, const DevSym &s, const int *cblks, int ncblk, T *L, T *U, T *tinv,
-                 const int64_t *tinv_off, const double *thr, unsigned long long *npiv, int *err, cudaStream_t st);
-// the same for cblks of at most nb (8, 16 or 32) columns, one warp per cblk, with the
-// panel solve of their rows below (no TRSM task for them)
+void launch_diag_lu(const DevSym &s, const int *cblks, int ncblk, T *L, T *U, const double *thr,
+                    unsigned long long *npiv, int *err, cudaStream_t st);
+template <typename T>
+void launch_lu_trsm(const DevSym &s, const RowTask *tasks, int ntasks, int TR, int nmax, T *L, T *U,
+                    cudaStream_t st);
+// tinv: per cblk 32 x ncols (x2 for LU) tile inverses, the diagonal-block inverses of the
+// cblks of at most 32 columns
+// cblks of at most nb (8, 16 or 32) columns, one warp per cblk: diagonal block, its inverse
+// and the panel solve of the rows below
 template <typename T>
 void launch_diag_small(int facto, const DevSym &s, const int *cblks, int ncblk, int nb, T *L, T *U, T *tinv,
                        const int64_t *tinv_off, const double *thr, unsigned long long *npiv, int *err,
                        cudaStream_t st);
-// X op(T) = B: mode 0 upper / 1 lower-transposed for the left-looking part; which = 0 (inv L) or 1 (inv U^T)
-// selects the tile inverse; scale_d divides by D (LDL^T)
-template <typename T>
-void launch_trsm(const DevSym &s, const RowTask *tasks, int ntasks, int TR, int nmax, T *P, const T *D, int mode,
-                 const T *tinv, const int64_t *tinv_off, int which, int getrf, int scale_d, cudaStream_t st);
-// every wide POTRF / LDL^T cblk of a level in one launch (panel_kernels.cu): items
+// every wide cblk of a level in one launch (panel_kernels.cu): items
 // taken in order from *ticket, dependencies through the solved / updated counters
 // (zeroed before the factorization, like *ticket and *abort_word)
 template <typename T>

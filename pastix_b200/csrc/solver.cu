@@ -123,7 +123,7 @@ struct b200_solver_s {
     Upd *d_upd = nullptr;
     int2 *d_updmap = nullptr;           // 64 x 64 tiles of the d_upd launches, level by level
     std::vector<Level> levels;
-    // cblks of each level that go through the one-CTA diagonal kernel (the others take the sub-panel path)
+    // LU cblks of each level that go through the one-CTA diagonal kernel, then the one-warp classes
     int *d_diag_list = nullptr;
     int *d_inv_small = nullptr;                        // cblks of <= 32 columns
     RowTask *d_inv_tile = nullptr, *d_inv_strip = nullptr;  // diagonal blocks and strips of the wider ones
@@ -190,7 +190,7 @@ struct b200_solver_s {
     std::vector<int> lvl_tr;            // TRSM rows per task of each level
     int nmax_all = 0;
     int64_t total_tiles = 0;
-    int trsm_smem = 0;                  // dynamic shared memory available to the panel TRSM
+    int trsm_smem = 0;                  // dynamic shared memory available to the LU panel solve
     double flops_class[4] = {0, 0, 0, 0};  // algorithmic flops per kernel class (see Trace)
     double flops_kind[9] = {};             // algorithmic flops of the kinds 3 (updates), 4 (panels), 6 (TC updates),
                                            // 8 (the tree-bottom launch's updates)
@@ -399,8 +399,13 @@ int build_schedule(b200_solver_t *s) {
     s->lvl_pi1.assign(nlev, 0);
     s->lvl_prows.assign(nlev, 0);
     s->lvl_pns.assign(nlev, 0);
-    // wider cblks take the panel launch (LU only in its row-block form, while that fits)
-    const int split_min = 96;
+    // cblks of more than 32 columns take the panel launch (LU only in its row-block form,
+    // while that fits: at most 384 columns in FP64, 832 in FP32).  Up to 96 columns they had
+    // a one-CTA diagonal kernel and a panel solve of their own: with the line at 96, 64, 48
+    // and 32 columns the factorization takes 1.18, 0.90, 0.92 and 0.84 ms at 20^3 FP64, 4.95,
+    // 4.82, 4.86 and 4.57 ms for the 37x30x41 LU, 20.37, 19.90, 19.91 and 19.79 ms at 80^3
+    // 27-point split BF16, 3.50, 3.46, 3.33 and 3.15 ms for a 512-system 2D forest
+    const int split_min = 32;
     auto is_big = [&](int k) {
         if (s->ncols[k] <= split_min) return false;
         return s->facto != FACTO_GETRF ||
@@ -469,8 +474,8 @@ int build_schedule(b200_solver_t *s) {
         s->lvl_st0[l] = (int)stile.size();
         s->lvl_dt0[l] = (int)dtask.size();
         s->lvl_db0[l] = (int)dtaskb.size();
-        // diagonal blocks: <= 32 columns by the one-warp kernel, up to the sub-panel
-        // width by the one-CTA kernel
+        // diagonal blocks: <= 32 columns by the one-warp kernel, LU's that the panel launch
+        // does not take by the one-CTA kernel
         s->lvl_ds0[l] = (int)diag_list.size();
         for (int i = L.c0; i < L.c1; i++)
             if (!is_big(lvl_cblk[i]) && s->ncols[lvl_cblk[i]] > 32) diag_list.push_back(lvl_cblk[i]);
@@ -1074,8 +1079,11 @@ int enqueue_numfact(b200_solver_t *s, cudaStream_t st, Trace *tr = nullptr) {
     for (size_t l = (size_t)s->dag_levels; l < s->levels.size(); l++) {
         const Level &Lv = s->levels[l];
         if (tr) tr->begin(st);
-        launch_diag<T>(s->facto, s->ds, s->d_diag_list + s->lvl_ds0[l], s->lvl_ds1[l] - s->lvl_ds0[l], L, U,
-                       (T *)s->dTinv, s->d_toff, s->d_thr, s->d_npiv, s->d_err, st);
+        const int nd = s->lvl_ds1[l] - s->lvl_ds0[l];
+        if (nd > 0) {
+            launch_diag_lu<T>(s->ds, s->d_diag_list + s->lvl_ds0[l], nd, L, U, s->d_thr, s->d_npiv, s->d_err, st);
+            launches++;
+        }
         {
             const int b[4] = {s->lvl_dsm0[l], s->lvl_dsm8[l], s->lvl_dsm16[l], s->lvl_dsm1[l]};
             const int nb[3] = {8, 16, 32};
@@ -1086,24 +1094,13 @@ int enqueue_numfact(b200_solver_t *s, cudaStream_t st, Trace *tr = nullptr) {
             }
         }
         if (tr) tr->end(1, st);
-        launches++;
         const int nt = Lv.t1 - Lv.t0;
-        if (tr) tr->begin(st);
         if (nt > 0) {
-            const int TR = s->lvl_tr[l];
-            const T *ti = (const T *)s->dTinv;
-            if (s->facto == FACTO_POTRF) {
-                launch_trsm<T>(s->ds, s->d_trsm + Lv.t0, nt, TR, Lv.nmax, L, L, 1, ti, s->d_toff, 0, 0, 0, st);
-            } else if (s->facto == FACTO_SYTRF) {
-                launch_trsm<T>(s->ds, s->d_trsm + Lv.t0, nt, TR, Lv.nmax, L, L, 0, ti, s->d_toff, 0, 0, 1, st);
-            } else {
-                launch_trsm<T>(s->ds, s->d_trsm + Lv.t0, nt, TR, Lv.nmax, L, L, 0, ti, s->d_toff, 1, 1, 0, st);
-                launch_trsm<T>(s->ds, s->d_trsm + Lv.t0, nt, TR, Lv.nmax, U, L, 1, ti, s->d_toff, 0, 1, 0, st);
-                launches++;
-            }
-            launches++;
+            if (tr) tr->begin(st);
+            launch_lu_trsm<T>(s->ds, s->d_trsm + Lv.t0, nt, s->lvl_tr[l], Lv.nmax, L, U, st);
+            launches += 2;
+            if (tr) tr->end(2, st);
         }
-        if (tr) tr->end(2, st);
         // wide cblks: the whole panel factorization in one launch
         if (s->lvl_pi1[l] > s->lvl_pi0[l]) {
             if (tr) tr->begin(st);

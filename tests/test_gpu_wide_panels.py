@@ -59,3 +59,25 @@ def test_lu_panels_replace_every_small_pivot():
     s.bcsc_load(bc)
     assert s.numfact(-1e3) == st.n
     s.close()
+
+
+@pytest.mark.parametrize("facto,shift", [("getrf", 0.0), ("potrf", 0.0), ("sytrf", -0.05)])
+def test_forms_without_resident_row_blocks(facto, shift, monkeypatch):
+    # the tile-item launch (Cholesky, LDL^T) and the one-CTA LU kernels, which cblks too
+    # wide for a resident row block take
+    st, bc, xt, b = analysis(facto, 7, (20, 20, 20), shift)
+    monkeypatch.setenv("B200_PANEL_TILES", "1")
+    s = native.Solver(st, facto, "fp64")
+    s.bcsc_load(bc)
+    s.numfact(1e-8)
+    Lg, Ug = s.factor()
+    orc = oracle.Oracle(st)
+    L, U = orc.fillin(bc)
+    orc.numfact(C.FACTO_ID[facto], L, U, s.stats()["threshold"])
+    mask = orc.factor_mask(C.FACTO_ID[facto])
+    assert np.linalg.norm((Lg - L)[mask]) <= 1e-12 * np.linalg.norm(L[mask])
+    if facto == "getrf":
+        assert np.linalg.norm(Ug - U) <= 1e-12 * np.linalg.norm(U)
+    x = s.solve(b)
+    s.close()
+    assert np.linalg.norm(x - xt) <= 1e-11 * np.linalg.norm(xt)
