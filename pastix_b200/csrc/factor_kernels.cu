@@ -720,8 +720,8 @@ __device__ void small_trsm_warp(const DevSym &s, int k, T *L, T *U, const T *til
 // *ferr its counters in shared memory.  On return the factored tile is still in tile
 // (the panel solve, small_trsm_warp, reads it from there).
 template <typename T, int FACTO, int NB>
-__device__ __forceinline__ void small_diag_warp(const DevSym &s, int k, T *L, T *U, T *tinv,
-                                                const int64_t *__restrict__ tinv_off, const double *__restrict__ thr_ptr,
+__device__ __forceinline__ void small_diag_warp(const DevSym &s, int k, T *L, T *U, T *WL, T *WU,
+                                                const int64_t *__restrict__ woff, const double *__restrict__ thr_ptr,
                                                 unsigned long long *npiv, int *err, T *tile, T *wl, T *wu, int *piv,
                                                 int *ferr, int lane) {
     const int n = s.ncols[k], ld = s.ld[k];
@@ -742,17 +742,16 @@ __device__ __forceinline__ void small_diag_warp(const DevSym &s, int k, T *L, T 
     factor_tile<T, FACTO, NB>(tile, n, lane, thr, piv, ferr);
     invert_lower_tile<T, NB>(tile, wl, n, lane, FACTO != FACTO_POTRF, 0);
     if (FACTO == FACTO_GETRF) invert_lower_tile<T, NB>(tile, wu, n, lane, 0, 1);  // inv(U^T)
-    T *tp = tinv + tinv_off[k];
+    T *Wl = WL + woff[k], *Wu = FACTO == FACTO_GETRF ? WU + woff[k] : nullptr;  // n x n, for the solves
     for (int idx = lane; idx < 32 * NB; idx += 32) {
         const int i = idx & 31, j = idx >> 5;
-        if (i < n && j < n && (FACTO != FACTO_POTRF || i >= j)) {
+        if (i >= n || j >= n) continue;
+        if (FACTO != FACTO_POTRF || i >= j) {
             A[i + (size_t)j * ld] = tile[i + j * TP];
             if (FACTO == FACTO_GETRF) U[s.off[k] + j + (size_t)i * ld] = tile[i + j * TP];
         }
-        if (j < n) {
-            tp[i + j * 32] = wl[i + j * TP];
-            if (FACTO == FACTO_GETRF) tp[32 * n + i + j * 32] = wu[i + j * TP];
-        }
+        Wl[i + j * n] = i >= j ? wl[i + j * TP] : (T)0;
+        if (FACTO == FACTO_GETRF) Wu[i + j * n] = i >= j ? wu[i + j * TP] : (T)0;
     }
     __syncwarp();
     if (lane == 0) {
@@ -763,15 +762,15 @@ __device__ __forceinline__ void small_diag_warp(const DevSym &s, int k, T *L, T 
 
 // Cblks with at most 32 columns, one warp per cblk (the bottom levels of the tree
 // hold tens of thousands): static pivoting, geadd of
-// U^T for LU, factor_tile, the tile inverse(s), write-back (and U^T for LU) -- and
+// U^T for LU, factor_tile, the tile inverse(s) for the solves, write-back (and U^T for LU) -- and
 // the panel solve of the rows below (small_trsm_warp), so that these cblks need no
 // TRSM launch.  One instance per width class NB (8, 16, 32 columns): the narrow
 // classes, most of the cblks, need a fraction of the registers and shared memory, so
 // more warps share an SM.
 template <typename T, int FACTO, int NB>
 __global__ void __launch_bounds__(32 * DS_WARPS) diag_small_kernel(DevSym s, const int *__restrict__ cblks, int ncblk,
-                                                                   T *L, T *U, T *tinv,
-                                                                   const int64_t *__restrict__ tinv_off,
+                                                                   T *L, T *U, T *WL, T *WU,
+                                                                   const int64_t *__restrict__ woff,
                                                                    const double *__restrict__ thr_ptr,
                                                                    unsigned long long *npiv, int *err) {
     extern __shared__ __align__(16) unsigned char ds_smem[];
@@ -784,7 +783,7 @@ __global__ void __launch_bounds__(32 * DS_WARPS) diag_small_kernel(DevSym s, con
     const int ci = blockIdx.x * DS_WARPS + warp;
     if (ci >= ncblk) return;
     const int k = cblks[ci];
-    small_diag_warp<T, FACTO, NB>(s, k, L, U, tinv, tinv_off, thr_ptr, npiv, err, tile, wl, wu, &s_piv[warp],
+    small_diag_warp<T, FACTO, NB>(s, k, L, U, WL, WU, woff, thr_ptr, npiv, err, tile, wl, wu, &s_piv[warp],
                                   &s_err[warp], lane);
     small_trsm_warp<T, FACTO, NB>(s, k, L, U, tile, wl, lane);
 }
@@ -954,7 +953,7 @@ template <typename T, int FACTO>
 __global__ void __launch_bounds__(32 * DG_WARPS) dag_bottom_kernel(DevSym s, const DagItem *__restrict__ items,
                                                                    int nitems, const Upd *__restrict__ upds, int *cnt,
                                                                    int *ticket, int *abort_word, T *L, T *U,
-                                                                   T *tinv, const int64_t *__restrict__ tinv_off,
+                                                                   T *WL, T *WU, const int64_t *__restrict__ woff,
                                                                    const double *__restrict__ thr_ptr,
                                                                    unsigned long long *npiv, int *err) {
     extern __shared__ __align__(16) unsigned char dg_smem[];
@@ -986,15 +985,15 @@ __global__ void __launch_bounds__(32 * DG_WARPS) dag_bottom_kernel(DevSym s, con
         const int n = s.ncols[k];
         if (it.fact) {
             if (n <= 8) {
-                small_diag_warp<T, FACTO, 8>(s, k, L, U, tinv, tinv_off, thr_ptr, npiv, err, tile, wl, wu,
+                small_diag_warp<T, FACTO, 8>(s, k, L, U, WL, WU, woff, thr_ptr, npiv, err, tile, wl, wu,
                                              &s_piv[warp], &s_err[warp], lane);
                 small_trsm_warp<T, FACTO, 8>(s, k, L, U, tile, wl, lane);
             } else if (n <= 16) {
-                small_diag_warp<T, FACTO, 16>(s, k, L, U, tinv, tinv_off, thr_ptr, npiv, err, tile, wl, wu,
+                small_diag_warp<T, FACTO, 16>(s, k, L, U, WL, WU, woff, thr_ptr, npiv, err, tile, wl, wu,
                                               &s_piv[warp], &s_err[warp], lane);
                 small_trsm_warp<T, FACTO, 16>(s, k, L, U, tile, wl, lane);
             } else {
-                small_diag_warp<T, FACTO, 32>(s, k, L, U, tinv, tinv_off, thr_ptr, npiv, err, tile, wl, wu,
+                small_diag_warp<T, FACTO, 32>(s, k, L, U, WL, WU, woff, thr_ptr, npiv, err, tile, wl, wu,
                                               &s_piv[warp], &s_err[warp], lane);
                 small_trsm_warp<T, FACTO, 32>(s, k, L, U, tile, wl, lane);
             }
@@ -1046,37 +1045,38 @@ template void launch_update_small<double>(const DevSym &, const Upd *, int, int,
 template void launch_update_small<float>(const DevSym &, const Upd *, int, int, float *, float *, cudaStream_t);
 
 template <typename T, int NB>
-static void launch_diag_small_nb(int facto, const DevSym &s, const int *cblks, int ncblk, T *L, T *U, T *tinv,
-                                 const int64_t *tinv_off, const double *thr, unsigned long long *npiv, int *err,
+static void launch_diag_small_nb(int facto, const DevSym &s, const int *cblks, int ncblk, T *L, T *U, T *WL, T *WU,
+                                 const int64_t *woff, const double *thr, unsigned long long *npiv, int *err,
                                  cudaStream_t st) {
     const int grid = (ncblk + DS_WARPS - 1) / DS_WARPS;
     const size_t smem = (size_t)DS_WARPS * (facto == FACTO_GETRF ? 3 : 2) * NB * TP * sizeof(T);
     if (facto == FACTO_POTRF)
-        diag_small_kernel<T, FACTO_POTRF, NB><<<grid, 32 * DS_WARPS, smem, st>>>(s, cblks, ncblk, L, U, tinv, tinv_off,
+        diag_small_kernel<T, FACTO_POTRF, NB><<<grid, 32 * DS_WARPS, smem, st>>>(s, cblks, ncblk, L, U, WL, WU, woff,
                                                                                thr, npiv, err);
     else if (facto == FACTO_GETRF)
-        diag_small_kernel<T, FACTO_GETRF, NB><<<grid, 32 * DS_WARPS, smem, st>>>(s, cblks, ncblk, L, U, tinv, tinv_off,
+        diag_small_kernel<T, FACTO_GETRF, NB><<<grid, 32 * DS_WARPS, smem, st>>>(s, cblks, ncblk, L, U, WL, WU, woff,
                                                                                thr, npiv, err);
     else
-        diag_small_kernel<T, FACTO_SYTRF, NB><<<grid, 32 * DS_WARPS, smem, st>>>(s, cblks, ncblk, L, U, tinv, tinv_off,
+        diag_small_kernel<T, FACTO_SYTRF, NB><<<grid, 32 * DS_WARPS, smem, st>>>(s, cblks, ncblk, L, U, WL, WU, woff,
                                                                                thr, npiv, err);
 }
 
 template <typename T>
-void launch_diag_small(int facto, const DevSym &s, const int *cblks, int ncblk, int nb, T *L, T *U, T *tinv,
-                       const int64_t *tinv_off, const double *thr, unsigned long long *npiv, int *err,
+void launch_diag_small(int facto, const DevSym &s, const int *cblks, int ncblk, int nb, T *L, T *U, T *WL, T *WU,
+                       const int64_t *woff, const double *thr, unsigned long long *npiv, int *err,
                        cudaStream_t st) {
     if (ncblk <= 0) return;
     if (nb <= 8)
-        launch_diag_small_nb<T, 8>(facto, s, cblks, ncblk, L, U, tinv, tinv_off, thr, npiv, err, st);
+        launch_diag_small_nb<T, 8>(facto, s, cblks, ncblk, L, U, WL, WU, woff, thr, npiv, err, st);
     else if (nb <= 16)
-        launch_diag_small_nb<T, 16>(facto, s, cblks, ncblk, L, U, tinv, tinv_off, thr, npiv, err, st);
+        launch_diag_small_nb<T, 16>(facto, s, cblks, ncblk, L, U, WL, WU, woff, thr, npiv, err, st);
     else
-        launch_diag_small_nb<T, 32>(facto, s, cblks, ncblk, L, U, tinv, tinv_off, thr, npiv, err, st);
+        launch_diag_small_nb<T, 32>(facto, s, cblks, ncblk, L, U, WL, WU, woff, thr, npiv, err, st);
 }
 template void launch_diag_small<double>(int, const DevSym &, const int *, int, int, double *, double *, double *,
-                                        const int64_t *, const double *, unsigned long long *, int *, cudaStream_t);
-template void launch_diag_small<float>(int, const DevSym &, const int *, int, int, float *, float *, float *,
+                                        double *, const int64_t *, const double *, unsigned long long *, int *,
+                                        cudaStream_t);
+template void launch_diag_small<float>(int, const DevSym &, const int *, int, int, float *, float *, float *, float *,
                                        const int64_t *, const double *, unsigned long long *, int *, cudaStream_t);
 
 static size_t dag_bottom_smem(int facto, size_t esz) {
@@ -1085,25 +1085,25 @@ static size_t dag_bottom_smem(int facto, size_t esz) {
 
 template <typename T>
 void launch_dag_bottom(int facto, const DevSym &s, int grid, const DagItem *items, int nitems, const Upd *upds,
-                       int *cnt, int *ticket, int *abort_word, T *L, T *U, T *tinv, const int64_t *tinv_off,
+                       int *cnt, int *ticket, int *abort_word, T *L, T *U, T *WL, T *WU, const int64_t *woff,
                        const double *thr, unsigned long long *npiv, int *err, cudaStream_t st) {
     if (nitems <= 0 || grid <= 0) return;
     const size_t smem = dag_bottom_smem(facto, sizeof(T));
     if (facto == FACTO_POTRF)
         dag_bottom_kernel<T, FACTO_POTRF><<<grid, 32 * DG_WARPS, smem, st>>>(
-            s, items, nitems, upds, cnt, ticket, abort_word, L, U, tinv, tinv_off, thr, npiv, err);
+            s, items, nitems, upds, cnt, ticket, abort_word, L, U, WL, WU, woff, thr, npiv, err);
     else if (facto == FACTO_GETRF)
         dag_bottom_kernel<T, FACTO_GETRF><<<grid, 32 * DG_WARPS, smem, st>>>(
-            s, items, nitems, upds, cnt, ticket, abort_word, L, U, tinv, tinv_off, thr, npiv, err);
+            s, items, nitems, upds, cnt, ticket, abort_word, L, U, WL, WU, woff, thr, npiv, err);
     else
         dag_bottom_kernel<T, FACTO_SYTRF><<<grid, 32 * DG_WARPS, smem, st>>>(
-            s, items, nitems, upds, cnt, ticket, abort_word, L, U, tinv, tinv_off, thr, npiv, err);
+            s, items, nitems, upds, cnt, ticket, abort_word, L, U, WL, WU, woff, thr, npiv, err);
 }
 template void launch_dag_bottom<double>(int, const DevSym &, int, const DagItem *, int, const Upd *, int *, int *,
-                                        int *, double *, double *, double *, const int64_t *, const double *,
-                                        unsigned long long *, int *, cudaStream_t);
+                                        int *, double *, double *, double *, double *, const int64_t *,
+                                        const double *, unsigned long long *, int *, cudaStream_t);
 template void launch_dag_bottom<float>(int, const DevSym &, int, const DagItem *, int, const Upd *, int *, int *,
-                                       int *, float *, float *, float *, const int64_t *, const double *,
+                                       int *, float *, float *, float *, float *, const int64_t *, const double *,
                                        unsigned long long *, int *, cudaStream_t);
 
 // Grid of the tree-bottom launch: the CTAs resident at once (more would only queue

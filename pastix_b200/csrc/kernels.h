@@ -19,13 +19,12 @@ void launch_diag_lu(const DevSym &s, const int *cblks, int ncblk, T *L, T *U, co
 template <typename T>
 void launch_lu_trsm(const DevSym &s, const RowTask *tasks, int ntasks, int TR, int nmax, T *L, T *U,
                     cudaStream_t st);
-// tinv: per cblk 32 x ncols (x2 for LU) tile inverses, the diagonal-block inverses of the
-// cblks of at most 32 columns
 // cblks of at most nb (8, 16 or 32) columns, one warp per cblk: diagonal block, its inverse
-// and the panel solve of the rows below
+// (WL, for LU also WU of the stored U^T: the arenas of the solves) and the panel solve of
+// the rows below
 template <typename T>
-void launch_diag_small(int facto, const DevSym &s, const int *cblks, int ncblk, int nb, T *L, T *U, T *tinv,
-                       const int64_t *tinv_off, const double *thr, unsigned long long *npiv, int *err,
+void launch_diag_small(int facto, const DevSym &s, const int *cblks, int ncblk, int nb, T *L, T *U, T *WL, T *WU,
+                       const int64_t *woff, const double *thr, unsigned long long *npiv, int *err,
                        cudaStream_t st);
 // every wide cblk of a level in one launch (panel_kernels.cu): items
 // taken in order from *ticket, dependencies through the solved / updated counters
@@ -67,7 +66,7 @@ void launch_update_f32(const DevSym &s, const Upd *upds, const int2 *tmap, int n
 // of err.
 template <typename T>
 void launch_dag_bottom(int facto, const DevSym &s, int grid, const DagItem *items, int nitems, const Upd *upds,
-                       int *cnt, int *ticket, int *abort_word, T *L, T *U, T *tinv, const int64_t *tinv_off,
+                       int *cnt, int *ticket, int *abort_word, T *L, T *U, T *WL, T *WU, const int64_t *woff,
                        const double *thr, unsigned long long *npiv, int *err, cudaStream_t st);
 // its grid: the CTAs resident at once on this device, capped by the items (-1 on error)
 int dag_bottom_grid(int facto, bool f32, int ncblk);
@@ -108,10 +107,6 @@ template <typename T>
 void launch_diag_inverse(const DevSym &s, const RowTask *tiles, int ntiles, const RowTask *strips, int nstrips,
                          int nmax, const T *L, const T *U, T *WL, T *WU, const int64_t *woff, int unit,
                          cudaStream_t st);
-// W_k of cblks with at most 32 columns, copied from the diagonal kernel's tile inverses (which: 0 L, 1 U^T)
-template <typename T>
-void launch_copy_tile_inverse(const DevSym &s, const int *cblks, int ncblk, const T *tinv, const int64_t *toff, T *W,
-                              const int64_t *woff, int which, cudaStream_t st);
 // xout[k] += W_k xin[k] (forward) or W_k^T xin[k] (backward), one 64 x 64 tile of W_k per task
 // {k, output row0, K chunk col0}, xout zeroed by the caller before the sweep
 template <typename T, typename V>

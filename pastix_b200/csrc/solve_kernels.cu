@@ -1175,36 +1175,3 @@ template void launch_solve_diag_inv<float, float>(const DevSym &, const SolveTil
                                                   cudaStream_t);
 
 }  // namespace b200
-
-// W_k for cblks of at most 32 columns: the diagonal kernel already stored the
-// inverse of their single 32x32 tile (and, for LU, of the stored U^T) in the
-// tile-inverse store; copy it to the n x n layout of the solves.
-namespace b200 {
-
-template <typename T>
-__global__ void copy_tile_inverse_kernel(DevSym s, const int *__restrict__ cblks, const T *__restrict__ tinv,
-                                         const int64_t *__restrict__ toff, T *W, const int64_t *__restrict__ woff,
-                                         int which) {
-    const int k = cblks[blockIdx.x];
-    const int n = s.ncols[k];
-    const T *src = tinv + toff[k] + (which ? 32 * n : 0);
-    T *dst = W + woff[k];
-    for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
-        const int i = idx % n, j = idx / n;
-        dst[idx] = (i >= j) ? src[i + j * 32] : (T)0;
-    }
-}
-
-template <typename T>
-void launch_copy_tile_inverse(const DevSym &s, const int *cblks, int ncblk, const T *tinv, const int64_t *toff, T *W,
-                              const int64_t *woff, int which, cudaStream_t st) {
-    if (ncblk <= 0) return;
-    copy_tile_inverse_kernel<T><<<ncblk, 128, 0, st>>>(s, cblks, tinv, toff, W, woff, which);
-}
-
-template void launch_copy_tile_inverse<double>(const DevSym &, const int *, int, const double *, const int64_t *,
-                                               double *, const int64_t *, int, cudaStream_t);
-template void launch_copy_tile_inverse<float>(const DevSym &, const int *, int, const float *, const int64_t *,
-                                              float *, const int64_t *, int, cudaStream_t);
-
-}  // namespace b200

@@ -116,18 +116,15 @@ struct b200_solver_s {
     // inverses of the diagonal blocks: W_L (forward sweep) and, for LU, W_U (backward)
     int64_t *d_woff = nullptr;
     int64_t winv_elems = 0;
-    int64_t *d_toff = nullptr;          // tile inverses of the panel TRSM: 32 x ncols (x2 for LU) per cblk
-    int64_t tinv_elems = 0;
-    void *dTinv = nullptr;
     void *dWL = nullptr, *dWU = nullptr;
     Upd *d_upd = nullptr;
     int2 *d_updmap = nullptr;           // 64 x 64 tiles of the d_upd launches, level by level
     std::vector<Level> levels;
     // LU cblks of each level that go through the one-CTA diagonal kernel, then the one-warp classes
     int *d_diag_list = nullptr;
-    int *d_inv_small = nullptr;                        // cblks of <= 32 columns
-    RowTask *d_inv_tile = nullptr, *d_inv_strip = nullptr;  // diagonal blocks and strips of the wider ones
-    int n_inv_small = 0, n_inv_tile = 0, n_inv_strip = 0, inv_nmax = 0;
+    // inverses of the diagonal blocks of more than 32 columns: 32-column blocks and strips
+    RowTask *d_inv_tile = nullptr, *d_inv_strip = nullptr;
+    int n_inv_tile = 0, n_inv_strip = 0, inv_nmax = 0;
     std::vector<int> lvl_ds0, lvl_ds1;
     std::vector<int> lvl_dsm0, lvl_dsm1;  // cblks of <= 32 columns (one warp each)
     std::vector<int> lvl_dsm8, lvl_dsm16; // ends of their <= 8 and <= 16 column classes
@@ -841,12 +838,11 @@ int build_schedule(b200_solver_t *s) {
     }
     RET(s->dupload(&s->d_diag_list, diag_list));
     {
-        std::vector<int> small, big;
-        for (int k = 0; k < cs; k++) (s->ncols[k] <= 32 ? small : big).push_back(k);
         // the strips with the most blocks below them first, so that they do not form the
         // launch's tail
         std::vector<RowTask> tiles, strips;
-        for (int k : big) {
+        for (int k = 0; k < cs; k++) {
+            if (s->ncols[k] <= 32) continue;  // the one-warp diagonal kernel writes theirs
             s->inv_nmax = std::max(s->inv_nmax, s->ncols[k]);
             for (int c = 0; c < s->ncols[k]; c += 32) tiles.push_back({k, c});
             for (int c = 0; c < (s->ncols[k] - 1) / 32 * 32; c += 16) strips.push_back({k, c});
@@ -854,10 +850,8 @@ int build_schedule(b200_solver_t *s) {
         auto below = [&](const RowTask &t) { return (s->ncols[t.k] + 31) / 32 - t.row0 / 32; };
         std::stable_sort(strips.begin(), strips.end(),
                          [&](const RowTask &x, const RowTask &y) { return below(x) > below(y); });
-        s->n_inv_small = (int)small.size();
         s->n_inv_tile = (int)tiles.size();
         s->n_inv_strip = (int)strips.size();
-        RET(s->dupload(&s->d_inv_small, small));
         RET(s->dupload(&s->d_inv_tile, tiles));
         RET(s->dupload(&s->d_inv_strip, strips));
     }
@@ -876,14 +870,6 @@ int build_schedule(b200_solver_t *s) {
     }
     s->winv_elems = (wpos + walign - 1) / walign * walign;
     RET(s->dupload(&s->d_woff, woff));
-    std::vector<int64_t> toff(N);
-    int64_t tpos = 0;
-    for (int k = 0; k < N; k++) {
-        toff[k] = tpos;
-        tpos += (int64_t)32 * s->ncols[k] * (s->facto == FACTO_GETRF ? 2 : 1);
-    }
-    s->tinv_elems = tpos;
-    RET(s->dupload(&s->d_toff, toff));
     RET(s->dupload(&s->d_upd, upds));
     RET(s->dupload(&s->d_updmap, updmap));
     RET(s->dupload(&s->d_tcupd, tcupds));
@@ -1071,7 +1057,7 @@ int enqueue_numfact(b200_solver_t *s, cudaStream_t st, Trace *tr = nullptr) {
         CU(cudaMemcpyAsync(s->d_dag_cnt, s->d_dag_cnt0, (size_t)N * sizeof(int), cudaMemcpyDeviceToDevice, st));
         CU(cudaMemsetAsync(s->d_dag_cnt + N, 0, 2 * sizeof(int), st));
         launch_dag_bottom<T>(s->facto, s->ds, s->dag_grid, s->d_dag_item, s->dag_nitems, s->d_dag_upd,
-                             s->d_dag_cnt, s->d_dag_cnt + N, s->d_dag_cnt + N + 1, L, U, (T *)s->dTinv, s->d_toff,
+                             s->d_dag_cnt, s->d_dag_cnt + N, s->d_dag_cnt + N + 1, L, U, (T *)s->dWL, (T *)s->dWU, s->d_woff,
                              s->d_thr, s->d_npiv, s->d_err, st);
         launches++;
         if (tr) tr->end(8, st);
@@ -1089,7 +1075,7 @@ int enqueue_numfact(b200_solver_t *s, cudaStream_t st, Trace *tr = nullptr) {
             const int nb[3] = {8, 16, 32};
             for (int c = 0; c < 3; c++) {
                 launch_diag_small<T>(s->facto, s->ds, s->d_diag_list + b[c], b[c + 1] - b[c], nb[c], L, U,
-                                     (T *)s->dTinv, s->d_toff, s->d_thr, s->d_npiv, s->d_err, st);
+                                     (T *)s->dWL, (T *)s->dWU, s->d_woff, s->d_thr, s->d_npiv, s->d_err, st);
                 launches += (b[c + 1] > b[c]);
             }
         }
@@ -1148,16 +1134,9 @@ int enqueue_numfact(b200_solver_t *s, cudaStream_t st, Trace *tr = nullptr) {
     }
     // inverses of the diagonal blocks for the solves (W_L of L; for LU also W_U of the stored U^T)
     if (tr) tr->begin(st);
-    launch_copy_tile_inverse<T>(s->ds, s->d_inv_small, s->n_inv_small, (const T *)s->dTinv, s->d_toff, (T *)s->dWL,
-                                s->d_woff, 0, st);
     launch_diag_inverse<T>(s->ds, s->d_inv_tile, s->n_inv_tile, s->d_inv_strip, s->n_inv_strip, s->inv_nmax, L, U,
                            (T *)s->dWL, (T *)s->dWU, s->d_woff, s->facto != FACTO_POTRF, st);
-    launches += (s->n_inv_small > 0) + (s->n_inv_tile > 0) + (s->n_inv_strip > 0);
-    if (s->facto == FACTO_GETRF) {
-        launch_copy_tile_inverse<T>(s->ds, s->d_inv_small, s->n_inv_small, (const T *)s->dTinv, s->d_toff,
-                                    (T *)s->dWU, s->d_woff, 1, st);
-        launches += s->n_inv_small > 0;
-    }
+    launches += (s->n_inv_tile > 0) + (s->n_inv_strip > 0);
     if (tr) tr->end(5, st);
     CU(cudaGetLastError());
     s->launches_fact = launches;
@@ -1897,7 +1876,6 @@ int b200_solver_create_tuned(const b200_symbol_t *sym, int facto, int precision,
     if (!rc) rc = dalloc((char **)&s->dL, (size_t)s->arena * s->esz);
     if (!rc && facto == FACTO_GETRF) rc = dalloc((char **)&s->dU, (size_t)s->arena * s->esz);
     if (!rc) rc = dalloc((char **)&s->dWL, (size_t)s->winv_elems * s->esz);
-    if (!rc) rc = dalloc((char **)&s->dTinv, (size_t)s->tinv_elems * s->esz);
     if (!rc && facto == FACTO_GETRF) rc = dalloc((char **)&s->dWU, (size_t)s->winv_elems * s->esz);
     if (!rc && s->use_tc) {
         // operand arenas and their tensor maps
@@ -1952,7 +1930,6 @@ int b200_solver_destroy(b200_solver_t *s) {
     if (s->dL) cudaFree(s->dL);
     if (s->dU) cudaFree(s->dU);
     if (s->dWL) cudaFree(s->dWL);
-    if (s->dTinv) cudaFree(s->dTinv);
     if (s->d_tarena) cudaFree(s->d_tarena);
     if (s->dWU) cudaFree(s->dWU);
     if (s->d_colptr) cudaFree(s->d_colptr);
