@@ -4,9 +4,8 @@
 //  diag_lu_kernel      diagonal block of a wide LU cblk that the panel launch does not take
 //                      (core_z{potrf,getrf,sytrf}sp, kernels/core_z*trfsp.c)
 //  lu_trsm_kernel      its off-diagonal panel solve (core_ztrsmsp_2d, kernels/core_ztrsmsp.c:147-181)
-//  update_f64_kernel   GEMM + scatter-add into the facing cblk on FP64 tensor cores (DMMA)
+//  update_tile_kernel  GEMM + scatter-add into the facing cblk: FP64 tensor cores (DMMA), FP32 CUDA cores
 //                      (core_zgemmsp_2d2d, kernels/core_zgemmsp.c:396-465)
-//  update_simt_kernel  the same update for FP32 factors on CUDA cores
 #include "b200_internal.h"
 #include "kernels.h"
 #include "tile_ops.cuh"
@@ -21,14 +20,11 @@ __device__ __forceinline__ unsigned smem_u32(const void *p) {
     return static_cast<unsigned>(__cvta_generic_to_shared(p));
 }
 
-// 8-byte asynchronous global->shared copy; src_bytes = 0 fills zeros.
-__device__ __forceinline__ void cp_async8(void *dst, const void *src, bool ok) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem_u32(dst)), "l"(src),
-                 "r"(ok ? 8 : 0));
-}
-__device__ __forceinline__ void cp_async4(void *dst, const void *src, bool ok) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_u32(dst)), "l"(src),
-                 "r"(ok ? 4 : 0));
+// Asynchronous global->shared copy of one element; zero where !ok.
+template <typename T>
+__device__ __forceinline__ void cp_async_el(T *dst, const T *src, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(smem_u32(dst)), "l"(src), "n"(sizeof(T)),
+                 "r"(ok ? (int)sizeof(T) : 0));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
@@ -391,11 +387,17 @@ __device__ __forceinline__ void dmma_16x8x4(double (&c)[4], const double (&a)[2]
 }
 
 constexpr int UT_M = 64, UT_N = 64, UT_K = 16, UT_STAGES = 3, UT_LDS = UT_M + 4;
-constexpr int UPD_F64_SMEM = 2 * UT_STAGES * UT_K * UT_LDS * sizeof(double);
-constexpr int UPD_F64_CTAS = 4;  // per SM: 128 registers per thread, 52 KB of shared memory each
+constexpr int UT_OP = UT_M + 1;  // FP32: pitch of a column of the staged sums
+template <typename T>
+constexpr int UPD_SMEM = (2 * UT_STAGES * UT_K * UT_LDS + (sizeof(T) == 4 ? UT_N * UT_OP : 0)) * (int)sizeof(T);
+constexpr int UPD_CTAS = 4;      // per SM: 128 registers per thread, 52 (43) KB of shared memory each
 
-// 64x64 output tiles, 4 warps (2x2) of 32x32, DMMA m16n8k4, 3-stage cp.async pipeline over
-// K in chunks of 16 columns.  The grid is persistent (UPD_F64_CTAS per SM) and the pipeline
+// Updates off the 5th-generation tensor cores: 64x64 output tiles, 4 warps, 3-stage cp.async
+// pipeline over K in chunks of 16 columns.  FP64: 2x2 warps of 32x32, DMMA m16n8k4.  FP32:
+// multiply-adds, 8 rows x 4 columns per thread read as three 16-byte vectors per k (4 x 4
+// in scalars, one CTA per tile, reached 9 TFLOP/s on the LDL^T updates, bound by its
+// shared-memory reads; the products and their order are the same), a warp has 16 columns,
+// and the sums go through shared memory so that a warp's reductions are whole lines.  The grid is persistent (UPD_CTAS per SM) and the pipeline
 // runs over the chunks of a CTA's tiles one after the other: while a tile's last chunks
 // are multiplied and its sums go out, the first chunks of the next tile are already on
 // their way, and its record (read two tiles ahead through the ring su) costs no wait.  A
@@ -404,13 +406,16 @@ constexpr int UPD_F64_CTAS = 4;  // per SM: 128 registers per thread, 52 KB of s
 // and 16-row groups past the update's edge and the 32 x 32 quarters above the diagonal of
 // a symmetric update (17 % of the issued products at 80^3); which quarter a warp takes
 // turns with the CTA, so that the skipped ones do not all idle the same SM sub-partition.
-__global__ void __launch_bounds__(128, UPD_F64_CTAS)
-    update_f64_kernel(DevSym s, const Upd *__restrict__ upds, const int2 *__restrict__ tmap, int ntiles, double *L,
-                      double *U) {
+template <typename T>
+__global__ void __launch_bounds__(128, UPD_CTAS)
+    update_tile_kernel(DevSym s, const Upd *__restrict__ upds, const int2 *__restrict__ tmap, int ntiles, T *L, T *U) {
+    constexpr bool F64 = sizeof(T) == 8;
     extern __shared__ __align__(16) unsigned char upd_smem[];
-    double(*As)[UT_K][UT_LDS] = reinterpret_cast<double(*)[UT_K][UT_LDS]>(upd_smem);
-    double(*Bs)[UT_K][UT_LDS] = reinterpret_cast<double(*)[UT_K][UT_LDS]>(upd_smem + sizeof(double) * UT_STAGES * UT_K * UT_LDS);
-    __shared__ double Ds[UT_STAGES][UT_K];
+    T(*As)[UT_K][UT_LDS] = reinterpret_cast<T(*)[UT_K][UT_LDS]>(upd_smem);
+    T(*Bs)[UT_K][UT_LDS] = As + UT_STAGES;
+    T *os = reinterpret_cast<T *>(Bs + UT_STAGES);  // FP32: the tile's sums, column after column
+    __shared__ __align__(16) T Ds[UT_STAGES][UT_K];
+    __shared__ int srow[UT_M];                      // FP32: destination rows
     constexpr int UW = sizeof(Upd) / 4;
     static_assert(UW <= 31 && sizeof(Upd) % 8 == 0, "one warp reads a record and its tile");
     __shared__ __align__(8) int su[8][32];  // records of the tiles from the one being summed to the next to load
@@ -430,7 +435,7 @@ __global__ void __launch_bounds__(128, UPD_F64_CTAS)
 
     // loads: tile lq, chunk at column lk
     int lq = 0, lk = 0, lK = 0, lld = 0;
-    const double *lA = nullptr, *lB = nullptr, *lD = nullptr;  // this thread's first element of each operand
+    const T *lA = nullptr, *lB = nullptr, *lD = nullptr;  // this thread's first element of each operand
     bool lokA = false, lokB = false;
     int2 ahead = make_int2(0, 0);  // tile lq + 2
     auto open_tile = [&]() {       // record lq is in su
@@ -451,12 +456,12 @@ __global__ void __launch_bounds__(128, UPD_F64_CTAS)
 #pragma unroll
         for (int i = 0; i < UT_K / 2; i++) {
             const bool ok = lk + c + 2 * i < lK;
-            cp_async8(&As[st][c + 2 * i][r], ok ? lA + (size_t)(2 * i) * lld : lA, ok && lokA);
-            cp_async8(&Bs[st][c + 2 * i][r], ok ? lB + (size_t)(2 * i) * lld : lB, ok && lokB);
+            cp_async_el(&As[st][c + 2 * i][r], ok ? lA + (size_t)(2 * i) * lld : lA, ok && lokA);
+            cp_async_el(&Bs[st][c + 2 * i][r], ok ? lB + (size_t)(2 * i) * lld : lB, ok && lokB);
         }
         if (tid < UT_K && lD) {
             const bool ok = lk + tid < lK;
-            cp_async8(&Ds[st][tid], ok ? lD : L, ok);
+            cp_async_el(&Ds[st][tid], ok ? lD : L, ok);
             lD += (size_t)UT_K * (lld + 1);
         }
         lA += (size_t)UT_K * lld;
@@ -499,162 +504,156 @@ __global__ void __launch_bounds__(128, UPD_F64_CTAS)
     }
     int st = 0;
     for (int q = 0; q < nmine; q++) {
-        double acc[2][4][4];
-#pragma unroll
-        for (int a = 0; a < 2; a++)
-#pragma unroll
-            for (int b = 0; b < 4; b++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) acc[a][b][e] = 0.0;
         const Upd &u = *reinterpret_cast<const Upd *>(su[q & 7]);
-        const int m0 = (su[q & 7][31] & 0xffff) * UT_M + wm * 32, n0 = (su[q & 7][31] >> 16) * UT_N + wn * 32;
+        const int tm0 = (su[q & 7][31] & 0xffff) * UT_M, tn0 = (su[q & 7][31] >> 16) * UT_N;
         const int flags = u.flags, nk = (u.K + UT_K - 1) / UT_K;
         const bool scale = (flags & UPD_SCALE_D) != 0, sym = (flags & UPD_SYM) != 0;
-        const bool skip = sym && m0 + 31 < n0;
-        const int mrem = skip ? 0 : u.M - m0, nrem = skip ? 0 : u.N - n0;  // of this warp's quarter
-        const int nmi = (mrem + 15) >> 4, nni = mrem > 0 ? (nrem + 7) >> 3 : 0;
-        int drow[2][2];
-        for (int kt = 0; kt < nk; kt++) {
+        const bool atomic = (flags & UPD_ATOMIC) != 0;
+        T *C = ((flags & UPD_C_U) ? U : L) + u.offC;
+        const int ldf = u.ldf;
+        // one chunk's turn: wait for it, start the load of the one after next
+        auto turn = [&]() -> bool {
             cp_async_wait<UT_STAGES - 2>();
             __syncthreads();
             const int nxt = st + UT_STAGES - 1 >= UT_STAGES ? st - 1 : st + UT_STAGES - 1;
             const bool keep = load_next(nxt);
             cp_async_commit();
-            if (kt == nk - 1) {
-                // destination rows, used after the last products
-#pragma unroll
-                for (int mi = 0; mi < 2; mi++)
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        const int row = mi * 16 + h * 8 + g;
-                        drow[mi][h] = row < mrem ? __ldg(s.rmap + u.rm0 + m0 + row) : -1;
-                    }
-            }
-            if (nni > 0) {
-#pragma unroll
-                for (int k4 = 0; k4 < UT_K; k4 += 4) {
-                    double a[2][2], b[4];
-                    const double dsc = scale ? Ds[st][k4 + tg] : 1.0;
-#pragma unroll
-                    for (int mi = 0; mi < 2; mi++) {
-                        const int row = wm * 32 + mi * 16 + g;
-                        a[mi][0] = As[st][k4 + tg][row];
-                        a[mi][1] = As[st][k4 + tg][row + 8];
-                        if (scale) {
-                            a[mi][0] *= dsc;
-                            a[mi][1] *= dsc;
-                        }
-                    }
-#pragma unroll
-                    for (int ni = 0; ni < 4; ni++) b[ni] = Bs[st][k4 + tg][wn * 32 + ni * 8 + g];
-#pragma unroll
-                    for (int ni = 0; ni < 4; ni++)
-                        if (ni < nni) {
-                            dmma_16x8x4(acc[0][ni], a[0], b[ni]);
-                            if (nmi > 1) dmma_16x8x4(acc[1][ni], a[1], b[ni]);
-                        }
-                }
-            }
+            return keep;
+        };
+        auto done = [&](bool keep) {
             if (keep) keep_record(lq + 1);
             st = st + 1 == UT_STAGES ? 0 : st + 1;
-        }
-        double *C = ((flags & UPD_C_U) ? U : L) + u.offC;
-        const int ldf = u.ldf;
-        const bool atomic = (flags & UPD_ATOMIC) != 0;
+        };
+        if constexpr (F64) {
+            double acc[2][4][4];
 #pragma unroll
-        for (int mi = 0; mi < 2; mi++) {
+            for (int a = 0; a < 2; a++)
 #pragma unroll
-            for (int ni = 0; ni < 4; ni++) {
-                if (ni >= nni) continue;
+                for (int b = 0; b < 4; b++)
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const int row = mi * 16 + g + (e >> 1) * 8, col = ni * 8 + 2 * tg + (e & 1);
-                    const int d = drow[mi][e >> 1];
-                    if (d < 0 || col >= nrem || (sym && m0 + row < n0 + col)) continue;
-                    double *p = C + d + (size_t)(n0 + col) * ldf;
-                    if (atomic) atomicAdd(p, -acc[mi][ni][e]);
-                    else *p -= acc[mi][ni][e];
+                    for (int e = 0; e < 4; e++) acc[a][b][e] = 0.0;
+            const int m0 = tm0 + wm * 32, n0 = tn0 + wn * 32;
+            const bool skip = sym && m0 + 31 < n0;
+            const int mrem = skip ? 0 : u.M - m0, nrem = skip ? 0 : u.N - n0;  // of this warp's quarter
+            const int nmi = (mrem + 15) >> 4, nni = mrem > 0 ? (nrem + 7) >> 3 : 0;
+            int drow[2][2];
+            for (int kt = 0; kt < nk; kt++) {
+                const bool keep = turn();
+                if (kt == nk - 1) {
+                    // destination rows, used after the last products
+#pragma unroll
+                    for (int mi = 0; mi < 2; mi++)
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const int row = mi * 16 + h * 8 + g;
+                            drow[mi][h] = row < mrem ? __ldg(s.rmap + u.rm0 + m0 + row) : -1;
+                        }
+                }
+                if (nni > 0) {
+#pragma unroll
+                    for (int k4 = 0; k4 < UT_K; k4 += 4) {
+                        double a[2][2], b[4];
+                        const double dsc = scale ? Ds[st][k4 + tg] : 1.0;
+#pragma unroll
+                        for (int mi = 0; mi < 2; mi++) {
+                            const int row = wm * 32 + mi * 16 + g;
+                            a[mi][0] = As[st][k4 + tg][row];
+                            a[mi][1] = As[st][k4 + tg][row + 8];
+                            if (scale) {
+                                a[mi][0] *= dsc;
+                                a[mi][1] *= dsc;
+                            }
+                        }
+#pragma unroll
+                        for (int ni = 0; ni < 4; ni++) b[ni] = Bs[st][k4 + tg][wn * 32 + ni * 8 + g];
+#pragma unroll
+                        for (int ni = 0; ni < 4; ni++)
+                            if (ni < nni) {
+                                dmma_16x8x4(acc[0][ni], a[0], b[ni]);
+                                if (nmi > 1) dmma_16x8x4(acc[1][ni], a[1], b[ni]);
+                            }
+                    }
+                }
+                done(keep);
+            }
+#pragma unroll
+            for (int mi = 0; mi < 2; mi++) {
+#pragma unroll
+                for (int ni = 0; ni < 4; ni++) {
+                    if (ni >= nni) continue;
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const int row = mi * 16 + g + (e >> 1) * 8, col = ni * 8 + 2 * tg + (e & 1);
+                        const int d = drow[mi][e >> 1];
+                        if (d < 0 || col >= nrem || (sym && m0 + row < n0 + col)) continue;
+                        double *p = C + d + (size_t)(n0 + col) * ldf;
+                        if (atomic) atomicAdd(p, -acc[mi][ni][e]);
+                        else *p -= acc[mi][ni][e];
+                    }
                 }
             }
+        } else {
+            // rows 4 tx .. and 32 + 4 tx .., columns 4 ty ..; quarter: the warp's 16 columns
+            const int tx = lane & 7, ty = 4 * quarter + (lane >> 3);
+            float acc[8][4];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+            const int nrem = u.N - tn0, mrem = u.M - tm0;
+            const bool idle = 16 * quarter >= nrem || (sym && tm0 + 63 < tn0 + 16 * quarter);
+            for (int kt = 0; kt < nk; kt++) {
+                const bool keep = turn();
+                if (kt == nk - 1 && tid < UT_M) srow[tid] = tid < mrem ? __ldg(s.rmap + u.rm0 + tm0 + tid) : -1;
+                if (!idle) {
+#pragma unroll
+                    for (int c = 0; c < UT_K; c++) {
+                        const float4 a0 = *reinterpret_cast<const float4 *>(&As[st][c][4 * tx]);
+                        const float4 a1 = *reinterpret_cast<const float4 *>(&As[st][c][32 + 4 * tx]);
+                        const float4 bq = *reinterpret_cast<const float4 *>(&Bs[st][c][4 * ty]);
+                        float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+                        const float bv[4] = {bq.x, bq.y, bq.z, bq.w};
+                        if (scale) {
+                            const float d = Ds[st][c];
+#pragma unroll
+                            for (int i = 0; i < 8; i++) av[i] *= d;
+                        }
+#pragma unroll
+                        for (int i = 0; i < 8; i++)
+#pragma unroll
+                            for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+                    }
+                }
+                done(keep);
+            }
+            // the warp's own columns of the sums, then lane = row
+            if (!idle) {
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+#pragma unroll
+                    for (int i = 0; i < 8; i++) os[(4 * ty + j) * UT_OP + (i & 4) * 8 + 4 * tx + (i & 3)] = acc[i][j];
+            }
+            __syncthreads();
+            if (!idle) {
+                const int c1 = min(16, nrem - 16 * quarter);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int row = lane + 32 * h, d = srow[row];
+                    if (d < 0) continue;
+                    for (int c = 0; c < c1; c++) {
+                        const int col = 16 * quarter + c;
+                        if (sym && tm0 + row < tn0 + col) break;
+                        float *p = C + d + (size_t)(tn0 + col) * ldf;
+                        const float v = os[col * UT_OP + row];
+                        if (atomic) atomicAdd(p, -v);
+                        else *p -= v;
+                    }
+                }
+            }
+            // (srow and the sums of the next tile are written after its first barrier)
         }
     }
     cp_async_wait<0>();
-}
-
-// FP32 factor update on CUDA cores: 64x64 tile, 256 threads (4x4 each), K chunks of 16.
-__global__ void __launch_bounds__(256) update_simt_f32_kernel(DevSym s, const Upd *__restrict__ upds,
-                                                              const int2 *__restrict__ tmap, float *L, float *U) {
-    __shared__ __align__(16) float As[2][UT_K][UT_M + 4];
-    __shared__ __align__(16) float Bs[2][UT_K][UT_N + 4];
-    __shared__ int drow[UT_M];
-    const int2 tc2 = tmap[blockIdx.x];
-    const Upd u = upds[tc2.x];
-    const int m0 = (tc2.y & 0xffff) * UT_M, n0 = (tc2.y >> 16) * UT_N, ldk = u.ldk;
-    const float *Ap = ((u.flags & UPD_A_U) ? U : L) + u.offA + m0;
-    const float *Bp = ((u.flags & UPD_B_U) ? U : L) + u.offB + n0;
-    const float *Dp = L + u.offD;
-    const bool scale = (u.flags & UPD_SCALE_D) != 0;
-    const int mrem = u.M - m0, nrem = u.N - n0;
-    const int tid = threadIdx.x;
-    const int tr = tid & 15, tc = tid >> 4;
-    float acc[4][4] = {};
-    const int nk = (u.K + UT_K - 1) / UT_K;
-    auto load_stage = [&](int st, int kc) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int idx = tid + i * 256;
-            const int r = idx & 63, c = idx >> 6;
-            const int kk = kc + c;
-            const bool okA = (r < mrem) && (kk < u.K);
-            const bool okB = (r < nrem) && (kk < u.K);
-            cp_async4(&As[st][c][r], okA ? Ap + r + (size_t)kk * ldk : Ap, okA);
-            cp_async4(&Bs[st][c][r], okB ? Bp + r + (size_t)kk * ldk : Bp, okB);
-        }
-    };
-    load_stage(0, 0);
-    cp_async_commit();
-    for (int kt = 0; kt < nk; kt++) {
-        const int st = kt & 1;
-        if (kt + 1 < nk) load_stage(st ^ 1, (kt + 1) * UT_K);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-#pragma unroll
-        for (int c = 0; c < UT_K; c++) {
-            const int kk = kt * UT_K + c;
-            const float dsc = (scale && kk < u.K) ? Dp[(size_t)kk * (ldk + 1)] : 1.0f;
-            float av[4], bv[4];
-#pragma unroll
-            for (int a = 0; a < 4; a++) av[a] = As[st][c][tr + 16 * a] * dsc;
-#pragma unroll
-            for (int b = 0; b < 4; b++) bv[b] = Bs[st][c][tc + 16 * b];
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) acc[a][b] = fmaf(av[a], bv[b], acc[a][b]);
-        }
-        __syncthreads();
-    }
-    if (tid < UT_M) drow[tid] = (m0 + tid < u.M) ? __ldg(s.rmap + u.rm0 + m0 + tid) : -1;
-    __syncthreads();
-    float *C = ((u.flags & UPD_C_U) ? U : L) + u.offC;
-    const int ldf = u.ldf;
-    const bool atomic = (u.flags & UPD_ATOMIC) != 0;
-    const bool sym = (u.flags & UPD_SYM) != 0;
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-            const int row = tr + 16 * a, col = tc + 16 * b;
-            if (n0 + col >= u.N) continue;
-            if (sym && m0 + row < n0 + col) continue;
-            const int d = drow[row];
-            if (d < 0) continue;
-            float *p = C + d + (size_t)(n0 + col) * ldf;
-            if (atomic) atomicAdd(p, -acc[a][b]);
-            else *p -= acc[a][b];
-        }
-    }
 }
 
 // ------------------------------------------------------------------ launchers
@@ -1144,19 +1143,16 @@ void launch_lu_trsm(const DevSym &s, const RowTask *tasks, int ntasks, int TR, i
     lu_trsm_kernel<T><<<ntasks, 256, smem, st>>>(s, tasks, TR, U, L, 1);
 }
 
-static int g_f64_grid = 0;  // resident CTAs of update_f64_kernel on the device
+static int g_upd_grid[2] = {0, 0};  // resident CTAs of update_tile_kernel on the device (FP64, FP32)
 
-void launch_update_f64(const DevSym &s, const Upd *upds, const int2 *tmap, int ntiles, double *L, double *U,
-                       cudaStream_t st) {
+template <typename T>
+void launch_update(const DevSym &s, const Upd *upds, const int2 *tmap, int ntiles, T *L, T *U, cudaStream_t st) {
     if (ntiles <= 0) return;
-    update_f64_kernel<<<std::min(ntiles, g_f64_grid), 128, UPD_F64_SMEM, st>>>(s, upds, tmap, ntiles, L, U);
+    update_tile_kernel<T><<<std::min(ntiles, g_upd_grid[sizeof(T) == 4]), 128, UPD_SMEM<T>, st>>>(s, upds, tmap, ntiles,
+                                                                                               L, U);
 }
-
-void launch_update_f32(const DevSym &s, const Upd *upds, const int2 *tmap, int ntiles, float *L, float *U,
-                       cudaStream_t st) {
-    if (ntiles <= 0) return;
-    update_simt_f32_kernel<<<ntiles, 256, 0, st>>>(s, upds, tmap, L, U);
-}
+template void launch_update<double>(const DevSym &, const Upd *, const int2 *, int, double *, double *, cudaStream_t);
+template void launch_update<float>(const DevSym &, const Upd *, const int2 *, int, float *, float *, cudaStream_t);
 
 template <typename K>
 static int raise_smem(K kernel) {
@@ -1184,19 +1180,22 @@ static int raise_diag_small_smem() {
     return 0;
 }
 
+template <typename T>
+static int configure_update() {
+    int dev = 0, sms = 0, occ = 0;
+    if (raise_smem(update_tile_kernel<T>) < UPD_SMEM<T> || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, update_tile_kernel<T>, 128, UPD_SMEM<T>) != cudaSuccess ||
+        occ < 1)
+        return -1;
+    g_upd_grid[sizeof(T) == 4] = occ * sms;
+    return 0;
+}
+
 int configure_factor_kernels() {
     int lim = 1 << 30;
     int v;
-    if ((v = raise_smem(update_f64_kernel)) < UPD_F64_SMEM) return -1;
-    {
-        int dev = 0, sms = 0, occ = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, update_f64_kernel, 128, UPD_F64_SMEM) != cudaSuccess ||
-            occ < 1)
-            return -1;
-        g_f64_grid = occ * sms;
-    }
+    if (configure_update<double>() || configure_update<float>()) return -1;
     if (raise_diag_small_smem<8>() < 0 || raise_diag_small_smem<16>() < 0 || raise_diag_small_smem<32>() < 0)
         return -1;
     if (raise_smem(dag_bottom_kernel<double, FACTO_POTRF>) < 0 || raise_smem(dag_bottom_kernel<double, FACTO_SYTRF>) < 0 ||

@@ -53,10 +53,8 @@ void launch_get_diag(const DevSym &s, const T *L, double *out, cudaStream_t st);
 template <typename T>
 void launch_update_small(const DevSym &s, const Upd *upds, int n8, int nupd, T *L, T *U, cudaStream_t st);
 // 64 x 64 tiles listed by tmap ({update, row tile | column tile << 16})
-void launch_update_f64(const DevSym &s, const Upd *upds, const int2 *tmap, int ntiles, double *L, double *U,
-                       cudaStream_t st);
-void launch_update_f32(const DevSym &s, const Upd *upds, const int2 *tmap, int ntiles, float *L, float *U,
-                       cudaStream_t st);
+template <typename T>
+void launch_update(const DevSym &s, const Upd *upds, const int2 *tmap, int ntiles, T *L, T *U, cudaStream_t st);
 // the bottom levels of the tree in one launch (cblks of at most 32 columns): items
 // (factor items, then update items, level by level) taken by warps from *ticket; a
 // factor item starts when cnt[k] (the update items k receives from the launch's cblks)

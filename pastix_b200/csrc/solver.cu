@@ -1110,10 +1110,7 @@ int enqueue_numfact(b200_solver_t *s, cudaStream_t st, Trace *tr = nullptr) {
             launches += (n8 > 0) + (nu > n8);
         }
         if (Lv.ntiles > 0) {
-            if (sizeof(T) == 8)
-                launch_update_f64(s->ds, s->d_upd + Lv.u0, s->d_updmap + Lv.m0, Lv.ntiles, (double *)L, (double *)U, st);
-            else
-                launch_update_f32(s->ds, s->d_upd + Lv.u0, s->d_updmap + Lv.m0, Lv.ntiles, (float *)L, (float *)U, st);
+            launch_update<T>(s->ds, s->d_upd + Lv.u0, s->d_updmap + Lv.m0, Lv.ntiles, L, U, st);
             launches++;
         }
         if (tr) tr->end(3, st);

@@ -1,7 +1,7 @@
 // GEMM + scatter-add update of FP32 factors on the 5th-generation tensor cores
 // (sm_100a: TMA, tcgen05.mma kind::tf32, accumulators in tensor memory).
 //
-// Same operation as update_simt_f32_kernel (core_zgemmsp_2d2d,
+// Same operation as update_tile_kernel (core_zgemmsp_2d2d,
 // kernels/core_zgemmsp.c:396-465): C_f[rows, cols of block j] -= A_k[rows] B_k[j]^T
 // with K = ncols_k, scattered into the facing cblk f through the block index map.
 //
