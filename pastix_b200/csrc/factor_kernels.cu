@@ -11,6 +11,7 @@
 #include "tile_ops.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace b200 {
 
@@ -406,6 +407,11 @@ constexpr int UPD_CTAS = 4;      // per SM: 128 registers per thread, 52 (43) KB
 // and 16-row groups past the update's edge and the 32 x 32 quarters above the diagonal of
 // a symmetric update (17 % of the issued products at 80^3); which quarter a warp takes
 // turns with the CTA, so that the skipped ones do not all idle the same SM sub-partition.
+// A quarter in use as a whole runs without the tests of its groups (FP64: 69.5 -> 64.1 ms of
+// updates at 80^3, 27-point, 25.6 TFLOP/s of useful work against the 35.9 of a library GEMM;
+// 74.3 ms with one CTA per tile), FP32's unscaled products without the test for D (LDL^T at
+// 44 x 40 x 39, scaled: 2.75 ms with one CTA per tile, 1.38 now).  Reading the next operands
+// ahead of the FP64 products gained nothing (65.0), nor did m16n8k8 (71.2 at 3 CTAs per SM).
 template <typename T>
 __global__ void __launch_bounds__(128, UPD_CTAS)
     update_tile_kernel(DevSym s, const Upd *__restrict__ upds, const int2 *__restrict__ tmap, int ntiles, T *L, T *U) {
@@ -549,7 +555,8 @@ __global__ void __launch_bounds__(128, UPD_CTAS)
                             drow[mi][h] = row < mrem ? __ldg(s.rmap + u.rm0 + m0 + row) : -1;
                         }
                 }
-                if (nni > 0) {
+                auto products = [&](auto all) {
+                    constexpr bool full = decltype(all)::value;
 #pragma unroll
                     for (int k4 = 0; k4 < UT_K; k4 += 4) {
                         double a[2][2], b[4];
@@ -568,12 +575,14 @@ __global__ void __launch_bounds__(128, UPD_CTAS)
                         for (int ni = 0; ni < 4; ni++) b[ni] = Bs[st][k4 + tg][wn * 32 + ni * 8 + g];
 #pragma unroll
                         for (int ni = 0; ni < 4; ni++)
-                            if (ni < nni) {
+                            if (full || ni < nni) {
                                 dmma_16x8x4(acc[0][ni], a[0], b[ni]);
-                                if (nmi > 1) dmma_16x8x4(acc[1][ni], a[1], b[ni]);
+                                if (full || nmi > 1) dmma_16x8x4(acc[1][ni], a[1], b[ni]);
                             }
                     }
-                }
+                };
+                if (nni >= 4 && nmi > 1) products(std::true_type{});
+                else if (nni > 0) products(std::false_type{});
                 done(keep);
             }
 #pragma unroll
@@ -605,7 +614,7 @@ __global__ void __launch_bounds__(128, UPD_CTAS)
             for (int kt = 0; kt < nk; kt++) {
                 const bool keep = turn();
                 if (kt == nk - 1 && tid < UT_M) srow[tid] = tid < mrem ? __ldg(s.rmap + u.rm0 + tm0 + tid) : -1;
-                if (!idle) {
+                auto products = [&](auto scaled) {
 #pragma unroll
                     for (int c = 0; c < UT_K; c++) {
                         const float4 a0 = *reinterpret_cast<const float4 *>(&As[st][c][4 * tx]);
@@ -613,7 +622,7 @@ __global__ void __launch_bounds__(128, UPD_CTAS)
                         const float4 bq = *reinterpret_cast<const float4 *>(&Bs[st][c][4 * ty]);
                         float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
                         const float bv[4] = {bq.x, bq.y, bq.z, bq.w};
-                        if (scale) {
+                        if constexpr (decltype(scaled)::value) {
                             const float d = Ds[st][c];
 #pragma unroll
                             for (int i = 0; i < 8; i++) av[i] *= d;
@@ -623,6 +632,10 @@ __global__ void __launch_bounds__(128, UPD_CTAS)
 #pragma unroll
                             for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
                     }
+                };
+                if (!idle) {
+                    if (scale) products(std::true_type{});
+                    else products(std::false_type{});
                 }
                 done(keep);
             }
