@@ -105,6 +105,14 @@ struct SolveTile {
     int col0;  // first column of the cblk
 };
 
+// Tile of a many-right-hand-side sweep: 64 outputs from o0 of cblk k, K values [k0, k1)
+// (off-diagonal products: outputs are panel rows and K columns forward, the other way
+// round backward; diagonal products: rows of W_k, or of its transpose).
+constexpr int WIDE_LEAF = 8;  // narrower cblks take the one-warp kernel of those sweeps
+struct WideTask {
+    int k, o0, k0, k1;
+};
+
 // Item of a dataflow solve sweep (one launch per sweep): FI_LEAF up to 16 cblks
 // of at most 32 columns of one level (k = first position in the leaf list, n their
 // number); FI_DIAG output rows [r0, r0 + 64) x K chunk [n, n + 64) of the
@@ -114,6 +122,14 @@ struct SolveTile {
 enum : int { FI_LEAF = 0, FI_DIAG = 1, FI_OFF = 2 };
 struct FlowItem {
     int type, k, r0, n, f0, nf;
+};
+
+// Items and counter targets of the many-right-hand-side dataflow sweeps (device arrays),
+// as those of the narrow ones; panel rows start at a multiple of 4.
+struct WideFlow {
+    FlowItem *f, *b;
+    int nf, nb;
+    int *flist, *need_f, *need_b, *nprev_f, *nprev_b;
 };
 
 // Wide cblk of a panel launch (POTRF / LDL^T cblks wider than the one-CTA diagonal

@@ -122,6 +122,34 @@ void launch_solve_flow(const DevSym &s, const FlowItem *items, int nitems, const
                        const int *need, const int *nprev, const T *P, const T *W, const int64_t *woff, V *x, V *aux,
                        int64_t ldx, int nrhs, int backward, int *ticket, int *cnt_a, int *cnt_b, int *abort_word,
                        int *err, cudaStream_t st);
+// sweeps of many right-hand sides on row-major vectors (solve_wide.cu): element (i, j)
+// at i * ldr + j.  Off-diagonal products out -= (atomic), diagonal products out =, both
+// products of the cblks of at most 32 columns, and the moves between column-major
+// blocks and row-major ones
+template <typename T>
+void launch_wide_off(const DevSym &s, const WideTask *tasks, int ntasks, const T *P, const T *in, T *out, int ldr,
+                     int nrhs, int backward, cudaStream_t st);
+template <typename T>
+void launch_wide_diag(const DevSym &s, const WideTask *tasks, int ntasks, const T *W, const int64_t *woff, const T *in,
+                      T *out, int ldr, int nrhs, int backward, cudaStream_t st);
+template <typename T>
+void launch_wide_leaf(const DevSym &s, const int *cblks, int ncblk, const T *P, const T *W, const int64_t *woff, T *x,
+                      T *aux, int ldr, int nrhs, int backward, cudaStream_t st);
+template <typename S, typename D>
+void launch_wide_transpose(int n, int nrhs, const S *src, int64_t lds, D *dst, int64_t ldd, int to_rows,
+                           cudaStream_t st);
+template <typename T>
+void launch_wide_scale(const DevSym &s, const int *cblks, int ncblk, const T *L, T *x, int ldr, int nrhs,
+                       cudaStream_t st);
+// one dataflow sweep over the top levels (launch_solve_flow's counters and abort word);
+// the rows it accumulates into are zeroed first
+template <typename T>
+void launch_wide_flow(const DevSym &s, const WideFlow &fw, const T *P, const T *W, const int64_t *woff, T *x, T *aux,
+                      int ldr, int nrhs, int backward, int *ticket, int *cnt_a, int *cnt_b, int *abort_word, int *err,
+                      cudaStream_t st);
+template <typename T>
+void launch_wide_zero(const DevSym &s, const int *cblks, int ncblk, T *x, int ldr, int nrhs, cudaStream_t st);
+int configure_wide_kernels();
 // dst = (D) src on an n x nrhs block
 template <typename S, typename D>
 void launch_convert(int n, int nrhs, const S *src, int64_t lds, D *dst, int64_t ldd, cudaStream_t st);

@@ -111,6 +111,13 @@ struct b200_solver_s {
     std::vector<int> lvl_dt0, lvl_dt1;
     SolveTile *d_dtaskb = nullptr;      // and backward (upper triangle of the transpose)
     std::vector<int> lvl_db0, lvl_db1;
+    // sweeps of many right-hand sides: tiles over the cblks of more than WIDE_LEAF columns,
+    // and the narrower cblks
+    WideTask *d_wide[4] = {};           // off-diagonal forward, backward, diagonal forward, backward
+    int *d_wleaf = nullptr;
+    std::vector<int> lvl_wide[4], lvl_wleaf;  // nlev + 1 offsets each
+    WideFlow wflow{};                   // the levels from wflow_level up, one launch per sweep
+    int wflow_level = 0;
     int *d_leaf = nullptr;              // cblks of <= 32 columns, solved by the one-warp kernel
     std::vector<int> lvl_lf0, lvl_lf1;
     // inverses of the diagonal blocks: W_L (forward sweep) and, for LU, W_U (backward)
@@ -753,6 +760,102 @@ int build_schedule(b200_solver_t *s) {
     RET(s->dupload(&s->d_dtaskb, dtaskb));
     RET(s->dupload(&s->d_leaf, leaf));
     {
+        // Many-right-hand-side tiles.  A tile's K range is as long as the level's number of
+        // tiles allows: full ranges where the level fills the GPU's SMs several times over
+        // (one atomic per output), shorter ones near the root, where few cblks are left
+        constexpr int kFill = 600;
+        constexpr int kWideFlowMin = 8;
+        std::vector<WideTask> w[4];
+        std::vector<int> wleaf;
+        for (int q = 0; q < 4; q++) s->lvl_wide[q].assign(nlev + 1, 0);
+        s->lvl_wleaf.assign(nlev + 1, 0);
+        for (int l = 0; l < nlev; l++) {
+            const Level &L = s->levels[l];
+            for (int i = L.c0; i < L.c1; i++)
+                if (s->ncols[lvl_cblk[i]] <= WIDE_LEAF) wleaf.push_back(lvl_cblk[i]);
+            s->lvl_wleaf[l + 1] = (int)wleaf.size();
+            int64_t ntf = 0, ntb = 0;
+            for (int i = L.c0; i < L.c1; i++) {
+                const int k = lvl_cblk[i], nc = s->ncols[k], m = s->stride[k] - nc;
+                if (nc <= WIDE_LEAF) continue;
+                ntf += (m + 63) / 64;
+                ntb += (int64_t)((nc + 63) / 64) * ((m + 511) / 512);
+            }
+            int kf = 1024, kb = 512;  // K values per tile
+            for (int64_t t = ntf; kf > 64 && t < kFill; kf >>= 1) t = ntf * (L.nmax + kf / 2 - 1) / (kf / 2);
+            for (int64_t t = ntb; kb > 64 && t < kFill; kb >>= 1) t *= 2;
+            for (int i = L.c0; i < L.c1; i++) {
+                const int k = lvl_cblk[i], nc = s->ncols[k], S = s->stride[k];
+                if (nc <= WIDE_LEAF) continue;
+                for (int o = nc & ~3; o < S; o += 64)
+                    for (int c = 0; c < nc; c += kf) w[0].push_back({k, o, c, std::min(nc, c + kf)});
+                for (int r = nc & ~3; r < S; r += kb)
+                    for (int o = 0; o < nc; o += 64) w[1].push_back({k, o, r, std::min(S, r + kb)});
+                for (int o = 0; o < nc; o += 64) {
+                    w[2].push_back({k, o, 0, std::min(nc, o + 64)});
+                    w[3].push_back({k, o, o, nc});
+                }
+            }
+            for (int q = 0; q < 4; q++) s->lvl_wide[q][l + 1] = (int)w[q].size();
+        }
+        // the top of the tree: as long as every level above has few cblks, none of them narrow
+        int wf = nlev;
+        while (wf > 0 && s->levels[wf - 1].c1 - s->levels[wf - 1].c0 < kWideFlowMin &&
+               s->lvl_wleaf[wf] == s->lvl_wleaf[wf - 1])
+            wf--;
+        s->wflow_level = wf;
+        std::vector<FlowItem> fwd, bwd, lf, lb;
+        std::vector<int> flist, need_f(N, 0), need_b(N, 0), nprev_f(N, 0), nprev_b(N, 0), mark(N, -1);
+        int stamp = 0;
+        for (int l = wf; l < nlev; l++)
+            for (int i = s->levels[l].c0; i < s->levels[l].c1; i++) {
+                const int k = lvl_cblk[i], nc = s->ncols[k], S = s->stride[k];
+                lf.clear();
+                lb.clear();
+                for (int r = 0; r < nc; r += 64)
+                    for (int c = 0; c < nc; c += 64) {
+                        if (c <= r) lf.push_back({FI_DIAG, k, r, c, 0, 0});
+                        if (c >= r) lb.push_back({FI_DIAG, k, r, c, 0, 0});
+                    }
+                nprev_f[k] = (int)lf.size();
+                need_b[k] = (int)lb.size();
+                const size_t off0 = lf.size();
+                for (int r = nc & ~3; r < S; r += 64) {
+                    FlowItem it{FI_OFF, k, r, 0, (int)flist.size(), 0};
+                    stamp++;
+                    for (int b = s->fblok[k] + 1; b < s->fblok[k + 1]; b++) {
+                        const int b0 = s->rowoff[b], b1 = b0 + s->lrow[b] - s->frow[b] + 1, f = s->fcblk[b];
+                        if (b1 <= r || b0 >= r + 64 || mark[f] == stamp) continue;
+                        mark[f] = stamp;
+                        flist.push_back(f);
+                        it.nf++;
+                    }
+                    for (int c = 0; c < nc; c += 64) {
+                        it.n = c;
+                        for (int q = 0; q < it.nf; q++) need_f[flist[it.f0 + q]]++;
+                        lf.push_back(it);
+                    }
+                }
+                nprev_b[k] = (int)(lf.size() - off0);
+                fwd.insert(fwd.end(), lf.begin(), lf.end());
+                // backward order: reversed by cblk below
+                bwd.insert(bwd.begin(), lb.begin(), lb.end());
+                bwd.insert(bwd.begin(), lf.begin() + off0, lf.end());
+            }
+        s->wflow.nf = (int)fwd.size();
+        s->wflow.nb = (int)bwd.size();
+        if (flist.empty()) flist.push_back(0);
+        RET(s->dupload(&s->wflow.f, fwd));
+        RET(s->dupload(&s->wflow.b, bwd));
+        RET(s->dupload(&s->wflow.flist, flist));
+        RET(s->dupload(&s->wflow.need_f, need_f));
+        RET(s->dupload(&s->wflow.need_b, need_b));
+        RET(s->dupload(&s->wflow.nprev_f, nprev_f));
+        RET(s->dupload(&s->wflow.nprev_b, nprev_b));
+        RET(s->dupload(&s->d_wleaf, wleaf));
+        for (int q = 0; q < 4; q++) RET(s->dupload(&s->d_wide[q], w[q]));
+    }
+    {
         // dataflow sweep items, level by level (forward bottom-up, backward top-down)
         std::vector<FlowItem> fwd, bwd;
         std::vector<int> flist, need_f(N, 0), need_b(N, 0), nprev_f(N, 0), nprev_b(N, 0);
@@ -1232,12 +1335,111 @@ int enqueue_sweeps(b200_solver_t *s, Lane *ln, T *x, T *aux, int64_t ldx, int nr
     return ERR_SUCCESS;
 }
 
+// Both sweeps of many right-hand sides on row-major vectors, level by level and, up to 64
+// of them, the top of the tree in one dataflow launch per sweep.  The solution's rows lie
+// in aux, the forward result's in x itself, so the workspace is the one of the narrow
+// sweeps; FP32 rows have room for a pitch of 16-byte multiples there, FP64 rows take the
+// pitch (even) that the caller's blocks hold.  x: n x nrhs, leading dimension n.
+template <typename T>
+int enqueue_wide_sweeps(b200_solver_t *s, Lane *ln, double *x, double *aux, int nrhs, int pitch, cudaStream_t st,
+                        int *launches, Trace *tr) {
+    const T *L = (const T *)s->dL, *WL = (const T *)s->dWL;
+    const bool lu = s->facto == FACTO_GETRF;
+    const T *Ub = lu ? (const T *)s->dU : L, *WB = lu ? (const T *)s->dWU : WL;
+    const int n = s->n, N = s->cblknbr, nlev = (int)s->levels.size();
+    const int wf = nrhs <= 64 ? s->wflow_level : nlev;  // the dataflow items take 64 columns at a time
+    // rows on 16-byte boundaries (an FP32 block is half the size of its double one)
+    auto align16 = [](double *p) { return reinterpret_cast<T *>(((uintptr_t)p + 15) & ~(uintptr_t)15); };
+    T *xr = align16(aux), *ar = align16(x);
+    const int ldr = sizeof(T) == 8 ? pitch : (nrhs + 3) / 4 * 4;
+    auto part = [&](int q, int l) { return s->lvl_wide[q][l + 1] - s->lvl_wide[q][l]; };
+    auto first = [&](int q, int l) { return s->d_wide[q] + s->lvl_wide[q][l]; };
+    auto run = [&](int cls, auto &&launch) {
+        if (tr) tr->begin(st);
+        launch();
+        if (tr) tr->end(cls, st);
+        *launches += 1;
+    };
+    // the dataflow launches' tickets, counters and abort word
+    int *fl = ln->d_sflags, *abort_word = fl + 2;
+    const int nflow = wf < nlev ? s->n_active - s->levels[wf].c0 : 0;
+    const int *flow_cblks = s->d_lvl_cblk + (nflow ? s->levels[wf].c0 : 0);
+    if (nflow) {
+        CU(cudaMemsetAsync(fl, 0, ((size_t)4 * N + 4) * sizeof(int), st));
+        if (flow_withheld()) CU(cudaMemsetAsync(fl, 1, 1, st));  // forward ticket = 1
+    }
+    run(1, [&] { launch_wide_transpose<double, T>(n, nrhs, x, n, xr, ldr, 1, st); });
+    for (int l = 0; l < wf; l++) {
+        const int nlf = s->lvl_wleaf[l + 1] - s->lvl_wleaf[l];
+        if (nlf > 0)
+            run(1, [&] {
+                launch_wide_leaf<T>(s->ds, s->d_wleaf + s->lvl_wleaf[l], nlf, L, WL, s->d_woff, xr, ar, ldr, nrhs, 0, st);
+            });
+        if (part(2, l) > 0)
+            run(1, [&] { launch_wide_diag<T>(s->ds, first(2, l), part(2, l), WL, s->d_woff, xr, ar, ldr, nrhs, 0, st); });
+        if (part(0, l) > 0)
+            run(1, [&] { launch_wide_off<T>(s->ds, first(0, l), part(0, l), L, ar, xr, ldr, nrhs, 0, st); });
+    }
+    if (nflow) {
+        run(1, [&] { launch_wide_zero<T>(s->ds, flow_cblks, nflow, ar, ldr, nrhs, st); });
+        run(1, [&] {
+            launch_wide_flow<T>(s->ds, s->wflow, L, WL, s->d_woff, xr, ar, ldr, nrhs, 0, fl, fl + 4, fl + 4 + N,
+                                abort_word, ln->d_serr, st);
+        });
+    }
+    if (s->facto == FACTO_SYTRF)
+        run(3, [&] { launch_wide_scale<T>(s->ds, s->d_lvl_cblk, s->n_active, L, ar, ldr, nrhs, st); });
+    if (nflow) {
+        run(2, [&] { launch_wide_zero<T>(s->ds, flow_cblks, nflow, xr, ldr, nrhs, st); });
+        run(2, [&] {
+            launch_wide_flow<T>(s->ds, s->wflow, Ub, WB, s->d_woff, xr, ar, ldr, nrhs, 1, fl + 1, fl + 4 + 2 * N,
+                                fl + 4 + 3 * N, abort_word, ln->d_serr, st);
+        });
+    }
+    for (int l = wf - 1; l >= 0; l--) {
+        const int nlf = s->lvl_wleaf[l + 1] - s->lvl_wleaf[l];
+        if (nlf > 0)
+            run(2, [&] {
+                launch_wide_leaf<T>(s->ds, s->d_wleaf + s->lvl_wleaf[l], nlf, Ub, WB, s->d_woff, xr, ar, ldr, nrhs, 1, st);
+            });
+        if (part(1, l) > 0)
+            run(2, [&] { launch_wide_off<T>(s->ds, first(1, l), part(1, l), Ub, xr, ar, ldr, nrhs, 1, st); });
+        if (part(3, l) > 0)
+            run(2, [&] { launch_wide_diag<T>(s->ds, first(3, l), part(3, l), WB, s->d_woff, ar, xr, ldr, nrhs, 1, st); });
+    }
+    run(2, [&] { launch_wide_transpose<T, double>(n, nrhs, xr, ldr, x, n, 0, st); });
+    CU(cudaGetLastError());
+    return ERR_SUCCESS;
+}
+
 // Sweeps on the permuted block x (double, leading dimension ldx) with the scratch
 // aux (n x nrhs doubles).  An FP32 factor runs the sweeps in FP32 -- they apply the
 // preconditioner of an FP64 refinement -- on two n x nrhs float blocks held in aux,
 // converted from and back to x.
+// Many right-hand sides take the row-major sweeps (pitch: columns that both blocks have room
+// for; FP64 rows need an even number).  From 8 on: below, their tiles of 16 columns are mostly
+// padding.  FP32 on larger systems from 48 on: there the column-major tiles fill the GPU at
+// every level, and 3xTF32 issues three products for each of the (padded) columns.  Solves on
+// B200, column-major / row-major (ms):
+//   FP64  12^3  8: 0.32 / 0.25, 33: 0.75 / 0.33;  80^3  8: 4.33 / 3.65, 17: 5.93 / 5.06, 40:
+//         8.76 / 7.55;  100^3  256: 89.2 / 58.0
+//   FP32  24^3  8: 0.45 / 0.35, 48: 1.03 / 0.53;  44^3  8: 0.76 / 0.75, 17: 1.13 / 1.01;  52^3
+//         27-point  8: 1.46 / 1.15, 33: 2.93 / 2.07
+//         60^3  8: 1.29 / 1.45, 17: 1.91 / 2.10, 40: 2.76 / 2.74;  90^3  17: 5.98 / 6.51, 40:
+//         8.80 / 8.92, 48: 9.58 / 9.45;  100^3  64: 18.1 / 15.5
+constexpr int WIDE_MIN_NRHS = 8, WIDE_MIN_NRHS_F32 = 48, WIDE_SMALL_N = 180000;
+
+inline bool wide_wanted(const b200_solver_t *s, int nrhs) {
+    return nrhs >= (s->f32 && s->n > WIDE_SMALL_N ? WIDE_MIN_NRHS_F32 : WIDE_MIN_NRHS);
+}
+
 int sweeps(b200_solver_t *s, Lane *ln, double *x, double *aux, int64_t ldx, int nrhs, cudaStream_t st,
-           int *launches, Trace *tr = nullptr) {
+           int *launches, Trace *tr = nullptr, int pitch = 0) {
+    if (pitch < nrhs) pitch = nrhs;
+    const bool fits = s->f32 || (pitch % 2 == 0 && ((uintptr_t)x | (uintptr_t)aux) % 16 == 0);
+    if (wide_wanted(s, nrhs) && ldx == s->n && s->n_active == s->cblknbr && fits)
+        return s->f32 ? enqueue_wide_sweeps<float>(s, ln, x, aux, nrhs, pitch, st, launches, tr)
+                      : enqueue_wide_sweeps<double>(s, ln, x, aux, nrhs, pitch, st, launches, tr);
     if (!s->f32) return enqueue_sweeps<double>(s, ln, x, aux, ldx, nrhs, st, launches, tr);
     float *xf = reinterpret_cast<float *>(aux), *af = xf + (size_t)s->n * nrhs;
     launch_convert<double, float>(s->n, nrhs, x, ldx, xf, s->n, st);
@@ -1285,11 +1487,12 @@ int sweep_step(b200_solver_t *s, Lane *ln, double *x, double *aux, int64_t ldx, 
 // the sweeps' scratch.
 int solve_device(b200_solver_t *s, Lane *ln, int nrhs, double *b, int64_t ldb, cudaStream_t st) {
     const int n = s->n;
-    RET(ensure_ws(ln, (size_t)2 * n * nrhs));
-    double *xp = ln->d_ws, *aux = ln->d_ws + (size_t)n * nrhs;
+    const int pitch = !s->f32 && wide_wanted(s, nrhs) ? (nrhs + 1) / 2 * 2 : nrhs;  // even FP64 rows for the row-major sweeps
+    RET(ensure_ws(ln, (size_t)2 * n * pitch));
+    double *xp = ln->d_ws, *aux = ln->d_ws + (size_t)n * pitch;
     int launches = 2;
     launch_permute(n, nrhs, s->d_peri, b, ldb, xp, n, 1, st);
-    RET(sweeps(s, ln, xp, aux, n, nrhs, st, &launches));
+    RET(sweeps(s, ln, xp, aux, n, nrhs, st, &launches, nullptr, pitch));
     launch_permute(n, nrhs, s->d_peri, xp, n, b, ldb, 0, st);
     CU(cudaGetLastError());
     ln->launches_solve = launches;
@@ -1829,7 +2032,7 @@ int b200_solver_create_tuned(const b200_symbol_t *sym, int facto, int precision,
     int rc = ERR_SUCCESS;
     s->trsm_smem = configure_factor_kernels();
     if (s->trsm_smem < 0 || configure_solve_kernels() < 0 || configure_inverse_kernels() < 0 ||
-        configure_panel_kernels() < 0 || (s->use_tc && configure_tc_kernels() < 0)) {
+        configure_panel_kernels() < 0 || configure_wide_kernels() < 0 || (s->use_tc && configure_tc_kernels() < 0)) {
         fprintf(stderr, "pastix_b200: cannot configure the shared memory of the kernels\n");
         rc = ERR_INTERNAL;
     }

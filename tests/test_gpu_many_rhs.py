@@ -1,0 +1,60 @@
+"""Sweeps of many right-hand sides (row-major vectors, the dataflow launch of the narrow
+top of the tree up to 64 of them): every width class of the tiles (16, 32, 48, 64 columns),
+odd and ragged numbers, cblks from 1 to 200 columns, against x_true (FP64) and the same
+factor's solutions one at a time (FP32).  Analysis of perf/cases.py, no PaStiX library."""
+import numpy as np
+import pytest
+
+from pastix_b200 import native
+from test_gpu_wide_panels import analysis
+
+pytestmark = pytest.mark.gpu
+
+CASES = [("potrf", 7, (20, 20, 20), 0.0), ("sytrf", 7, (13, 12, 17), -0.05), ("getrf", 7, (15, 18, 11), 0.0),
+         ("potrf", 27, (9, 23, 10), 1e-3), ("sytrf", 7, (37, 41, 1), -0.01)]
+
+
+def factored(facto, points, dims, shift, prec):
+    st, bc, _, _ = analysis(facto, points, dims, shift)
+    s = native.Solver(st, facto, prec)
+    s.bcsc_load(bc)
+    s.numfact(1e-8)
+    return st, s
+
+
+@pytest.mark.parametrize("facto,points,dims,shift", CASES)
+def test_fp64_solutions(facto, points, dims, shift):
+    st, s = factored(facto, points, dims, shift, "fp64")
+    rng = np.random.default_rng(5)
+    for nrhs in (8, 9, 16, 17, 31, 34, 48, 50, 64, 65, 130):
+        xt = rng.uniform(-1.0, 1.0, (st.n, nrhs))
+        x = s.solve(s.spmv(xt))
+        err = np.linalg.norm(x - xt, axis=0) / np.linalg.norm(xt, axis=0)
+        # rounding times the conditioning of the shifted systems, every column
+        assert err.max() <= 1e-10, nrhs
+    s.close()
+
+
+@pytest.mark.parametrize("facto,points,dims,shift", CASES)
+def test_fp32_solutions_equal_one_at_a_time(facto, points, dims, shift):
+    st, s = factored(facto, points, dims, shift, "fp32")
+    b = np.asfortranarray(np.random.default_rng(6).uniform(-1.0, 1.0, (st.n, 67)))
+    one = np.stack([s.solve(b[:, j]) for j in range(67)], axis=1)
+    for nrhs in (8, 11, 16, 18, 32, 33, 47, 49, 64, 67):
+        x = s.solve(b[:, :nrhs])
+        d = np.linalg.norm(x - one[:, :nrhs], axis=0) / np.linalg.norm(one[:, :nrhs], axis=0)
+        # two summation orders of the same FP32 products: FP32 rounding times the growth
+        # of the indefinite systems' solutions
+        assert d.max() <= 2e-3, nrhs
+        assert np.median(d) <= 1e-4, nrhs
+    s.close()
+
+
+def test_refinement_of_many_right_hand_sides():
+    st, s = factored("potrf", 7, (20, 20, 20), 0.0, "tf32x3")
+    xt = np.random.default_rng(7).uniform(-1.0, 1.0, (st.n, 21))
+    b = s.spmv(xt)
+    x, nit, berr = s.refine(b, s.solve(b), "cg")
+    s.close()
+    assert berr.max() <= 1e-12 and nit <= 3
+    assert np.linalg.norm(x - xt) <= 1e-8 * np.linalg.norm(xt)
