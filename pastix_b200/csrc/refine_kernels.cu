@@ -4,28 +4,34 @@
 #include "b200_internal.h"
 #include "kernels.h"
 
+#include <type_traits>
+
 namespace b200 {
 
 // y = alpha * A x + beta * y.  The matrix is the bcsc in the permuted basis, read
 // row-wise: for a symmetric matrix the bcsc columns hold both triangles so column
 // i is row i; for a general matrix the values passed are A^T in the same pattern
 // (Uvalues), whose column i is row i of A (bcsc/bcsc_zspmv.c:127-240).
-// One warp per row.
+// W lanes per row, 32 / W rows per warp.  Bound by the latency of a row's three dependent
+// loads, so rows in flight are what counts: as many lanes as an average row has entries
+// (launch_spmv).  With a warp per row 27 of 32 lanes idled on a 5-point matrix: 2.0 M rows of
+// 5 entries 596 us, with 8 lanes 122 us.
+template <int W>
 __global__ void __launch_bounds__(256) spmv_kernel(int n, int nrhs, const int64_t *__restrict__ colptr,
                                                    const int *__restrict__ rowtab, const double *__restrict__ vals,
                                                    const double *__restrict__ x, int64_t ldx, double *y, int64_t ldy,
                                                    double alpha, double beta) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= n) return;
-    const int64_t e0 = colptr[warp], e1 = colptr[warp + 1];
+    const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / W;
+    const int lane = threadIdx.x & (W - 1);
+    const bool in = row < n;  // the lanes past the last row stay for the warp's shuffles
+    const int64_t e0 = in ? colptr[row] : 0, e1 = in ? colptr[row + 1] : 0;
     for (int r = 0; r < nrhs; r++) {
         double acc = 0.0;
-        for (int64_t e = e0 + lane; e < e1; e += 32) acc += vals[e] * x[rowtab[e] + r * ldx];
+        for (int64_t e = e0 + lane; e < e1; e += W) acc += vals[e] * x[rowtab[e] + r * ldx];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) {
-            double *yp = y + warp + r * ldy;
+        for (int o = W / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (in && lane == 0) {
+            double *yp = y + row + r * ldy;
             *yp = (beta == 0.0) ? alpha * acc : alpha * acc + beta * *yp;
         }
     }
@@ -186,7 +192,7 @@ __global__ void __launch_bounds__(256) spmv_rows_kernel(int n, int R, const int6
     }
 }
 
-void launch_spmv(int n, int nrhs, const int64_t *colptr, const int *rowtab, const double *vals, const double *x,
+void launch_spmv(int n, int64_t nnz, int nrhs, const int64_t *colptr, const int *rowtab, const double *vals, const double *x,
                  int64_t ldx, double *y, int64_t ldy, double alpha, double beta, cudaStream_t st, double *xt) {
     if (n <= 0) return;
     if (nrhs > 1 && xt) {
@@ -197,8 +203,18 @@ void launch_spmv(int n, int nrhs, const int64_t *colptr, const int *rowtab, cons
                                                                               y + (int64_t)r0 * ldy, ldy, alpha, beta);
         }
     } else {
-        spmv_kernel<<<nblk((int64_t)n * 32, 256), 256, 0, st>>>(n, nrhs, colptr, rowtab, vals, x, ldx, y, ldy, alpha,
-                                                                 beta);
+        auto run = [&](auto w) {
+            constexpr int W = decltype(w)::value;
+            spmv_kernel<W><<<nblk((int64_t)n * W, 256), 256, 0, st>>>(n, nrhs, colptr, rowtab, vals, x, ldx, y, ldy,
+                                                                      alpha, beta);
+        };
+        // the smallest power of two that covers an average row: fewer lanes would take a row
+        // in several steps, more would idle
+        const int64_t avg = (nnz + n - 1) / n;
+        if (avg <= 4) run(std::integral_constant<int, 4>{});
+        else if (avg <= 8) run(std::integral_constant<int, 8>{});
+        else if (avg <= 16) run(std::integral_constant<int, 16>{});
+        else run(std::integral_constant<int, 32>{});
     }
 }
 

@@ -1517,7 +1517,7 @@ struct RefineCtx {
     int spmv(const double *x, double *y, double alpha, double beta) {
         const double *vals = (s->facto == FACTO_GETRF) ? s->d_Uv : s->d_Lv;
         if (nrhs > 1 && !ln->d_xt) RET(dalloc(&ln->d_xt, (size_t)n * 16));
-        launch_spmv(n, nrhs, s->d_colptr, s->d_rowtab, vals, x, n, y, n, alpha, beta, st, ln->d_xt);
+        launch_spmv(n, s->nnz, nrhs, s->d_colptr, s->d_rowtab, vals, x, n, y, n, alpha, beta, st, ln->d_xt);
         s->kernel_launches += nrhs > 1 ? 2 * ((nrhs + 15) / 16) : 1;
         return ERR_SUCCESS;
     }
@@ -2768,7 +2768,7 @@ int b200_spmv(b200_solver_t *s, int64_t nrhs, double alpha, const double *x, int
         const double *vals = (s->facto == FACTO_GETRF) ? s->d_Uv : s->d_Lv;
         if (nrhs > 1 && !s->main.d_xt && dalloc(&s->main.d_xt, (size_t)n * 16)) rc = ERR_OOM;
         if (!rc)
-            launch_spmv(n, (int)nrhs, s->d_colptr, s->d_rowtab, vals, px, n, py, n, alpha, beta, s->st, s->main.d_xt);
+            launch_spmv(n, s->nnz, (int)nrhs, s->d_colptr, s->d_rowtab, vals, px, n, py, n, alpha, beta, s->st, s->main.d_xt);
         launch_permute(n, (int)nrhs, s->d_peri, py, n, dy, n, 0, s->st);
         if (cudaMemcpy2DAsync(y, ldy * sizeof(double), dy, n * sizeof(double), n * sizeof(double), nrhs,
                               cudaMemcpyDeviceToHost, s->st) != cudaSuccess) rc = ERR_INTERNAL;
@@ -2793,7 +2793,7 @@ int b200_spmv_device(b200_solver_t *s, int64_t nrhs, double alpha, const double 
     const double *vals = (s->facto == FACTO_GETRF) ? s->d_Uv : s->d_Lv;
     launch_permute(n, (int)nrhs, s->d_peri, d_x, ldx, px, n, 1, st);
     launch_permute(n, (int)nrhs, s->d_peri, d_y, ldy, py, n, 1, st);
-    launch_spmv(n, (int)nrhs, s->d_colptr, s->d_rowtab, vals, px, n, py, n, alpha, beta, st, ln->d_xt);
+    launch_spmv(n, s->nnz, (int)nrhs, s->d_colptr, s->d_rowtab, vals, px, n, py, n, alpha, beta, st, ln->d_xt);
     launch_permute(n, (int)nrhs, s->d_peri, py, n, d_y, ldy, 0, st);
     CU(cudaGetLastError());
     s->kernel_launches += 3 + (nrhs > 1 ? 2 * ((nrhs + 15) / 16) : 1);
