@@ -1,5 +1,5 @@
 """The refinement's kernels on an analysis that needs no PaStiX library: the matrix-vector
-product with 4, 8, 16 and 32 lanes per row."""
+product with 4, 8, 16 and 32 lanes per row, and GMRES over restarts."""
 import numpy as np
 import pytest
 
@@ -27,4 +27,21 @@ def test_spmv_lanes(points, dims, facto):
     # alpha and beta, two roundings more on terms of twice and three times the size
     y = s.spmv(xt[:, 0], 2.0, -3.0, b[:, 0])
     assert np.abs(y + b[:, 0]).max() <= 6 * tol
+    s.close()
+
+
+@pytest.mark.parametrize("im", [1, 2, 25])
+@pytest.mark.parametrize("facto,shift", [("getrf", 0.0), ("sytrf", -0.05)])
+def test_gmres_restarts(facto, shift, im):
+    st, bc, xt, b = analysis(facto, 7, (17, 16, 15), shift)
+    s = native.Solver(st, facto, "fp32")
+    s.bcsc_load(bc)
+    s.numfact(1e-8)
+    x, it, berr = s.refine(b, s.solve(b), "gmres", eps=1e-12, itermax=60, gmres_im=im)
+    assert it <= 60 and np.all(np.asarray(berr) <= 1e-12)
+    # the reported error is the recurrence's; the true residual adds the roundings of a few
+    # products of A x, below 1e-13 of |b| here
+    for j in range(2):
+        r = np.linalg.norm(b[:, j] - s.spmv(x[:, j])) / np.linalg.norm(b[:, j])
+        assert r <= 1.2e-12
     s.close()
