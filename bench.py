@@ -511,7 +511,7 @@ def main():
     except Exception:
         peak = None
     achieved = dk["flops"] / (dk["ms"] * 1e-3) / 1e12 if dk["ms"] > 0 else 0.0
-    kname = {"update": "update_f64_kernel" if head["prec"] == "fp64" else "update_simt_f32_kernel",
+    kname = {"update": "update_tile_kernel<double>" if head["prec"] == "fp64" else "update_tile_kernel<float>",
              "panel": "panel_kernel",
              "tc_update": "update_tc_kernel<%d>" % (1 if head["prec"] == "tf32x3" else 0),
              "tree_bottom": "dag_bottom_kernel"}[dom]
