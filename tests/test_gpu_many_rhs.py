@@ -11,7 +11,7 @@ from test_gpu_wide_panels import analysis
 pytestmark = pytest.mark.gpu
 
 CASES = [("potrf", 7, (20, 20, 20), 0.0), ("sytrf", 7, (13, 12, 17), -0.05), ("getrf", 7, (15, 18, 11), 0.0),
-         ("potrf", 27, (9, 23, 10), 1e-3), ("sytrf", 7, (37, 41, 1), -0.01)]
+         ("potrf", 27, (9, 23, 10), 1e-3), ("sytrf", 7, (37, 41, 1), -0.01), ("potrf", 7, (7, 1, 1), 0.01)]
 
 
 def factored(facto, points, dims, shift, prec):
