@@ -49,8 +49,10 @@ __device__ __forceinline__ void mma_tf32_k8(float (&c)[4], const uint32_t (&a)[4
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
+// x = hi + lo: hi is x rounded to TF32's 11 bits (half an ulp added, the rest masked), so lo
+// has either sign and the bit of it that the tensor core drops is not one-sided.
 __device__ __forceinline__ void split_tf32(float x, uint32_t &hi, uint32_t &lo) {
-    hi = __float_as_uint(x) & 0xFFFFE000u;
+    hi = (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u;
     lo = __float_as_uint(x - __uint_as_float(hi));
 }
 
@@ -111,23 +113,22 @@ struct WideTile {
     }
 };
 
-// FP32: 3xTF32 on mma.sync m16n8k8 (x = hi + lo with hi exact in TF32), the narrow sweeps'
-// arithmetic, warp = 16 outputs x all columns.  The tensor cores' sums of a stage (32 K
-// values; the narrow tiles' 64) are added to the tile's in FP32: one accumulator over a
-// whole K range of 320 rounds worse (the residual after one CG iteration at 80^3 rose from
-// 6.6e-13 to 9.3e-13 and took a second iteration).  Plain multiply-adds (8 x 4 and 8 x 8 sums per thread) are bound by their
-// shared-memory reads and were slower.
+// FP32: 3xTF32 on mma.sync m16n8k8 (x = hi + lo, both in TF32), warp = 16 outputs x all
+// columns.  The tensor core rounds its sums towards zero, which adds up over products of one
+// sign: every 8 products start from zero, the small correction products first, and join the
+// tile's sum in FP32.  The solutions' error against the 64-bit solve with the same FP32
+// factor (b > 0, 40 x 41 x 39): 5.1e-7, the column-major tiles' 5.0e-6; a truncated hi, and
+// sums over 32 products with the correction products in them, had 9.3e-6, and took 4.5 %
+// less time (100^3, 64 right-hand sides, solve and CG: 53.3 ms, 55.8 now).  Plain
+// multiply-adds (8 x 4 and 8 x 8 sums per thread) are bound by their shared-memory reads and
+// were slower.
 template <int MODE, int NT>
 struct WideTile<float, MODE, NT> {
     using SM = WideSmem<float, MODE, NT>;
-    // the correction products' own accumulators where the registers allow 4 CTAs per SM
-    static constexpr bool OWN_COR = NT < 8;
-    static constexpr int NC = OWN_COR ? NT : 1;
-    float sum[NT][4] = {}, cor[NC][4] = {};
+    float sum[NT][4] = {};
     __device__ __forceinline__ void mul(const float *ms, const float *xs, int nout, int ntn) {
         const int lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3, o0w = (threadIdx.x >> 5) * 16;
         if (o0w >= nout) return;
-        float acc[NT][4] = {};
 #pragma unroll
         for (int kk = 0; kk < WK; kk += 8) {
             uint32_t ah[4], al[4];
@@ -142,21 +143,15 @@ struct WideTile<float, MODE, NT> {
                     uint32_t bh[2], bl[2];
                     split_tf32(xs[(kk + tg) * SM::XP + nt * 8 + g], bh[0], bl[0]);
                     split_tf32(xs[(kk + tg + 4) * SM::XP + nt * 8 + g], bh[1], bl[1]);
-                    mma_tf32_k8(acc[nt], ah, bh);
-                    if constexpr (OWN_COR) {
-                        mma_tf32_k8(cor[nt], ah, bl);
-                        mma_tf32_k8(cor[nt], al, bh);
-                    } else {
-                        mma_tf32_k8(acc[nt], ah, bl);
-                        mma_tf32_k8(acc[nt], al, bh);
-                    }
+                    float t[4] = {};
+                    mma_tf32_k8(t, al, bh);
+                    mma_tf32_k8(t, ah, bl);
+                    mma_tf32_k8(t, ah, bh);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) sum[nt][e] += t[e];
                 }
             }
         }
-#pragma unroll
-        for (int nt = 0; nt < NT; nt++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) sum[nt][e] += acc[nt][e];
     }
     __device__ __forceinline__ void out(float *os) {
         const int lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3, o0w = (threadIdx.x >> 5) * 16;
@@ -164,8 +159,7 @@ struct WideTile<float, MODE, NT> {
         for (int nt = 0; nt < NT; nt++)
 #pragma unroll
             for (int e = 0; e < 4; e++)
-                os[(o0w + g + (e >> 1) * 8) * SM::OP + nt * 8 + 2 * tg + (e & 1)] =
-                    OWN_COR ? sum[nt][e] + cor[nt % NC][e] : sum[nt][e];
+                os[(o0w + g + (e >> 1) * 8) * SM::OP + nt * 8 + 2 * tg + (e & 1)] = sum[nt][e];
     }
 };
 

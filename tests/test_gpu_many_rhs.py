@@ -5,7 +5,9 @@ factor's solutions one at a time (FP32).  Analysis of perf/cases.py, no PaStiX l
 import numpy as np
 import pytest
 
+import oracle
 from pastix_b200 import native
+from perf import cases as C
 from test_gpu_wide_panels import analysis
 
 pytestmark = pytest.mark.gpu
@@ -58,3 +60,29 @@ def test_refinement_of_many_right_hand_sides():
     s.close()
     assert berr.max() <= 1e-12 and nit <= 3
     assert np.linalg.norm(x - xt) <= 1e-8 * np.linalg.norm(xt)
+
+
+# cblks of 9 to 32 columns (the 2D grids) and wider ones, of M-matrices and an indefinite system
+@pytest.mark.parametrize("facto,points,dims,shift", [("potrf", 7, (20, 20, 20), 0.0), ("potrf", 27, (20, 21, 19), 1e-3),
+                                                     ("potrf", 7, (70, 70, 1), 0.0), ("getrf", 7, (22, 20, 21), 0.0),
+                                                     ("sytrf", 7, (60, 70, 1), 0.01)])
+@pytest.mark.parametrize("low", [-1.0, 0.0])
+def test_fp32_many_as_accurate_as_few(facto, points, dims, shift, low):
+    # both forms against the 64-bit solve with the same FP32 factor; right-hand sides of one
+    # sign give products of one sign, whose rounding must not be one-sided either
+    st, s = factored(facto, points, dims, shift, "fp32")
+    f = C.FACTO_ID[facto]
+    b = np.asfortranarray(np.random.default_rng(8).uniform(low, 1.0, (st.n, 64)))
+    exact = oracle.Oracle(st).solve(f, *s.factor(), b)
+
+    def error(nrhs):  # rms over the columns of the relative errors
+        x = np.concatenate([s.solve(np.asfortranarray(b[:, i:i + nrhs])).reshape(st.n, -1)
+                            for i in range(0, 64 - nrhs + 1, nrhs)], axis=1)
+        d = np.linalg.norm(x - exact[:, :x.shape[1]], axis=0) / np.linalg.norm(exact[:, :x.shape[1]], axis=0)
+        return np.sqrt((d ** 2).mean())
+
+    few = error(4)
+    # the same roundings in another order: a tenth for the sample
+    for nrhs in (8, 16, 17, 40, 64):
+        assert error(nrhs) <= 1.1 * few, nrhs
+    s.close()
