@@ -36,14 +36,12 @@ void launch_panel(int facto, const DevSym &s, const PanelCblk *pcb, const PanelI
 // the row-block form (one item per row block, resident in shared memory for all
 // steps): items = the diagonal blocks' 64-row blocks first, then the rb-row blocks
 // below, for LU one item per side (PanelItem::j: 0 L, 1 U^T); nsmax = the most
-// 64-column steps of a cblk of the launch; solved_v counts LU's side 1; WL / woff: the
-// arena of the diagonal-block inverses, where POTRF keeps its tiles' inverses (the
-// inverse launch rewrites it); panel_rows_block gives the rb (128 or 64) whose blocks of
-// such a cblk fit in shared memory, 0 if none does
+// 64-column steps of a cblk of the launch; solved_v counts LU's side 1; panel_rows_block
+// gives the rb (128 or 64) whose blocks of such a cblk fit in shared memory, 0 if none does
 template <typename T>
 void launch_panel_rows(int facto, const DevSym &s, const PanelCblk *pcb, const PanelItem *items, int nitems,
-                       int nsmax, int rb, int *ticket, int *solved, int *solved_v, int *abort_word, T *L, T *U, T *WL,
-                       const int64_t *woff, const double *thr, unsigned long long *npiv, int *err, cudaStream_t st);
+                       int nsmax, int rb, int *ticket, int *solved, int *solved_v, int *abort_word, T *L, T *U,
+                       const double *thr, unsigned long long *npiv, int *err, cudaStream_t st);
 int panel_rows_block(int nsmax, size_t esz);
 int configure_panel_kernels();
 // the diagonal of the factor's diagonal blocks, in the permuted numbering (n doubles)

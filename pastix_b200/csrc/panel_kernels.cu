@@ -118,20 +118,40 @@ __device__ __forceinline__ void store4(T *p, T a, T b, T c, T d) {
 // LU keeps unit L below and U on and above the diagonal (its row strip is solved with the
 // unit block by the threads that read it).
 //
-// POTRF: the blocks above the diagonal (tx < ty), idle otherwise, carry the inverse W of
-// the tile: they hold W[ty, tx]^T, start from zero and take the same step (their strip is
-// their own raw block, the identity in step tx), and wdiag is the diagonal block of W.
-// strip: 2 x STRIP elements.
+// An entry gathers the products of the 16-column blocks before its own from zero (its value
+// waits in a slot of the strip's) and takes their sum in one subtraction when its own block's
+// turn comes: 64 products subtracted one by one from the entry itself rounded 1.2 to 1.4 times
+// worse than 32-column tiles (backward error of dense LU and LDL^T; twice in
+// the factor of an indefinite 44 x 40 x 39 system).
+// strip: 2 x STRIP elements, then 16 for each of 144 threads.
 template <typename T, int FACTO>
-__device__ void factor_tile_regs(T (&acc)[4][4], T (&wdiag)[4][4], int wd, T *strip, double thr, int *s_piv,
-                                 int *s_err) {
+__device__ void factor_tile_regs(T (&acc)[4][4], int wd, T *strip, double thr, int *s_piv, int *s_err) {
     constexpr int STRIP = 8 * PB;  // 4 solved columns, then LU's 4 raw rows; LDL^T's 4 pivots
     constexpr bool LU = FACTO == FACTO_GETRF;
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     int piv = 0, neg = 0;
+    constexpr int SLOTS = 144;
+    const int turn = min(tx, ty) & ~3;  // the step at which the entry's own 16-column block begins
+    const bool late = turn > 0 && 4 * turn < wd;
+    T *slot = strip + 2 * STRIP + (tx - 4) + 12 * (ty - 4);  // this thread's, every SLOTS elements
+    if (late) {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                slot[SLOTS * (4 * i + q)] = acc[i][q];
+                acc[i][q] = 0;
+            }
+    }
 #pragma unroll 1
     for (int p = 0; 4 * p < wd; p++) {
         T *cb = strip + (p & 1) * STRIP, *rb = cb + 4 * PB;
+        if (p == turn && late) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) acc[i][q] += slot[SLOTS * (4 * i + q)];
+        }
         if (ty == p) {
             const unsigned half = 0xffffu << (16 * (p & 1));
             T g[4][4], P[4][4], d[4], iv[4];
@@ -140,7 +160,7 @@ __device__ void factor_tile_regs(T (&acc)[4][4], T (&wdiag)[4][4], int wd, T *st
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     if (LU || i >= k) g[i][k] = __shfl_sync(half, acc[i][k], p, 16);
-                    P[i][k] = (FACTO == FACTO_POTRF && tx == p) ? (i == k ? (T)1 : (T)0) : acc[i][k];
+                    P[i][k] = acc[i][k];
                 }
 #pragma unroll
             for (int c = 0; c < 4; c++) {
@@ -195,11 +215,9 @@ __device__ void factor_tile_regs(T (&acc)[4][4], T (&wdiag)[4][4], int wd, T *st
 #pragma unroll
                 for (int i = 0; i < 4; i++)
 #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        if (FACTO == FACTO_POTRF) wdiag[i][k] = P[i][k];
+                    for (int k = 0; k < 4; k++)
                         if (LU || i >= k) acc[i][k] = g[i][k];
-                    }
-            } else if (tx > p || FACTO == FACTO_POTRF) {
+            } else if (tx > p) {
 #pragma unroll
                 for (int i = 0; i < 4; i++)
 #pragma unroll
@@ -212,7 +230,7 @@ __device__ void factor_tile_regs(T (&acc)[4][4], T (&wdiag)[4][4], int wd, T *st
         }
         __syncthreads();
         if (ty <= p) continue;
-        if (LU ? tx < p : !(tx >= ty || (FACTO == FACTO_POTRF && tx <= p))) continue;
+        if (LU ? tx < p : tx < ty) continue;
         T P[4][4], Q[4][4];  // [row][k], [column][k]
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -281,94 +299,87 @@ __device__ __forceinline__ void load_tile_regs(T (&acc)[4][4], int wd, Load a) {
 }
 
 // Solve of the R rows of xs (64 columns, pitch XP) against the lower triangular tile lt
-// (lt[c + l * 64], l < c; identity past the step's width) by substitution in 4-column
-// blocks over the CTA's threads, thread (tx, ty) rows 4 tx + 64 h .. and columns 4 ty ..:
-// the half-warp of block column p solves its columns against the 4 x 4 diagonal block and
-// puts them in the strip (inside xs, whose values are in registers); after one barrier the
-// threads right of it subtract their product with the tile.  x_c = (a_c - sum_{l<c} x_l
-// t_cl) * rdiag[c]; LDL^T then multiplies by dinv[c] = 1 / D_c.  All PT threads; xs final
-// after the closing barrier.
+// (lt[c + l * 64], l < c; identity past the step's width), x_c = (a_c - sum_{l<c} x_l t_cl)
+// * rdiag[c], LDL^T then times dinv[c] = 1 / D_c, in 16-column blocks: one thread per row
+// substitutes the block's columns in registers, then the threads of the columns right of it
+// (thread (tx, ty): rows 4 tx + 64 h .., columns 4 ty ..) add its products to their sums,
+// which are subtracted when the columns' own block comes.  A block's substitution keeps one
+// warp per SM sub-partition busy (R = 128), its chain of 16 columns no longer than its
+// multiply-adds; 4-column blocks of the threads (tx, ty), with 16 hand-offs, took 29.2 ms at
+// 80^3 27-point split BF16 (28.2 now) and 20.4 ms for the 64^3 LU (19.9).  All PT threads; xs final after the closing barrier.
 template <typename T, int FACTO, int R, int XP>
 __device__ void trsm_tile(T *xs, const T *lt, const T *rdiag, const T *dinv) {
-    constexpr int G = R / 64;  // groups of 64 rows
+    constexpr int G = R / 64, CB = 16;  // groups of 64 rows; columns of a block
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    T acc[G][4][4];  // [group][row][column]
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-#pragma unroll
-        for (int h = 0; h < G; h++) {
-            T v[4];
-            load4(xs + 4 * tx + 64 * h + (4 * ty + q) * XP, v);
-#pragma unroll
-            for (int i = 0; i < 4; i++) acc[h][i][q] = v[i];
-        }
-    __syncthreads();
+    T *own = xs + 4 * tx + 4 * ty * XP;
+    T acc[G][4][4] = {};  // [group][row][column]
 #pragma unroll 1
-    for (int p = 0; p < 16; p++) {
-        T *st = xs + (p & 1) * 4 * R;
-        if (ty == p) {
-            T g[4][4], rd[4];
+    for (int c0 = 0; c0 < PB; c0 += CB) {
+        if (c0 > 0) {
+            if (4 * ty / CB == c0 / CB) {
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                T v[4];
-                load4(lt + 4 * p + (4 * p + k) * PB, v);
+                for (int q = 0; q < 4; q++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) g[j][k] = v[j];
-            }
-            load4(rdiag + 4 * p, rd);
-#pragma unroll
-            for (int h = 0; h < G; h++) {
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        acc[h][i][k] *= rd[k];
-#pragma unroll
-                        for (int j = k + 1; j < 4; j++) acc[h][i][j] -= acc[h][i][k] * g[j][k];
+                    for (int h = 0; h < G; h++) {
+                        T v[4];
+                        load4(own + 64 * h + q * XP, v);
+                        store4(own + 64 * h + q * XP, v[0] - acc[h][0][q], v[1] - acc[h][1][q], v[2] - acc[h][2][q],
+                               v[3] - acc[h][3][q]);
                     }
-                    store4(st + k * R + 4 * tx + 64 * h, acc[h][0][k], acc[h][1][k], acc[h][2][k], acc[h][3][k]);
+            }
+            __syncthreads();
+        }
+        if (tid < R) {
+            T *row = xs + tid + c0 * XP;
+            T x[CB];
+#pragma unroll
+            for (int c = 0; c < CB; c++) x[c] = row[c * XP];
+#pragma unroll
+            for (int l = 0; l < CB; l++) {
+                x[l] *= rdiag[c0 + l];
+#pragma unroll
+                for (int c = l / 4 * 4; c < CB; c += 4) {
+                    T t[4];
+                    load4(lt + c0 + c + (c0 + l) * PB, t);
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        if (c + q > l) x[c + q] -= x[l] * t[q];
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < CB; c++) row[c * XP] = x[c];
+        }
+        __syncthreads();
+        if (4 * ty / CB > c0 / CB) {
+#pragma unroll 4
+            for (int l = c0; l < c0 + CB; l++) {
+                T t[4];
+                load4(lt + 4 * ty + l * PB, t);
+#pragma unroll
+                for (int h = 0; h < G; h++) {
+                    T v[4];
+                    load4(xs + 4 * tx + 64 * h + l * XP, v);
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int q = 0; q < 4; q++) acc[h][i][q] += v[i] * t[q];
                 }
             }
         }
-        T t[4][4];  // own columns' rows of the tile [column][k]
-        if (ty > p) {
+    }
+    if (FACTO == FACTO_SYTRF) {
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
+        for (int q = 0; q < 4; q++) {
+            const T m = dinv[4 * ty + q];
+#pragma unroll
+            for (int h = 0; h < G; h++) {
                 T v[4];
-                load4(lt + 4 * ty + (4 * p + k) * PB, v);
-#pragma unroll
-                for (int j = 0; j < 4; j++) t[j][k] = v[j];
+                load4(own + 64 * h + q * XP, v);
+                store4(own + 64 * h + q * XP, v[0] * m, v[1] * m, v[2] * m, v[3] * m);
             }
         }
         __syncthreads();
-        if (ty <= p) continue;
-#pragma unroll
-        for (int h = 0; h < G; h++) {
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                T v[4];
-                load4(st + k * R + 4 * tx + 64 * h, v);
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-#pragma unroll
-                    for (int j = 0; j < 4; j++) acc[h][i][j] -= v[i] * t[j][k];
-            }
-        }
     }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const T m = (FACTO == FACTO_SYTRF) ? dinv[4 * ty + q] : (T)1;
-#pragma unroll
-        for (int h = 0; h < G; h++) {
-            if (FACTO == FACTO_SYTRF) {
-#pragma unroll
-                for (int i = 0; i < 4; i++) acc[h][i][q] *= m;
-            }
-            store4(xs + 4 * tx + 64 * h + (4 * ty + q) * XP, acc[h][0][q], acc[h][1][q], acc[h][2][q], acc[h][3][q]);
-        }
-    }
-    __syncthreads();
 }
 
 template <typename T>
@@ -387,7 +398,7 @@ __device__ __forceinline__ void store_vec(T *p, const T *v) {
     else *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
 }
 
-// acc = X B over the first nl (a multiple of 8) of 64 K values: X[r, l] = xs[l * R + r],
+// acc = X B over 64 K values: X[r, l] = xs[l * R + r],
 // B[l, c] = bs[l * 64 + c].  Thread (tx, ty): columns 4 ty .. 4 ty + 3, rows in groups of
 // 16 bytes, group h at rows EPV (tx + 16 h) .. (a warp's reads of a group are 256
 // contiguous bytes; 8 contiguous rows per thread met every bank twice).  The operands of
@@ -398,7 +409,7 @@ template <typename T, int R>
 struct RowTile {
     static constexpr int MR = R / 16, EPV = 16 / (int)sizeof(T), G = MR / EPV;
     static __device__ __forceinline__ int row(int i) { return EPV * ((threadIdx.x & 15) + 16 * (i / EPV)) + i % EPV; }
-    static __device__ __forceinline__ void mul(T (&acc)[MR][4], const T *xs, const T *bs, int nl) {
+    static __device__ __forceinline__ void mul(T (&acc)[MR][4], const T *xs, const T *bs) {
         const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
         const T *xp = xs + EPV * tx, *bp = bs + 4 * ty;
 #pragma unroll
@@ -413,10 +424,10 @@ struct RowTile {
         };
         fetch(0, 0);
 #pragma unroll 1
-        for (int l0 = 0; l0 < nl; l0 += 8) {
+        for (int l0 = 0; l0 < PB; l0 += 8) {
 #pragma unroll
             for (int u = 0; u < 8; u++) {
-                if (u < 7 || l0 + 8 < nl) fetch(l0 + u + 1, (u + 1) & 1);
+                if (u < 7 || l0 + 8 < PB) fetch(l0 + u + 1, (u + 1) & 1);
 #pragma unroll
                 for (int i = 0; i < MR; i++)
 #pragma unroll
@@ -425,27 +436,6 @@ struct RowTile {
         }
     }
 };
-
-// The same solve as the product with the tile's inverse, bs[l * 64 + c] = W[c, l] (POTRF
-// row blocks): no dependent chain, 64 x 64 / 2 multiply-adds per row.
-template <typename T, int R>
-__device__ void trsm_inverse(T *xs, const T *bs) {
-    using RT = RowTile<T, R>;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    T acc[RT::MR][4];
-    RT::mul(acc, xs, bs, 8 * (ty / 2 + 1));  // W[c, l] = 0 for l > c
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-#pragma unroll
-        for (int h = 0; h < RT::G; h++) {
-            T v[RT::EPV];
-#pragma unroll
-            for (int i = 0; i < RT::EPV; i++) v[i] = acc[RT::EPV * h + i][q];
-            store_vec(xs + RT::EPV * (tx + 16 * h) + (4 * ty + q) * R, v);
-        }
-    __syncthreads();
-}
 
 template <typename T, int FACTO>
 __global__ void __launch_bounds__(PT, sizeof(T) == 4 ? 2 : 1) panel_kernel(DevSym s, const PanelCblk *__restrict__ pcb,
@@ -492,9 +482,9 @@ __global__ void __launch_bounds__(PT, sizeof(T) == 4 ? 2 : 1) panel_kernel(DevSy
         if (b == j) {
             // ---------------------------------------------- diagonal tile
             T *A = P + c0 + (size_t)c0 * ld;
-            T acc[4][4], wdiag[4][4];
+            T acc[4][4];
             load_tile_regs<T, FACTO>(acc, wd, [&](int r, int c) { return __ldcg(A + r + (size_t)c * ld); });
-            factor_tile_regs<T, FACTO>(acc, wdiag, wd, lt, thr, &s_piv, &s_err);
+            factor_tile_regs<T, FACTO>(acc, wd, lt, thr, &s_piv, &s_err);
 #pragma unroll
             for (int q = 0; q < 4; q++)
 #pragma unroll
@@ -630,8 +620,11 @@ __global__ void __launch_bounds__(PT, sizeof(T) == 4 ? 2 : 1) panel_kernel(DevSy
 // steps for the rows below the diagonal block) -- and, for b < ns, finally
 // factors its diagonal tile (b, b).  Each solved step of the diagonal block's
 // rows is written back and announced at once (solved[b] = j + 1; b + 1 after the
-// factorization), the only cross-item reads being the factored tiles L[j, j] (POTRF:
-// their inverses) and the diagonal block's solved tiles L[c, j].  Row blocks: 64 rows in
+// factorization), the only cross-item reads being the factored tiles L[j, j] and the
+// diagonal block's solved tiles L[c, j].  Cholesky solves by substitution like the others:
+// products with the tiles' inverses (no chain; 80^3 27-point split BF16 27.2 ms, 28.2 with
+// it) lose digits with the tile's condition number: dense matrices of condition 1e13, 60 + 40
+// columns, had a backward error of 6.9e-16, now 1.7e-16.  Row blocks: 64 rows in
 // the diagonal block, R rows (64 or 128) below it.  Items: the diagonal blocks' row
 // blocks of every cblk first (b ascending), then the rows below.
 //
@@ -667,8 +660,8 @@ __device__ __forceinline__ bool rows_need(const RowsCtx &x, int side, int c, int
 }
 
 template <typename T, int FACTO, int R>
-__device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, int side, T *L, T *U, T *Wk, T *lt, T *rdiag,
-                          T *dinv, T *dd, T *xs, const RowsCtx &x) {
+__device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, int side, T *L, T *U, T *lt, T *rdiag, T *dinv,
+                          T *dd, T *xs, const RowsCtx &x) {
     constexpr bool LU = FACTO == FACTO_GETRF;
     const int tid = threadIdx.x;
     const int k = pc.k, W = s.ncols[k], S = s.stride[k], ld = s.ld[k];
@@ -715,17 +708,14 @@ __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, int side,
     __syncthreads();
     const int tx = tid & 15, ty = tid >> 4;
     T pf[PB * PB / PT];  // tile read ahead: the next update operand, or the next step's diagonal tile
+    // the tile the rows are solved against: lower triangle and diagonal, identity past W
     auto load_diag = [&](int j) {
         const int c0 = PB * j, wd = min(PB, W - c0);
-        // POTRF: the inverse's column l; else the tile the rows are solved against, unit
-        // where it is not scaled by rdiag
-        const T *Dg = FACTO == FACTO_POTRF ? Wk + c0 + (size_t)c0 * W : Q + c0 + (size_t)c0 * ld;
-        const int dl = FACTO == FACTO_POTRF ? W : ld;
+        const T *Dg = Q + c0 + (size_t)c0 * ld;
 #pragma unroll
         for (int u = 0; u < PB * PB / PT; u++) {
             const int idx = tid + PT * u, c = idx & 63, l = idx >> 6;
-            if (FACTO == FACTO_POTRF) pf[u] = (c < wd && l <= c) ? __ldcg(Dg + c + (size_t)l * dl) : (T)0;
-            else pf[u] = (c < wd && l < c) ? __ldcg(Dg + c + (size_t)l * dl) : (c == l ? (T)1 : (T)0);
+            pf[u] = (c < wd && l <= c) ? __ldcg(Dg + c + (size_t)l * ld) : (c == l ? (T)1 : (T)0);
         }
     };
     auto load_b = [&](int j, int c) {
@@ -747,16 +737,19 @@ __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, int side,
         have = false;
         // ---------------------------------------------- solve of step j's columns
 #pragma unroll
-        for (int u = 0; u < PB * PB / PT; u++) lt[tid + PT * u] = pf[u];
-        if (FACTO != FACTO_POTRF && tid < PB) {
-            const T dgv = tid < wd ? __ldcg(Q + (c0 + tid) + (size_t)(c0 + tid) * ld) : (T)1;
-            rdiag[tid] = (LU && side == 0) ? (T)1 / dgv : (T)1;
-            dinv[tid] = (FACTO == FACTO_SYTRF) ? (T)1 / dgv : (T)1;
-            dd[tid] = (FACTO == FACTO_SYTRF) ? dgv : (T)1;
+        for (int u = 0; u < PB * PB / PT; u++) {
+            const int idx = tid + PT * u, c = idx & 63;
+            lt[idx] = pf[u];
+            if (c == idx >> 6) {  // the diagonal, which the products do not read
+                rdiag[c] = FACTO == FACTO_POTRF || (LU && side == 0) ? (T)1 / pf[u] : (T)1;
+                if (FACTO == FACTO_SYTRF) {
+                    dinv[c] = (T)1 / pf[u];
+                    dd[c] = pf[u];
+                }
+            }
         }
         __syncthreads();
-        if (FACTO == FACTO_POTRF) trsm_inverse<T, R>(xs + c0 * R, lt);
-        else trsm_tile<T, FACTO, R, R>(xs + c0 * R, lt, rdiag, dinv);
+        trsm_tile<T, FACTO, R, R>(xs + c0 * R, lt, rdiag, dinv);
 #pragma unroll 8
         for (int u = 0; u < R * PB / PT; u++) {
             const int r = (tid + PT * u) % R, c = (tid + PT * u) / R;
@@ -803,7 +796,7 @@ __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, int side,
             }
             using RT = RowTile<T, R>;
             T acc[RT::MR][4];
-            RT::mul(acc, xs + c0 * R, bs, PB);  // a step with columns right of it is a full one
+            RT::mul(acc, xs + c0 * R, bs);  // a step with columns right of it is a full one
             T *xc = xs + (PB * c) * R;
             if (own) {
 #pragma unroll
@@ -834,49 +827,27 @@ __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, int side,
         // ---------------------------------------------- the row block's diagonal tile
         const int c0 = PB * b, wd = min(PB, W - c0);
         T *xt = xs + c0 * R;
-        T acc[4][4], wdiag[4][4];
+        T acc[4][4];
         load_tile_regs<T, FACTO>(acc, wd, [&](int r, int c) { return xt[r + c * R]; });
         __syncthreads();
-        factor_tile_regs<T, FACTO>(acc, wdiag, wd, xt, x.thr, x.s_piv, x.s_err);
+        factor_tile_regs<T, FACTO>(acc, wd, xt, x.thr, x.s_piv, x.s_err);
         __syncthreads();
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            if (LU || tx >= ty) {
-                store4(xt + 4 * tx + (4 * ty + q) * R, acc[0][q], acc[1][q], acc[2][q], acc[3][q]);
-            } else if (FACTO == FACTO_POTRF) {
-                // W[ty, tx] = acc^T: column 4 tx + q of W, rows 4 ty ..
-                store4(lt + 4 * ty + (4 * tx + q) * PB, acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
-            }
-            if (FACTO == FACTO_POTRF && tx == ty)
-                store4(lt + 4 * tx + (4 * tx + q) * PB, wdiag[q][0], wdiag[q][1], wdiag[q][2], wdiag[q][3]);
-        }
+        for (int q = 0; q < 4; q++)
+            if (LU || tx >= ty) store4(xt + 4 * tx + (4 * ty + q) * R, acc[0][q], acc[1][q], acc[2][q], acc[3][q]);
         __syncthreads();
-        if (FACTO == FACTO_POTRF && b + 1 < pc.ns + (S > W ? 1 : 0)) {
-            for (int idx = tid; idx < PB * PB; idx += PT) {
-                const int c = idx & 63, l = idx >> 6;
-                if (c < wd && l <= c) Wk[(c0 + c) + (size_t)(c0 + l) * W] = lt[idx];
-            }
-        } else {
-            for (int idx = tid; idx < PB * PB; idx += PT) {
-                const int i = idx & 63, jj = idx >> 6;
-                if (i < wd && jj < wd && (LU || i >= jj)) P[c0 + i + (size_t)(c0 + jj) * ld] = xt[i + jj * R];
-            }
-            if (LU)
-                for (int t = tid >> 5; t < (PB / 8) * ((wd + 3) / 4); t += PT / 32) {
-                    const int i = 8 * (t % (PB / 8)) + (tid & 7), jj = 4 * (t / (PB / 8)) + ((tid & 31) >> 3);
-                    if (i < wd && jj < wd) Q[c0 + jj + (size_t)(c0 + i) * ld] = xt[i + jj * R];
-                }
+        for (int idx = tid; idx < PB * PB; idx += PT) {
+            const int i = idx & 63, jj = idx >> 6;
+            if (i < wd && jj < wd && (LU || i >= jj)) P[c0 + i + (size_t)(c0 + jj) * ld] = xt[i + jj * R];
         }
+        if (LU)
+            for (int t = tid >> 5; t < (PB / 8) * ((wd + 3) / 4); t += PT / 32) {
+                const int i = 8 * (t % (PB / 8)) + (tid & 7), jj = 4 * (t / (PB / 8)) + ((tid & 31) >> 3);
+                if (i < wd && jj < wd) Q[c0 + jj + (size_t)(c0 + i) * ld] = xt[i + jj * R];
+            }
         __syncthreads();
         if (tid == 0) {
             st_release(sol + b, b + 1);
-        }
-        if (FACTO == FACTO_POTRF && b + 1 < pc.ns + (S > W ? 1 : 0)) {
-            // the factored tile itself is read by later launches only
-            for (int idx = tid; idx < PB * PB; idx += PT) {
-                const int i = idx & 63, jj = idx >> 6;
-                if (i < wd && jj < wd && i >= jj) P[c0 + i + (size_t)(c0 + jj) * ld] = xt[i + jj * R];
-            }
         }
     }
 }
@@ -884,11 +855,10 @@ __device__ void rows_item(const DevSym &s, const PanelCblk &pc, int b, int side,
 template <typename T, int FACTO, int RB>
 __global__ void __launch_bounds__(PT, 1)
     panel_rows_kernel(DevSym s, const PanelCblk *__restrict__ pcb, const PanelItem *__restrict__ items, int nitems,
-                      int *ticket, int *solved, int *solved_v, int *abort_word, T *L, T *U, T *WL,
-                      const int64_t *__restrict__ woff, const double *__restrict__ thr_ptr,
-                      unsigned long long *npiv, int *err) {
+                      int *ticket, int *solved, int *solved_v, int *abort_word, T *L, T *U,
+                      const double *__restrict__ thr_ptr, unsigned long long *npiv, int *err) {
     extern __shared__ __align__(16) unsigned char pn_smem[];
-    T *lt = reinterpret_cast<T *>(pn_smem);  // the solve's tile (or its inverse); the update's operand
+    T *lt = reinterpret_cast<T *>(pn_smem);  // the solve's tile; the update's operand
     T *rdiag = lt + PB * PB, *dinv = rdiag + PB, *dd = dinv + PB;
     T *xs = dd + PB;                         // the row block, column-major (pitch = its rows)
     __shared__ int s_item, s_ok, s_piv, s_err;
@@ -910,9 +880,8 @@ __global__ void __launch_bounds__(PT, 1)
         const PanelCblk pc = pcb[it.p];
         const RowsCtx x{solved + pc.flag0, solved_v + pc.flag0, abort_word, s_known, &s_ok, &s_piv, &s_err,
                         cblk_threshold(s, thr_ptr, pc.k)};
-        T *Wk = WL + woff[pc.k];
-        if (it.b < pc.ns) rows_item<T, FACTO, PB>(s, pc, it.b, it.j, L, U, Wk, lt, rdiag, dinv, dd, xs, x);
-        else rows_item<T, FACTO, RB>(s, pc, it.b, it.j, L, U, Wk, lt, rdiag, dinv, dd, xs, x);
+        if (it.b < pc.ns) rows_item<T, FACTO, PB>(s, pc, it.b, it.j, L, U, lt, rdiag, dinv, dd, xs, x);
+        else rows_item<T, FACTO, RB>(s, pc, it.b, it.j, L, U, lt, rdiag, dinv, dd, xs, x);
         __syncthreads();
         if (!s_ok) {
             aborted = true;
@@ -997,24 +966,24 @@ int panel_rows_block(int nsmax, size_t esz) {
 
 template <typename T, int FACTO, int RB>
 static void launch_rows(const DevSym &s, const PanelCblk *pcb, const PanelItem *items, int nitems, int nsmax,
-                        int *ticket, int *solved, int *solved_v, int *abort_word, T *L, T *U, T *WL,
-                        const int64_t *woff, const double *thr, unsigned long long *npiv, int *err, cudaStream_t st) {
+                        int *ticket, int *solved, int *solved_v, int *abort_word, T *L, T *U,
+                        const double *thr, unsigned long long *npiv, int *err, cudaStream_t st) {
     const size_t smem = rows_smem_elems(nsmax, RB) * sizeof(T);
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, panel_rows_kernel<T, FACTO, RB>, PT, smem);
     const int grid = std::min(nitems, std::max(occ, 1) * g_sms);
     panel_rows_kernel<T, FACTO, RB><<<grid, PT, smem, st>>>(s, pcb, items, nitems, ticket, solved, solved_v, abort_word,
-                                                           L, U, WL, woff, thr, npiv, err);
+                                                           L, U, thr, npiv, err);
 }
 
 template <typename T>
 void launch_panel_rows(int facto, const DevSym &s, const PanelCblk *pcb, const PanelItem *items, int nitems,
-                       int nsmax, int rb, int *ticket, int *solved, int *solved_v, int *abort_word, T *L, T *U, T *WL,
-                       const int64_t *woff, const double *thr, unsigned long long *npiv, int *err, cudaStream_t st) {
+                       int nsmax, int rb, int *ticket, int *solved, int *solved_v, int *abort_word, T *L, T *U,
+                       const double *thr, unsigned long long *npiv, int *err, cudaStream_t st) {
     if (nitems <= 0) return;
     auto run = [&](auto f, auto r) {
         launch_rows<T, decltype(f)::value, decltype(r)::value>(s, pcb, items, nitems, nsmax, ticket, solved, solved_v,
-                                                               abort_word, L, U, WL, woff, thr, npiv, err, st);
+                                                               abort_word, L, U, thr, npiv, err, st);
     };
     auto by_facto = [&](auto r) {
         if (facto == FACTO_POTRF) run(std::integral_constant<int, FACTO_POTRF>{}, r);
@@ -1031,10 +1000,10 @@ void launch_panel_rows(int facto, const DevSym &s, const PanelCblk *pcb, const P
 }
 
 template void launch_panel_rows<double>(int, const DevSym &, const PanelCblk *, const PanelItem *, int, int, int, int *,
-                                        int *, int *, int *, double *, double *, double *, const int64_t *,
+                                        int *, int *, int *, double *, double *,
                                         const double *, unsigned long long *, int *, cudaStream_t);
 template void launch_panel_rows<float>(int, const DevSym &, const PanelCblk *, const PanelItem *, int, int, int, int *,
-                                       int *, int *, int *, float *, float *, float *, const int64_t *,
+                                       int *, int *, int *, float *, float *,
                                        const double *, unsigned long long *, int *, cudaStream_t);
 
 template void launch_panel<double>(int, const DevSym &, const PanelCblk *, const PanelItem *, int, int *, int *, int *,

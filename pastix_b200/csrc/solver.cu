@@ -1198,8 +1198,7 @@ int enqueue_numfact(b200_solver_t *s, cudaStream_t st, Trace *tr = nullptr) {
             if (s->lvl_prows[l])
                 launch_panel_rows<T>(s->facto, s->ds, s->d_pcb, s->d_pitem + s->lvl_pi0[l],
                                      s->lvl_pi1[l] - s->lvl_pi0[l], s->lvl_pns[l], s->lvl_prows[l], tickets + l,
-                                     solved, updated, abort_word, L, U, (T *)s->dWL, s->d_woff, s->d_thr, s->d_npiv,
-                                     s->d_err, st);
+                                     solved, updated, abort_word, L, U, s->d_thr, s->d_npiv, s->d_err, st);
             else
                 launch_panel<T>(s->facto, s->ds, s->d_pcb, s->d_pitem + s->lvl_pi0[l], s->lvl_pi1[l] - s->lvl_pi0[l],
                                 tickets + l, solved, updated, abort_word, L, s->d_thr, s->d_npiv, s->d_err, st);

@@ -1,6 +1,6 @@
 """Panels of wide cblks on the GPU against the oracle, on an analysis that needs no PaStiX
 library (the geometric nested dissection of perf/cases.py): the row-block launch of LU
-(both sides of the factor), Cholesky (tile inverses) and LDL^T, with diagonal blocks of
+(both sides of the factor), Cholesky and LDL^T, with diagonal blocks of
 one to five 64-column steps, full and ragged last steps."""
 import numpy as np
 import pytest
