@@ -999,18 +999,24 @@ int build_schedule(b200_solver_t *s) {
     return ERR_SUCCESS;
 }
 
-int ensure_ws(Lane *ln, size_t doubles) {
-    if (doubles <= ln->ws_cap) return ERR_SUCCESS;
-    if (ln->d_ws) {
-        CU(cudaStreamSynchronize(ln->st));
-        cudaFree(ln->d_ws);
+// Makes p (cap elements) hold count: a smaller block is freed once st's work with it is done.
+// After a failed allocation p is null and cap 0, so that a later call with a smaller count
+// allocates instead of using the lost block.
+template <typename T, typename N>
+int ensure_scratch(T *&p, N &cap, N count, cudaStream_t st) {
+    if (count <= cap) return ERR_SUCCESS;
+    if (p) {
+        CU(cudaStreamSynchronize(st));
+        cudaFree(p);
     }
-    ln->d_ws = nullptr;
-    ln->ws_cap = 0;
-    RET(dalloc(&ln->d_ws, doubles));
-    ln->ws_cap = doubles;
+    p = nullptr;
+    cap = 0;
+    RET(dalloc(&p, (size_t)count));
+    cap = count;
     return ERR_SUCCESS;
 }
+
+int ensure_ws(Lane *ln, size_t doubles) { return ensure_scratch(ln->d_ws, ln->ws_cap, doubles, ln->st); }
 
 void free_lane(Lane *ln) {
     if (ln->d_ws) cudaFree(ln->d_ws);
@@ -1055,29 +1061,10 @@ int lane_for(b200_solver_t *s, cudaStream_t st, Lane **out) {
 // instance, grown only when a call needs more, so repeated calls allocate nothing
 // and never pay cudaFree's device synchronization.
 int ensure_stage(b200_solver_t *s, size_t doubles) {
-    if (doubles <= s->stage_cap) return ERR_SUCCESS;
-    if (s->d_stage) {
-        CU(cudaStreamSynchronize(s->st));
-        cudaFree(s->d_stage);
-    }
-    s->d_stage = nullptr;
-    s->stage_cap = 0;
-    RET(dalloc(&s->d_stage, doubles));
-    s->stage_cap = doubles;
-    return ERR_SUCCESS;
+    return ensure_scratch(s->d_stage, s->stage_cap, doubles, s->st);
 }
 
-int ensure_scal(Lane *ln, int64_t count) {
-    if (count <= ln->scal_cap) return ERR_SUCCESS;
-    if (ln->d_scal) {
-        CU(cudaStreamSynchronize(ln->st));
-        cudaFree(ln->d_scal);
-    }
-    ln->d_scal = nullptr;
-    RET(dalloc(&ln->d_scal, (size_t)count));
-    ln->scal_cap = count;
-    return ERR_SUCCESS;
-}
+int ensure_scal(Lane *ln, int64_t count) { return ensure_scratch(ln->d_scal, ln->scal_cap, count, ln->st); }
 
 // ---------------------------------------------------------------- numfact
 
