@@ -804,7 +804,8 @@ int build_schedule(b200_solver_t *s) {
                s->lvl_wleaf[wf] == s->lvl_wleaf[wf - 1])
             wf--;
         s->wflow_level = wf;
-        std::vector<FlowItem> fwd, bwd, lf, lb;
+        std::vector<FlowItem> fwd, bwd, up, lf, lb;  // up: the backward items, cblk by cblk
+        std::vector<size_t> up0;
         std::vector<int> flist, need_f(N, 0), need_b(N, 0), nprev_f(N, 0), nprev_b(N, 0), mark(N, -1);
         int stamp = 0;
         for (int l = wf; l < nlev; l++)
@@ -838,10 +839,14 @@ int build_schedule(b200_solver_t *s) {
                 }
                 nprev_b[k] = (int)(lf.size() - off0);
                 fwd.insert(fwd.end(), lf.begin(), lf.end());
-                // backward order: reversed by cblk below
-                bwd.insert(bwd.begin(), lb.begin(), lb.end());
-                bwd.insert(bwd.begin(), lf.begin() + off0, lf.end());
+                up0.push_back(up.size());
+                up.insert(up.end(), lf.begin() + off0, lf.end());
+                up.insert(up.end(), lb.begin(), lb.end());
             }
+        // backward: the last cblk first
+        up0.push_back(up.size());
+        bwd.reserve(up.size());
+        for (size_t i = up0.size() - 1; i > 0; i--) bwd.insert(bwd.end(), up.begin() + up0[i - 1], up.begin() + up0[i]);
         s->wflow.nf = (int)fwd.size();
         s->wflow.nb = (int)bwd.size();
         if (flist.empty()) flist.push_back(0);

@@ -72,3 +72,23 @@ fake.fake_nulls()
 s.refine(b, b, "cg")
 assert fake.fake_nulls() == 0
 """)
+
+
+def test_creation_is_linear_in_a_chain(run):
+    # the schedule of four times the cblks is four times the work (a list built by insertions
+    # at its front took sixteen times)
+    run("""
+import time
+
+def create(ncblk):
+    st = chain_structure([12] * ncblk, "potrf")
+    t = time.perf_counter()
+    s = native.Solver(st, "potrf", "fp64")
+    t = time.perf_counter() - t
+    s.close()
+    return t
+
+create(100)
+short, long = (min(create(n) for _ in range(3)) for n in (10000, 40000))
+assert long <= 8 * short + 0.02, (short, long)
+""")
