@@ -66,22 +66,20 @@ enum : int {
     UPD_SCALE_D = 32  // multiply A by D (LDL^T: C -= (L_i D) L_j^T)
 };
 
+// One record per update (a million in a 512-system forest), read whole by its warps.
 struct Upd {
-    int k, j, f;
-    int colK0;    // first column of k in the K-range (0 except for sub-panel self-updates)
+    int k, f;
     int rowA0;    // panel row of k where the M-range starts
     int rowB0;    // panel row of k of block j
     int M, N, K;
     int colbase;  // column in f of block j's first row
-    int tiles_m, tiles_n;
     int flags;
     int nb;       // tensor-core updates: columns per tile (a multiple of 32, at most the launch's tile width)
     int rm0;      // first entry of its row map (M entries: row rowA0 + i of k -> row of f, or -1)
-    // where the operands lie, so that a kernel reads this record only: element offsets in
-    // their arenas (flags) of row rowA0 and of row rowB0 in column colK0, of column
-    // colbase of f, and of D's entry colK0; leading dimensions of k and f
+    // where the operands lie, so that a kernel reads this record only: leading dimensions of
+    // k and f, element offsets in their arenas (flags) of k's panel and of column colbase of f
     int ldk, ldf;
-    int64_t offA, offB, offC, offD;
+    int64_t offK, offC;
 };
 
 // Item of the tree-bottom launch, in ticket order: fact = 1 factors cblk k (diagonal

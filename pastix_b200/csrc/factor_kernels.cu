@@ -452,9 +452,9 @@ __global__ void __launch_bounds__(128, UPD_CTAS)
         lld = u.ldk;
         lokA = r < u.M - m0;
         lokB = r < u.N - n0;
-        lA = ((u.flags & UPD_A_U) ? U : L) + u.offA + (lokA ? m0 + r : 0) + (size_t)c * lld;
-        lB = ((u.flags & UPD_B_U) ? U : L) + u.offB + (lokB ? n0 + r : 0) + (size_t)c * lld;
-        lD = (u.flags & UPD_SCALE_D) ? L + u.offD + (size_t)(tid & (UT_K - 1)) * (lld + 1) : nullptr;
+        lA = ((u.flags & UPD_A_U) ? U : L) + u.offK + u.rowA0 + (lokA ? m0 + r : 0) + (size_t)c * lld;
+        lB = ((u.flags & UPD_B_U) ? U : L) + u.offK + u.rowB0 + (lokB ? n0 + r : 0) + (size_t)c * lld;
+        lD = (u.flags & UPD_SCALE_D) ? L + u.offK + (size_t)(tid & (UT_K - 1)) * (lld + 1) : nullptr;
         lk = 0;
     };
     auto load_stage = [&](int st) {
@@ -819,8 +819,8 @@ __global__ void __launch_bounds__(32 * US_WARPS, KB == 8 ? 5 : sizeof(T) == 4 ? 
     if (ui >= nupd) return;
     const Upd u = upds[ui];
     const int ldk = u.ldk, ldf = u.ldf;
-    const T *Ap = ((u.flags & UPD_A_U) ? U : L) + u.offA;
-    const T *Bp = ((u.flags & UPD_B_U) ? U : L) + u.offB;
+    const T *Ap = ((u.flags & UPD_A_U) ? U : L) + u.offK + u.rowA0;
+    const T *Bp = ((u.flags & UPD_B_U) ? U : L) + u.offK + u.rowB0;
     const bool scale = (u.flags & UPD_SCALE_D) != 0;
     const bool atomic = (u.flags & UPD_ATOMIC) != 0;
     const bool sym = (u.flags & UPD_SYM) != 0;
@@ -831,7 +831,7 @@ __global__ void __launch_bounds__(32 * US_WARPS, KB == 8 ? 5 : sizeof(T) == 4 ? 
     T(*bs)[KB] = bsm[threadIdx.x >> 5];
 #pragma unroll
     for (int q = 0; q < KB; q++) bs[lane][q] = (lane < u.N && q < u.K) ? Bp[lane + (size_t)q * ldk] : (T)0;
-    T dk = (scale && lane < u.K) ? L[u.offD + (size_t)lane * (ldk + 1)] : (T)1;
+    T dk = (scale && lane < u.K) ? L[u.offK + (size_t)lane * (ldk + 1)] : (T)1;
     __syncwarp();
     for (int r0 = 0; r0 < u.M; r0 += 32) {
         const int i = r0 + lane;
@@ -921,13 +921,13 @@ __device__ bool dag_wait(const int *cnt, int target, const int *abort_word) {
 // chunks of 32 rows staged in bs (32 x TP).
 template <typename T, int KB>
 __device__ void warp_update(const DevSym &s, const Upd &u, T *L, T *U, T *bs, int lane, int rb, int re) {
-    const int k = u.k, ldk = s.ld[k];
-    const T *Ap = ((u.flags & UPD_A_U) ? U : L) + s.off[k] + u.rowA0 + (size_t)u.colK0 * ldk;
-    const T *Bp = ((u.flags & UPD_B_U) ? U : L) + s.off[k] + u.rowB0 + (size_t)u.colK0 * ldk;
-    const T *Dp = L + s.off[k] + (size_t)u.colK0 * (ldk + 1);
+    const int ldk = u.ldk;
+    const T *Ap = ((u.flags & UPD_A_U) ? U : L) + u.offK + u.rowA0;
+    const T *Bp = ((u.flags & UPD_B_U) ? U : L) + u.offK + u.rowB0;
+    const T *Dp = L + u.offK;
     const bool scale = (u.flags & UPD_SCALE_D) != 0, sym = (u.flags & UPD_SYM) != 0;
-    T *C = ((u.flags & UPD_C_U) ? U : L) + s.off[u.f];
-    const int ldf = s.ld[u.f];
+    T *C = ((u.flags & UPD_C_U) ? U : L) + u.offC;
+    const int ldf = u.ldf;
     const T dk = (scale && lane < u.K) ? Dp[(size_t)lane * (ldk + 1)] : (T)1;
     for (int n0 = 0; n0 < u.N; n0 += 32) {
         const int nw = min(32, u.N - n0);
@@ -949,7 +949,7 @@ __device__ void warp_update(const DevSym &s, const Upd &u, T *L, T *U, T *bs, in
             }
             const int d = in ? __ldg(s.rmap + u.rm0 + i) : -1;
             if (d < 0) continue;
-            T *crow = C + d + (size_t)(u.colbase + n0) * ldf;
+            T *crow = C + d + (size_t)n0 * ldf;
             for (int c = 0; c < nw; c++) {
                 T acc = 0;
 #pragma unroll

@@ -310,29 +310,42 @@ int build_schedule(b200_solver_t *s) {
     // walk, kernels/core_zgemmsp.c:420-440), so that
     // the update kernels read one entry instead of searching the block tables
     std::vector<int> rmap;
+    int64_t n_updates = 0;
+    {
+        // of every update that make_upd may give: their number and their rows
+        int64_t nupd = 0, nrow = 0;
+        for (int k = 0; k < cs; k++)
+            for (int j = s->fblok[k] + 1; j < s->fblok[k + 1]; j++) {
+                nupd++;
+                nrow += s->stride[k] - s->rowoff[j];
+            }
+        const int sides = s->facto == FACTO_GETRF ? 2 : 1;
+        n_updates = nupd * sides;
+        if (nrow * sides <= INT32_MAX) rmap.reserve(nrow * sides);
+    }
+    // row by row this took most of an instance's creation; a run is where a block of k lies
+    // inside one block of f
     auto map_rows = [&](Upd &u) -> bool {
         if (rmap.size() + (size_t)u.M > (size_t)INT32_MAX) return false;
         u.rm0 = (int)rmap.size();
-        rmap.resize(rmap.size() + u.M, -1);
-        int bf = s->fblok[u.f];
-        const int bfe = s->fblok[u.f + 1];
-        for (int b = s->fblok[u.k] + 1; b < s->fblok[u.k + 1]; b++) {
-            const int r0 = s->rowoff[b], nbr = s->lrow[b] - s->frow[b] + 1;
-            if (r0 + nbr <= u.rowA0) continue;
-            for (int t = 0; t < nbr; t++) {
-                const int prow = r0 + t, grow = s->frow[b] + t;
-                if (prow < u.rowA0) continue;
-                while (bf < bfe && s->lrow[bf] < grow) bf++;
-                int d = -1;
-                if (bf < bfe && grow >= s->frow[bf] && grow <= s->lrow[bf]) d = s->rowoff[bf] + (grow - s->frow[bf]);
-                rmap[(size_t)u.rm0 + (prow - u.rowA0)] = d;
+        rmap.resize(rmap.size() + u.M);
+        int *out = rmap.data() + u.rm0;
+        const int *lrow = s->lrow.data(), bfe = s->fblok[u.f + 1];
+        int bf = s->fblok[u.f], b = s->fblok[u.k] + 1;
+        while (s->rowoff[b] < u.rowA0) b++;
+        for (; b < s->fblok[u.k + 1]; b++)
+            for (int g = s->frow[b], last = lrow[b]; g <= last;) {
+                if (bf < bfe && lrow[bf] < g) bf = (int)(std::lower_bound(lrow + bf + 1, lrow + bfe, g) - lrow);
+                const bool in = bf < bfe && s->frow[bf] <= g;
+                const int end = in ? std::min(last, lrow[bf]) : bf < bfe ? std::min(last, s->frow[bf] - 1) : last;
+                for (int d = in ? s->rowoff[bf] + g - s->frow[bf] : -1; g <= end; g++, d += in) *out++ = d;
             }
-        }
         return true;
     };
     std::vector<int2> updmap;         // tiles of the 64 x 64 update launches: {update of the level, row | col << 16}
     std::vector<int2> tcmap, tcmapw;  // tile maps of the 64- and 128-column tensor-core launches
     std::vector<Upd> smallupds;
+    smallupds.reserve(n_updates);
     s->lvl_us0.assign(nlev, 0);
     s->lvl_us8.assign(nlev, 0);
     s->lvl_us1.assign(nlev, 0);
@@ -351,7 +364,7 @@ int build_schedule(b200_solver_t *s) {
     // kernel of an FP32 update by the tuning table: 0 CUDA cores, 64 or 128 the
     // tensor cores with tiles of that many columns
     auto tc_choice = [&](const Upd &u) -> int {
-        if (!s->use_tc || (u.flags & UPD_SCALE_D) || !(u.colK0 == 0 || u.K % 32 == 0)) return 0;
+        if (!s->use_tc || (u.flags & UPD_SCALE_D)) return 0;
         const int w = u.K < 16 ? 0 : u.K < 32 ? 1 : u.K < 48 ? 2 : u.K < 64 ? 3 : u.K < 128 ? 4 : 5;
         const int h = u.M < 64 ? 0 : u.M < 128 ? 1 : u.M < 256 ? 2 : u.M < 512 ? 3 : 4;
         const int wide = u.N > 64 ? 128 : 64;
@@ -379,11 +392,10 @@ int build_schedule(b200_solver_t *s) {
     auto push_tc = [&](Upd u, int bn, int &t0, int &t0w, int base) {
         s->flops_kind[6] += upd_flops(u);
         u.nb = bn;
-        u.tiles_m = (u.M + 127) / 128;
-        u.tiles_n = (u.N + u.nb - 1) / u.nb;
+        const int tiles_m = (u.M + 127) / 128, tiles_n = (u.N + u.nb - 1) / u.nb;
         const int ui = (int)tcupds.size() - base;
-        for (int nt = 0; nt < u.tiles_n; nt++)
-            for (int mt = 0; mt < u.tiles_m; mt++) {
+        for (int nt = 0; nt < tiles_n; nt++)
+            for (int mt = 0; mt < tiles_m; mt++) {
                 if ((u.flags & UPD_SYM) && mt * 128 + 127 < nt * u.nb) continue;  // above the diagonal
                 (bn == 128 ? tcmapw : tcmap).push_back(make_int2(ui, mt | (nt << 16)));
                 (bn == 128 ? t0w : t0)++;
@@ -433,7 +445,6 @@ int build_schedule(b200_solver_t *s) {
     auto make_upd = [&](int k, int j, int side, int atomic, Upd &u) -> bool {
         u = Upd{};
         u.k = k;
-        u.j = j;
         u.f = s->fcblk[j];
         u.rowB0 = s->rowoff[j];
         if (side == 0) {
@@ -453,10 +464,8 @@ int build_schedule(b200_solver_t *s) {
         u.colbase = s->frow[j] - s->fcol[u.f];
         u.ldk = s->ld[k];
         u.ldf = s->ld[u.f];
-        u.offA = s->off[k] + u.rowA0;
-        u.offB = s->off[k] + u.rowB0;
+        u.offK = s->off[k];
         u.offC = s->off[u.f] + (int64_t)u.colbase * u.ldf;
-        u.offD = s->off[k];
         return true;
     };
     const size_t trsm_smem = (size_t)s->trsm_smem;
@@ -617,11 +626,9 @@ int build_schedule(b200_solver_t *s) {
                         (u.K <= 8 ? smallupds : small16).push_back(u);
                         continue;
                     }
-                    u.tiles_m = (u.M + 63) / 64;
-                    u.tiles_n = (u.N + 63) / 64;
-                    const int ui = (int)upds.size() - L.u0;
-                    for (int nt = 0; nt < u.tiles_n; nt++)
-                        for (int mt = (u.flags & UPD_SYM) ? nt : 0; mt < u.tiles_m; mt++) {
+                    const int ui = (int)upds.size() - L.u0, tiles_m = (u.M + 63) / 64, tiles_n = (u.N + 63) / 64;
+                    for (int nt = 0; nt < tiles_n; nt++)
+                        for (int mt = (u.flags & UPD_SYM) ? nt : 0; mt < tiles_m; mt++) {
                             updmap.push_back(make_int2(ui, mt | (nt << 16)));
                             tile0++;
                         }

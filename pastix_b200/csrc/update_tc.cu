@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) update_tc_kernel(DevSym s, cons
                     mbar_expect_tx(bar, tx);
                     last_ph[st] = (it / NST) & 1;
                     const uint32_t base = smem_addr(smem + (size_t)st * Cfg::STAGE);
-                    const int x = kc * BK + u.colK0;
+                    const int x = kc * BK;
 #pragma unroll
                     for (int g = 0; g < TC_BM / 64; g++) tma_load_2d(base + g * 8192, ma, x, ya + 64 * g, bar);
                     for (int g = 0; g < nb / 64; g++) tma_load_2d(base + TC_A_BYTES + g * 8192, mb, x, yb + 64 * g, bar);

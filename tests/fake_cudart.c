@@ -4,13 +4,16 @@
 #include <stdlib.h>
 #include <string.h>
 
-typedef struct { size_t limit, largest; long nulls; } fake_t;
-fake_t fake = {(size_t)-1, 0, 0};
+typedef struct { size_t limit, largest, watch; long nulls; void *watched; } fake_t;
+fake_t fake = {(size_t)-1, 0, 0, 0, NULL};
 /* allocations of more bytes than limit fail */
 void fake_limit(size_t limit) { fake.limit = limit; }
 /* largest allocation asked for, and copies from or to a null pointer, since the last call */
 size_t fake_largest(void) { size_t v = fake.largest; fake.largest = 0; return v; }
 long fake_nulls(void) { long v = fake.nulls; fake.nulls = 0; return v; }
+/* keep what the next copies of exactly so many bytes are given, and return the last one */
+void fake_watch(size_t bytes) { fake.watch = bytes; free(fake.watched); fake.watched = NULL; }
+void *fake_watched(void) { return fake.watched; }
 
 #define OK(name) int name(void) { return 0; }
 OK(__cudaPopCallConfiguration) OK(__cudaPushCallConfiguration) OK(__cudaRegisterFatBinaryEnd)
@@ -44,12 +47,19 @@ int cudaMalloc(void **p, size_t n) {
     *p = malloc(16);
     return 0;
 }
-static int copy(const void *d, const void *s) { if (!d || !s) fake.nulls++; return 0; }
-int cudaMemcpy(void *d, const void *s, size_t n, int k) { (void)n; (void)k; return copy(d, s); }
-int cudaMemcpyAsync(void *d, const void *s, size_t n, int k, void *st) { (void)n; (void)k; (void)st; return copy(d, s); }
+static int copy(const void *d, const void *s, size_t n, int kind) {
+    if (!d || !s) fake.nulls++;
+    if (n == fake.watch && n && kind == 1) { /* from the host */
+        free(fake.watched);
+        fake.watched = memcpy(malloc(n), s, n);
+    }
+    return 0;
+}
+int cudaMemcpy(void *d, const void *s, size_t n, int k) { return copy(d, s, n, k); }
+int cudaMemcpyAsync(void *d, const void *s, size_t n, int k, void *st) { (void)st; return copy(d, s, n, k); }
 int cudaMemcpy2DAsync(void *d, size_t dp, const void *s, size_t sp, size_t w, size_t h, int k, void *st) {
-    (void)dp; (void)sp; (void)w; (void)h; (void)k; (void)st;
-    return copy(d, s);
+    (void)dp; (void)sp; (void)w; (void)h; (void)st;
+    return copy(d, s, 0, k);
 }
 int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *f, int b, size_t s, unsigned fl) {
     (void)f; (void)b; (void)s; (void)fl;

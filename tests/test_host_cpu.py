@@ -92,3 +92,56 @@ create(100)
 short, long = (min(create(n) for _ in range(3)) for n in (10000, 40000))
 assert long <= 8 * short + 0.02, (short, long)
 """)
+
+
+def test_update_records_stay_small(tmp_path):
+    # a million of them are filled, uploaded and read for a 512-system forest
+    src = tmp_path / "size.cpp"
+    src.write_text('#include "b200_internal.h"\nstatic_assert(sizeof(b200::Upd) <= 72, "record");\nint main() {}\n')
+    subprocess.run(["g++", "-std=c++17", "-I", os.path.join(REPO, "pastix_b200", "csrc"), "-I",
+                    "/usr/local/cuda/include", "-fsyntax-only", str(src)], check=True)
+
+
+def test_row_maps(run):
+    # the destination rows of every update, which are uploaded, against a search row by row
+    run("""
+from block_structure import block_structure, dense_structure
+from perf import cases as C
+
+fake.fake_watch.argtypes = [ctypes.c_size_t]
+fake.fake_watch.restype = None
+fake.fake_watched.restype = ctypes.POINTER(ctypes.c_int)
+
+
+def expected(st, sides):
+    first, last, own, face = st.blok_frownum, st.blok_lrownum, st.cblk_fblok, st.blok_fcblknm
+    level = [0] * st.cblknbr
+    for k in range(st.cblknbr):
+        for f in face[own[k] + 1:own[k + 1]]:
+            level[f] = max(level[f], level[k] + 1)
+    out = []
+    for k in sorted(range(st.cblknbr), key=lambda k: (level[k], k)):
+        for j in range(own[k] + 1, own[k + 1]):
+            f = face[j]
+            row = {}
+            at = 0
+            for b in range(own[f], own[f + 1]):
+                for r in range(first[b], last[b] + 1):
+                    row[r] = at
+                    at += 1
+            for side in range(sides):
+                out += [row.get(r, -1) for b in range(j + side, own[k + 1]) for r in range(first[b], last[b] + 1)]
+    return out
+
+
+for facto, st in [("potrf", C._structure(7, 6, 5, 27, "potrf")), ("getrf", C._structure(9, 4, 6, 7, "getrf")),
+                  ("potrf", dense_structure([5, 40, 3], "potrf")),
+                  # cblk 1 lacks rows that cblk 0 updates it in: entries of -1
+                  ("getrf", block_structure([3, 4, 5, 2], [[1, 2, 3], [3], [3], []], "getrf"))]:
+    want = expected(st, 2 if facto == "getrf" else 1)
+    fake.fake_watch(4 * len(want))
+    s = native.Solver(st, facto, "fp64")
+    got = fake.fake_watched()
+    assert got and got[:len(want)] == want
+    s.close()
+""")
