@@ -157,8 +157,9 @@ int configure_solve_kernels();
 int configure_inverse_kernels();
 
 // refinement vectors (refine_kernels.cu)
-// xt (n x 16 doubles, may be null): row-major staging of 16 columns of x at a time
-void launch_spmv(int n, int64_t nnz, int nrhs, const int64_t *colptr, const int *rowtab, const double *vals, const double *x,
+// xt (n x 16 doubles, may be null): row-major staging of 16 columns of x at a time;
+// max_row: the entries of the longest row
+void launch_spmv(int n, int64_t nnz, int64_t max_row, int nrhs, const int64_t *colptr, const int *rowtab, const double *vals, const double *x,
                  int64_t ldx, double *y, int64_t ldy, double alpha, double beta, cudaStream_t st,
                  double *xt = nullptr);
 // dst[e] = src[map[e]], e < nnz

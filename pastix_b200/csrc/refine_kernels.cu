@@ -37,6 +37,30 @@ __global__ void __launch_bounds__(256) spmv_kernel(int n, int nrhs, const int64_
     }
 }
 
+// The same for a matrix with long rows, whose chains of loads bound it: a warp per row, in a
+// loop that the compiler unrolls (the one above is not; 200 000 rows of 2 entries and a dense
+// one: 8.3 ms with 4 lanes, 0.78 here; 27 entries a row: 143 us above, 175 here).
+__global__ void __launch_bounds__(256) spmv_long_kernel(int n, int nrhs, const int64_t *__restrict__ colptr,
+                                                        const int *__restrict__ rowtab,
+                                                        const double *__restrict__ vals, const double *__restrict__ x,
+                                                        int64_t ldx, double *y, int64_t ldy, double alpha,
+                                                        double beta) {
+    const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (row >= n) return;
+    const int64_t e0 = colptr[row], e1 = colptr[row + 1];
+    for (int r = 0; r < nrhs; r++) {
+        double acc = 0.0;
+        for (int64_t e = e0 + lane; e < e1; e += 32) acc += vals[e] * x[rowtab[e] + r * ldx];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) {
+            double *yp = y + row + r * ldy;
+            *yp = (beta == 0.0) ? alpha * acc : alpha * acc + beta * *yp;
+        }
+    }
+}
+
 // Column dot products, one CTA per (column, chunk), atomically accumulated.
 __global__ void dots_kernel(int n, const double *__restrict__ x, int64_t ldx, const double *__restrict__ y,
                             int64_t ldy, double *out) {
@@ -192,7 +216,7 @@ __global__ void __launch_bounds__(256) spmv_rows_kernel(int n, int R, const int6
     }
 }
 
-void launch_spmv(int n, int64_t nnz, int nrhs, const int64_t *colptr, const int *rowtab, const double *vals, const double *x,
+void launch_spmv(int n, int64_t nnz, int64_t max_row, int nrhs, const int64_t *colptr, const int *rowtab, const double *vals, const double *x,
                  int64_t ldx, double *y, int64_t ldy, double alpha, double beta, cudaStream_t st, double *xt) {
     if (n <= 0) return;
     if (nrhs > 1 && xt) {
@@ -209,11 +233,16 @@ void launch_spmv(int n, int64_t nnz, int nrhs, const int64_t *colptr, const int 
                                                                       alpha, beta);
         };
         // the smallest power of two that covers an average row: fewer lanes would take a row
-        // in several steps, more would idle
+        // in several steps, more would idle.  A warp when a row would take more than 16 steps
+        // of so few lanes
         const int64_t avg = (nnz + n - 1) / n;
-        if (avg <= 4) run(std::integral_constant<int, 4>{});
-        else if (avg <= 8) run(std::integral_constant<int, 8>{});
-        else if (avg <= 16) run(std::integral_constant<int, 16>{});
+        const int w = avg <= 4 ? 4 : avg <= 8 ? 8 : avg <= 16 ? 16 : 32;
+        if (max_row > 16 * w)
+            spmv_long_kernel<<<nblk((int64_t)n * 32, 256), 256, 0, st>>>(n, nrhs, colptr, rowtab, vals, x, ldx, y,
+                                                                        ldy, alpha, beta);
+        else if (w == 4) run(std::integral_constant<int, 4>{});
+        else if (w == 8) run(std::integral_constant<int, 8>{});
+        else if (w == 16) run(std::integral_constant<int, 16>{});
         else run(std::integral_constant<int, 32>{});
     }
 }

@@ -202,6 +202,7 @@ struct b200_solver_s {
 
     // bcsc
     int64_t nnz = -1;
+    int64_t max_row = 0;  // entries of the longest row of the bcsc
     int64_t *d_colptr = nullptr;
     int *d_rowtab = nullptr;
     double *d_Lv = nullptr, *d_Uv = nullptr;
@@ -1515,7 +1516,7 @@ struct RefineCtx {
     int spmv(const double *x, double *y, double alpha, double beta) {
         const double *vals = (s->facto == FACTO_GETRF) ? s->d_Uv : s->d_Lv;
         if (nrhs > 1 && !ln->d_xt) RET(dalloc(&ln->d_xt, (size_t)n * 16));
-        launch_spmv(n, s->nnz, nrhs, s->d_colptr, s->d_rowtab, vals, x, n, y, n, alpha, beta, st, ln->d_xt);
+        launch_spmv(n, s->nnz, s->max_row, nrhs, s->d_colptr, s->d_rowtab, vals, x, n, y, n, alpha, beta, st, ln->d_xt);
         s->kernel_launches += nrhs > 1 ? 2 * ((nrhs + 15) / 16) : 1;
         return ERR_SUCCESS;
     }
@@ -2392,6 +2393,8 @@ int b200_bcsc_load(b200_solver_t *s, int64_t nnz, const int64_t *colptr, const i
         if (s->fact_graph) cudaGraphExecDestroy(s->fact_graph);
         s->fact_graph = nullptr;
         s->h_colptr.assign(colptr, colptr + n + 1);
+        s->max_row = 0;
+        for (int i = 0; i < n; i++) s->max_row = std::max(s->max_row, colptr[i + 1] - colptr[i]);
         s->h_rowtab.assign(rowtab, rowtab + nnz);
         // destination of every bcsc entry in the panel arena (cpucblk_zfillin_fr,
         // kernels/cpucblk_zinit.c:229-309): rows above the diagonal are skipped,
@@ -2774,7 +2777,7 @@ int b200_spmv(b200_solver_t *s, int64_t nrhs, double alpha, const double *x, int
         const double *vals = (s->facto == FACTO_GETRF) ? s->d_Uv : s->d_Lv;
         if (nrhs > 1 && !s->main.d_xt && dalloc(&s->main.d_xt, (size_t)n * 16)) rc = ERR_OOM;
         if (!rc)
-            launch_spmv(n, s->nnz, (int)nrhs, s->d_colptr, s->d_rowtab, vals, px, n, py, n, alpha, beta, s->st, s->main.d_xt);
+            launch_spmv(n, s->nnz, s->max_row, (int)nrhs, s->d_colptr, s->d_rowtab, vals, px, n, py, n, alpha, beta, s->st, s->main.d_xt);
         launch_permute(n, (int)nrhs, s->d_peri, py, n, dy, n, 0, s->st);
         if (cudaMemcpy2DAsync(y, ldy * sizeof(double), dy, n * sizeof(double), n * sizeof(double), nrhs,
                               cudaMemcpyDeviceToHost, s->st) != cudaSuccess) rc = ERR_INTERNAL;
@@ -2799,7 +2802,7 @@ int b200_spmv_device(b200_solver_t *s, int64_t nrhs, double alpha, const double 
     const double *vals = (s->facto == FACTO_GETRF) ? s->d_Uv : s->d_Lv;
     launch_permute(n, (int)nrhs, s->d_peri, d_x, ldx, px, n, 1, st);
     launch_permute(n, (int)nrhs, s->d_peri, d_y, ldy, py, n, 1, st);
-    launch_spmv(n, s->nnz, (int)nrhs, s->d_colptr, s->d_rowtab, vals, px, n, py, n, alpha, beta, st, ln->d_xt);
+    launch_spmv(n, s->nnz, s->max_row, (int)nrhs, s->d_colptr, s->d_rowtab, vals, px, n, py, n, alpha, beta, st, ln->d_xt);
     launch_permute(n, (int)nrhs, s->d_peri, py, n, d_y, ldy, 0, st);
     CU(cudaGetLastError());
     s->kernel_launches += 3 + (nrhs > 1 ? 2 * ((nrhs + 15) / 16) : 1);

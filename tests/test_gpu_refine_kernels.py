@@ -2,7 +2,10 @@
 product with 4, 8, 16 and 32 lanes per row, and GMRES over restarts."""
 import numpy as np
 import pytest
+import scipy.sparse as sp
+import torch
 
+from block_structure import bcsc_of, block_structure
 from pastix_b200 import native
 from test_gpu_wide_panels import analysis
 
@@ -45,3 +48,55 @@ def test_gmres_restarts(facto, shift, im):
         r = np.linalg.norm(b[:, j] - s.spmv(x[:, j])) / np.linalg.norm(b[:, j])
         assert r <= 1.2e-12
     s.close()
+
+
+def arrowhead(n, dense, facto, full=False):
+    """n rows of a diagonal entry (full: of a dense 20 x 20 block) and the dense columns',
+    then dense rows of n + 1 entries."""
+    st = block_structure([20] * (n // 20) + [dense], [[n // 20]] * (n // 20) + [[]], facto)
+    r = np.random.default_rng(4)
+    B = sp.csr_matrix(r.uniform(-1, 1, (dense, n)))
+    C = B if facto != "getrf" else sp.csr_matrix(r.uniform(-1, 1, (dense, n)))
+    D = sp.kron(sp.identity(n // 20), np.full((20, 20), 0.5)) if full else sp.diags([r.uniform(1, 2, n)], [0])
+    A = sp.bmat([[D, C.T], [B, sp.diags([np.full(dense, 2.0 * n)], [0])]]).tocsr()
+    s = native.Solver(st, facto, "fp64")
+    s.bcsc_load(bcsc_of(A, facto))
+    return s, A
+
+
+# 2 to 17 entries in the short rows; n + 1 in the dense ones: below and above 16 steps of 4, 8
+# and 16 lanes
+@pytest.mark.parametrize("n", [20, 60, 100, 200, 1000])
+@pytest.mark.parametrize("dense", [1, 4, 7, 16])
+@pytest.mark.parametrize("facto", ["potrf", "getrf"])
+def test_spmv_of_an_arrowhead(facto, dense, n):
+    s, A = arrowhead(n, dense, facto)
+    x = np.random.default_rng(5).uniform(-1, 1, A.shape[0])
+    # entries + 2 roundings of at most 2^-53 times the row's sum, on both sides
+    tol = 2 * (np.diff(A.indptr) + 2) * 2.0 ** -53 * np.asarray(abs(A).sum(axis=1)).ravel()
+    y = s.spmv(x)
+    assert np.all(np.abs(y - A @ x) <= tol)
+    assert np.all(np.abs(s.spmv(x, 2.0, -3.0, y) + y) <= 6 * tol)
+    s.close()
+
+
+def test_dense_rows_take_whole_warps():
+    # a row of 200 000 entries, read by one chain of loads: no longer among rows of 2 entries
+    # than among rows of 21, which have a warp each
+    def product(full):
+        s, A = arrowhead(200000, 1, "potrf", full)
+        x = torch.ones(A.shape[0], dtype=torch.float64, device="cuda")
+        y = torch.zeros_like(x)
+        stream = torch.cuda.Stream()
+        times = []
+        for _ in range(10):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            with torch.cuda.stream(stream):
+                a.record()
+                s.spmv_device(x.data_ptr(), y.data_ptr(), 1, stream=stream.cuda_stream)
+                b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        s.close()
+        return min(times)
+    assert product(False) <= 1.25 * product(True)
