@@ -45,6 +45,7 @@ int dalloc(T **p, size_t count) {
     cudaError_t e = cudaMalloc((void **)p, count * sizeof(T));
     if (e != cudaSuccess) {
         fprintf(stderr, "pastix_b200: cudaMalloc(%zu bytes) failed: %s\n", count * sizeof(T), cudaGetErrorString(e));
+        cudaGetLastError();  // not the error of the next launch that is checked
         return ERR_OOM;
     }
     return ERR_SUCCESS;
@@ -1416,7 +1417,9 @@ int enqueue_wide_sweeps(b200_solver_t *s, Lane *ln, double *x, double *aux, int 
 // preconditioner of an FP64 refinement -- on two n x nrhs float blocks held in aux,
 // converted from and back to x.
 // Many right-hand sides take the row-major sweeps (pitch: columns that both blocks have room
-// for; FP64 rows need an even number).  From 8 on: below, their tiles of 16 columns are mostly
+// for; FP64 rows need an even number, so that an odd count takes them in a solve, whose
+// blocks are padded, and the column-major form in a refinement and in the solve that
+// allocates nothing).  From 8 on: below, their tiles of 16 columns are mostly
 // padding.  FP32 on larger systems from 48 on: there the column-major tiles fill the GPU at
 // every level, and 3xTF32 issues three products for each of the (padded) columns.  Solves on
 // B200, column-major / row-major (ms):
@@ -1481,14 +1484,28 @@ int sweep_step(b200_solver_t *s, Lane *ln, double *x, double *aux, int64_t ldx, 
     return ERR_SUCCESS;
 }
 
+// The two blocks of a solve in the lane's workspace, the permuted right-hand sides and the
+// sweeps' scratch, of pitch columns each: even where FP64 rows go to the row-major sweeps,
+// unless the device has no room for the column of padding.
+int solve_blocks(b200_solver_t *s, Lane *ln, int nrhs, int *pitch, double **xp, double **aux) {
+    *pitch = !s->f32 && wide_wanted(s, nrhs) ? (nrhs + 1) / 2 * 2 : nrhs;
+    int rc = ensure_ws(ln, (size_t)2 * s->n * *pitch);
+    if (rc == ERR_OOM && *pitch > nrhs) {
+        *pitch = nrhs;
+        rc = ensure_ws(ln, (size_t)2 * s->n * nrhs);
+    }
+    *xp = ln->d_ws;
+    *aux = ln->d_ws + (size_t)s->n * *pitch;
+    return rc;
+}
+
 // Full solve of device b (original ordering) on the lane of stream st: permute,
-// sweeps, permute back, with the lane's ws[0 : 2 n nrhs] as the permuted block and
-// the sweeps' scratch.
+// sweeps, permute back.
 int solve_device(b200_solver_t *s, Lane *ln, int nrhs, double *b, int64_t ldb, cudaStream_t st) {
     const int n = s->n;
-    const int pitch = !s->f32 && wide_wanted(s, nrhs) ? (nrhs + 1) / 2 * 2 : nrhs;  // even FP64 rows for the row-major sweeps
-    RET(ensure_ws(ln, (size_t)2 * n * pitch));
-    double *xp = ln->d_ws, *aux = ln->d_ws + (size_t)n * pitch;
+    int pitch;
+    double *xp, *aux;
+    RET(solve_blocks(s, ln, nrhs, &pitch, &xp, &aux));
     int launches = 2;
     launch_permute(n, nrhs, s->d_peri, b, ldb, xp, n, 1, st);
     RET(sweeps(s, ln, xp, aux, n, nrhs, st, &launches, nullptr, pitch));
@@ -2522,15 +2539,16 @@ int b200_numfact_trace(b200_solver_t *s, double epsilon_magn_ctrl, double *ms, d
 int b200_solve_trace(b200_solver_t *s, int64_t nrhs, double *ms, double *bytes) {
     if (!s || !s->factored || nrhs <= 0 || !ms) return ERR_BADPARAM;
     const int n = s->n;
-    RET(ensure_ws(&s->main, (size_t)2 * n * nrhs));
-    double *xp = s->main.d_ws, *aux = s->main.d_ws + (size_t)n * nrhs;
+    int pitch;
+    double *xp, *aux;
+    RET(solve_blocks(s, &s->main, (int)nrhs, &pitch, &xp, &aux));
     CU(cudaMemsetAsync(xp, 0, (size_t)n * nrhs * sizeof(double), s->st));
     Trace tr;
     tr.detail = &s->trace_detail;
     int launches = 0;
     tr.begin(s->st);
     tr.end(0, s->st);
-    int rc = sweeps(s, &s->main, xp, aux, n, (int)nrhs, s->st, &launches, &tr);
+    int rc = sweeps(s, &s->main, xp, aux, n, (int)nrhs, s->st, &launches, &tr, pitch);
     if (rc) return rc;
     CU(cudaStreamSynchronize(s->st));
     s->kernel_launches += launches;

@@ -145,3 +145,34 @@ for facto, st in [("potrf", C._structure(7, 6, 5, 27, "potrf")), ("getrf", C._st
     assert got and got[:len(want)] == want
     s.close()
 """)
+
+
+@pytest.mark.parametrize("nrhs", [8, 9])
+def test_solve_without_room_for_padding(run, nrhs):
+    # an odd number of FP64 columns is padded to an even one where that fits
+    run(f"""
+s = solver(2000, "fp64")
+fake.fake_limit(2 * 2000 * {nrhs} * 8)
+s.solve(np.ones((2000, {nrhs}), order="F"))
+""")
+
+
+def test_trace_runs_the_sweeps_of_the_solve(run):
+    # the same launches, one by one: 12-column cblks, whose top of the tree is one launch per
+    # sweep row-major and column-major alike, and 60-column ones
+    run("""
+def counts(s, nrhs):
+    s.solve(np.ones((s.n, nrhs), order="F"))
+    s.solve_trace(nrhs)
+    cls, _ = s.trace_launches()
+    return s.stats()["launches_solve"] - 2, int((cls > 0).sum())  # without the permutations
+
+for width in (5, 12, 60):
+    st = chain_structure([width] * 40, "potrf")
+    s = native.Solver(st, "potrf", "fp64")
+    s.bcsc_load(bcsc_of(sp.diags([np.full(st.n, 4.0)], [0]).tocsc(), "potrf"))
+    s.numfact(0.0)
+    for nrhs in (2, 8, 9, 65):
+        solve, trace = counts(s, nrhs)
+        assert solve == trace, (width, nrhs, solve, trace)
+""")
