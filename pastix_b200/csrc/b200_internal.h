@@ -106,7 +106,7 @@ struct SolveTile {
 // Tile of a many-right-hand-side sweep: 64 outputs from o0 of cblk k, K values [k0, k1)
 // (off-diagonal products: outputs are panel rows and K columns forward, the other way
 // round backward; diagonal products: rows of W_k, or of its transpose).
-constexpr int WIDE_LEAF = 8;  // narrower cblks take the one-warp kernel of those sweeps
+constexpr int WIDE_LEAF = 8;  // cblks of at most so many columns take the one-warp kernel of those sweeps
 struct WideTask {
     int k, o0, k0, k1;
 };
@@ -130,8 +130,8 @@ struct WideFlow {
     int *flist, *need_f, *need_b, *nprev_f, *nprev_b;
 };
 
-// Wide cblk of a panel launch (POTRF / LDL^T cblks wider than the one-CTA diagonal
-// kernel): ns steps of 64 columns, nrb row blocks of 64 rows (the first ns cover the
+// Wide cblk of a panel launch (wider than the one-warp diagonal kernel; LU while its row
+// blocks fit in shared memory): ns steps of 64 columns, nrb row blocks of 64 rows (the first ns cover the
 // diagonal block, the others the rows below it), flag0 its first slot in the
 // per-row-block dependency counters.
 struct PanelCblk {

@@ -121,9 +121,9 @@ void launch_solve_flow(const DevSym &s, const FlowItem *items, int nitems, const
                        int64_t ldx, int nrhs, int backward, int *ticket, int *cnt_a, int *cnt_b, int *abort_word,
                        int *err, cudaStream_t st);
 // sweeps of many right-hand sides on row-major vectors (solve_wide.cu): element (i, j)
-// at i * ldr + j.  Off-diagonal products out -= (atomic), diagonal products out =, both
-// products of the cblks of at most 32 columns, and the moves between column-major
-// blocks and row-major ones
+// at i * ldr + j, ldr a multiple of 16 bytes.  Off-diagonal products out -= (atomic), diagonal
+// products out =, both products of the cblks of at most WIDE_LEAF columns, and the moves
+// between column-major blocks and row-major ones
 template <typename T>
 void launch_wide_off(const DevSym &s, const WideTask *tasks, int ntasks, const T *P, const T *in, T *out, int ldr,
                      int nrhs, int backward, cudaStream_t st);
@@ -139,7 +139,8 @@ void launch_wide_transpose(int n, int nrhs, const S *src, int64_t lds, D *dst, i
 template <typename T>
 void launch_wide_scale(const DevSym &s, const int *cblks, int ncblk, const T *L, T *x, int ldr, int nrhs,
                        cudaStream_t st);
-// one dataflow sweep over the top levels (launch_solve_flow's counters and abort word);
+// one dataflow sweep of at most 64 right-hand sides over the top levels (launch_solve_flow's
+// counters and abort word);
 // the rows it accumulates into are zeroed first
 template <typename T>
 void launch_wide_flow(const DevSym &s, const WideFlow &fw, const T *P, const T *W, const int64_t *woff, T *x, T *aux,

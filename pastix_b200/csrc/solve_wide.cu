@@ -191,7 +191,7 @@ __device__ __forceinline__ void stage_factor(T *ms, const T *Mk, int ldm, int kc
 }
 
 // One tile: 64 outputs of task {k, o0, k0, k1} x the right-hand sides
-// [q0, q0 + 8 NT), q0 = 8 NT blockIdx.y:
+// [q0, q0 + 8 NT), q0 = 8 NT blockIdx.y (rows of the vectors start on 16-byte boundaries):
 //   OFF_FWD  x[row o] -= sum_{k0 <= c < k1} P[o, c] aux[c]     (o panel rows; atomic)
 //   OFF_BWD  aux[o]   -= sum_{k0 <= r < k1} P[r, o] x[row r]   (o columns; atomic)
 //   DIAG_FWD aux[o]    = sum_c W[o, c] x[c]      DIAG_BWD x[o] = sum_r W[r, o] aux[r]
@@ -216,7 +216,6 @@ __global__ void __launch_bounds__(WideSmem<T, MODE, NT>::THREADS) wide_mm_kernel
     const T *Mk = M + (OFF ? s.off[k] : woff[k]);
     const int *prow = OFF ? s.prow + s.rbase[k] : nullptr;
     const bool vec = OFF || n % EPV == 0;  // 16-byte copies of the factor
-    const bool vecx = ldr % EPV == 0;      // and of the vectors
 
     auto load = [&](int st, int kc) {
         T *ms = sm + st * SM::STAGE, *xs = ms + SM::MS;
@@ -224,21 +223,12 @@ __global__ void __launch_bounds__(WideSmem<T, MODE, NT>::THREADS) wide_mm_kernel
         // right-hand sides of the chunk's K values
         auto xrow = [&](int kk) { return in + (size_t)(MODE == W_OFF_BWD ? __ldg(prow + kk) : f0 + kk) * ldr + q0; };
         auto used = [&](int kk) { return kk < t.k1 && (MODE != W_OFF_BWD || kk >= n); };
-        if (vecx) {
-            constexpr int CPL = SM::RW / EPV;
+        constexpr int CPL = SM::RW / EPV;
 #pragma unroll
-            for (int u = 0; u < (WK * CPL + SM::THREADS - 1) / SM::THREADS; u++) {
-                const int idx = tid + SM::THREADS * u, l = idx / CPL, j = (idx % CPL) * EPV;
-                const bool ok = used(kc + l) && j < R;
-                cp_async_n<16>(xs + l * XP + j, ok ? xrow(kc + l) + j : in, ok ? 16 : 0);
-            }
-        } else {
-#pragma unroll 4
-            for (int u = 0; u < WK * SM::RW / SM::THREADS; u++) {
-                const int idx = tid + SM::THREADS * u, l = idx / SM::RW, j = idx % SM::RW;
-                const bool ok = used(kc + l) && j < R;
-                cp_async_n<sizeof(T)>(xs + l * XP + j, ok ? xrow(kc + l) + j : in, ok ? (int)sizeof(T) : 0);
-            }
+        for (int u = 0; u < (WK * CPL + SM::THREADS - 1) / SM::THREADS; u++) {
+            const int idx = tid + SM::THREADS * u, l = idx / CPL, j = (idx % CPL) * EPV;
+            const bool ok = used(kc + l) && j < R;
+            cp_async_n<16>(xs + l * XP + j, ok ? xrow(kc + l) + j : in, ok ? 16 : 0);
         }
     };
 
@@ -370,7 +360,8 @@ __global__ void __launch_bounds__(32 * WL_WARPS) wide_leaf_kernel(DevSym s, cons
 // outputs x 64 K values taken in order from a ticket, each waiting for the counters of its
 // inputs (solve_flow_kernel's, FI_DIAG and FI_OFF items; the cblks have more than WIDE_LEAF
 // columns).  An item's factor tile is on its way before it waits; its vectors, which other
-// items of the launch write, are read through L2.  Outputs accumulate: the rows of aux
+// items of the launch write, are read through L2.  One tile covers all the right-hand sides
+// (8 NT at most).  Outputs accumulate: the rows of aux
 // (forward) and x (backward) of the launch's cblks are zero before it.
 constexpr long long WFLOW_WAIT_CYCLES = 1000000000LL;  // about 0.5 s at the maximum SM clock
 
@@ -413,7 +404,7 @@ __global__ void __launch_bounds__(WideSmem<T, BWD ? W_OFF_BWD : W_OFF_FWD, NT>::
     __shared__ int s_item, s_ok;
     const int *need = BWD ? fw.need_b : fw.need_f, *nprev = BWD ? fw.nprev_b : fw.nprev_f;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const bool vecx = ldr % EPV == 0;
+    const int ntn = (nrhs + 7) >> 3;
     bool aborted = false;
     for (;;) {
         if (tid == 0) {
@@ -458,48 +449,37 @@ __global__ void __launch_bounds__(WideSmem<T, BWD ? W_OFF_BWD : W_OFF_FWD, NT>::
         const bool rows_out = !BWD && !diag;  // outputs are
         const T *in = diag == (BWD != 0) ? aux : x;
         T *out = diag == (BWD != 0) ? x : aux;
-        for (int q0 = 0; q0 < nrhs; q0 += SM::RW) {
-            const int R = min(SM::RW, nrhs - q0), ntn = (R + 7) >> 3;
-            auto xrow = [&](int kk) { return in + (size_t)(rows_in ? __ldg(prow + kk) : f0 + kk) * ldr + q0; };
-            auto used = [&](int kk) { return kk < k1 && (!rows_in || kk >= n); };
-            if (vecx) {
-                constexpr int CPL = SM::RW / EPV;
+        auto xrow = [&](int kk) { return in + (size_t)(rows_in ? __ldg(prow + kk) : f0 + kk) * ldr; };
+        auto used = [&](int kk) { return kk < k1 && (!rows_in || kk >= n); };
+        constexpr int CPL = SM::RW / EPV;
 #pragma unroll
-                for (int u = 0; u < 2 * WK * CPL / SM::THREADS; u++) {
-                    const int idx = tid + SM::THREADS * u, l = idx / CPL, j = (idx % CPL) * EPV;
-                    const bool ok = used(k0 + l) && j < R;
-                    cp_async_n<16>(xs + l * XP + j, ok ? xrow(k0 + l) + j : in, ok ? 16 : 0);
-                }
-            } else {
-#pragma unroll 4
-                for (int u = 0; u < 2 * WK * SM::RW / SM::THREADS; u++) {
-                    const int idx = tid + SM::THREADS * u, l = idx / SM::RW, j = idx % SM::RW;
-                    xs[l * XP + j] = used(k0 + l) && j < R ? __ldcg(xrow(k0 + l) + j) : (T)0;
-                }
-            }
-            cp_commit_g();
-            cp_wait_g<0>();
-            __syncthreads();
-            WideTile<T, MODE, NT> tile;
-            tile.mul(ms, xs, o1 - o0, ntn);
-            if (k0 + WK < k1) tile.mul(ms + SM::MS, xs + WK * XP, o1 - o0, ntn);
-            __syncthreads();
-            tile.out(os);
-            __syncthreads();
-            constexpr int CG = SM::RW < 32 ? SM::RW : 32, RG = 32 / CG;
-#pragma unroll 4
-            for (int i = warp * RG + lane / CG; i < o1 - o0; i += SM::THREADS / 32 * RG) {
-                const int o = o0 + i;
-                if (rows_out && o < n) continue;
-                T *row = out + (size_t)(rows_out ? __ldg(prow + o) : f0 + o) * ldr + q0;
-#pragma unroll
-                for (int j0 = 0; j0 < SM::RW; j0 += CG) {
-                    const int j = j0 + lane % CG;
-                    if (j < R) atomicAdd(row + j, diag ? os[i * SM::OP + j] : -os[i * SM::OP + j]);
-                }
-            }
-            __syncthreads();
+        for (int u = 0; u < 2 * WK * CPL / SM::THREADS; u++) {
+            const int idx = tid + SM::THREADS * u, l = idx / CPL, j = (idx % CPL) * EPV;
+            const bool ok = used(k0 + l) && j < nrhs;
+            cp_async_n<16>(xs + l * XP + j, ok ? xrow(k0 + l) + j : in, ok ? 16 : 0);
         }
+        cp_commit_g();
+        cp_wait_g<0>();
+        __syncthreads();
+        WideTile<T, MODE, NT> tile;
+        tile.mul(ms, xs, o1 - o0, ntn);
+        if (k0 + WK < k1) tile.mul(ms + SM::MS, xs + WK * XP, o1 - o0, ntn);
+        __syncthreads();
+        tile.out(os);
+        __syncthreads();
+        constexpr int CG = SM::RW < 32 ? SM::RW : 32, RG = 32 / CG;
+#pragma unroll 4
+        for (int i = warp * RG + lane / CG; i < o1 - o0; i += SM::THREADS / 32 * RG) {
+            const int o = o0 + i;
+            if (rows_out && o < n) continue;
+            T *row = out + (size_t)(rows_out ? __ldg(prow + o) : f0 + o) * ldr;
+#pragma unroll
+            for (int j0 = 0; j0 < SM::RW; j0 += CG) {
+                const int j = j0 + lane % CG;
+                if (j < nrhs) atomicAdd(row + j, diag ? os[i * SM::OP + j] : -os[i * SM::OP + j]);
+            }
+        }
+        __syncthreads();
         if (tid == 0) {
             __threadfence();
             if (diag) {
