@@ -2,8 +2,12 @@
 top of the tree up to 64 of them): every width class of the tiles (16, 32, 48, 64 columns),
 odd and ragged numbers, cblks from 1 to 200 columns, against x_true (FP64) and the same
 factor's solutions one at a time (FP32).  Analysis of perf/cases.py, no PaStiX library."""
+import ctypes
+import time
+
 import numpy as np
 import pytest
+import torch
 
 import oracle
 from pastix_b200 import native
@@ -86,3 +90,66 @@ def test_fp32_many_as_accurate_as_few(facto, points, dims, shift, low):
     for nrhs in (8, 16, 17, 40, 64):
         assert error(nrhs) <= 1.1 * few, nrhs
     s.close()
+
+
+def test_withheld_item_ends_the_dataflow_sweep(monkeypatch):
+    # the top of the tree in one launch up to 64 columns (fewer launches than level by level,
+    # from 65 on); its first item withheld: bounded waits, an error status, and the instance
+    # solves again
+    st, s = factored("potrf", 7, (20, 20, 20), 0.0, "fp64")
+    xt = np.random.default_rng(9).uniform(-1.0, 1.0, (st.n, 66))
+    b = s.spmv(xt)
+    s.solve(b)
+    level_by_level = s.stats()["launches_solve"]
+    for nrhs in (8, 17, 33, 64):
+        x = s.solve(b[:, :nrhs])
+        assert s.stats()["launches_solve"] < level_by_level
+        monkeypatch.setenv("B200_TEST_WITHHOLD", "flow")
+        t = time.perf_counter()
+        with pytest.raises(native.B200Error):
+            s.solve(b[:, :nrhs])
+        assert time.perf_counter() - t < 20.0
+        monkeypatch.delenv("B200_TEST_WITHHOLD")
+        assert np.linalg.norm(s.solve(b[:, :nrhs]) - x) <= 1e-13 * np.linalg.norm(x)
+    s.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("nrhs", [8, 9])
+def test_solve_that_allocates_nothing(prec, nrhs):
+    st, s = factored("sytrf", 7, (13, 12, 17), 0.05, prec)
+    b = np.asfortranarray(np.random.default_rng(10).uniform(-1.0, 1.0, (st.n, nrhs)))
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        d = torch.from_numpy(b.T.copy()).cuda()
+        assert native.lib().b200_solve_device_noalloc(s.h, nrhs, ctypes.c_void_p(d.data_ptr()), st.n,
+                                                      ctypes.c_void_p(stream.cuda_stream)) == 0
+    stream.synchronize()
+    x = s.solve(b)
+    assert np.linalg.norm(d.cpu().numpy().T - x) <= (1e-12 if prec == "fp64" else 1e-5) * np.linalg.norm(x)
+    s.close()
+
+
+@pytest.mark.parametrize("nrhs", [8, 9])
+@pytest.mark.parametrize("facto,shift,method", [("potrf", 0.0, "cg"), ("sytrf", -0.05, "gmres")])
+def test_refinement_with_an_fp64_factor(facto, shift, method, nrhs):
+    # an even number of columns takes the row-major sweeps, an odd one does not
+    st, s = factored(facto, 7, (17, 16, 15), shift, "fp64")
+    xt = np.random.default_rng(11).uniform(-1.0, 1.0, (st.n, nrhs))
+    b = s.spmv(xt)
+    x, nit, berr = s.refine(b, np.zeros_like(b), method, eps=1e-13)
+    assert berr.max() <= 1e-13 and nit <= 3
+    assert np.linalg.norm(x - xt) <= 1e-10 * np.linalg.norm(xt)
+    s.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_batch_of_systems(prec):
+    case = dict(kind="step", facto="sytrf", points=5, nx=16, ny=40, nz=12, prec=prec, nrhs=9, shift=-0.02)
+    S = C.prepare(case, 5)
+    x = C.run(S)
+    torch.cuda.synchronize()
+    xt = C.exact(case, 5)
+    tol = C.tolerance(case)["rel"]
+    assert torch.linalg.norm(x - xt) <= tol * torch.linalg.norm(xt)
+    S["s"].close()
