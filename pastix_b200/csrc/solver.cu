@@ -120,6 +120,9 @@ struct b200_solver_s {
     WideFlow wflow{};                   // the levels from wflow_level up, one launch per sweep
     int wflow_level = 0;
     int *d_leaf = nullptr;              // cblks of <= 32 columns, solved by the one-warp kernel
+    // chain of that kernel over the levels below the dataflow sweeps: columns x (1 + 32-row
+    // groups below) of each level's longest
+    int64_t leaf_chain = 0;
     std::vector<int> lvl_lf0, lvl_lf1;
     // inverses of the diagonal blocks: W_L (forward sweep) and, for LU, W_U (backward)
     int64_t *d_woff = nullptr;
@@ -897,6 +900,15 @@ int build_schedule(b200_solver_t *s) {
                 s->flow_level = l;
                 break;
             }
+        s->leaf_chain = 0;
+        for (int l = 0; l < s->flow_level; l++) {
+            int longest = 0;
+            for (int p = s->lvl_lf0[l]; p < s->lvl_lf1[l]; p++) {
+                const int nc = s->ncols[leaf[p]];
+                longest = std::max(longest, nc * (1 + (s->stride[leaf[p]] - nc + 31) / 32));
+            }
+            s->leaf_chain += longest;
+        }
         for (int l = s->flow_level; l < nlev; l++) {
             const Level &L = s->levels[l];
             for (int p = s->lvl_lf0[l]; p < s->lvl_lf1[l]; p += 16) {
@@ -1419,20 +1431,27 @@ int enqueue_wide_sweeps(b200_solver_t *s, Lane *ln, double *x, double *aux, int 
 // Many right-hand sides take the row-major sweeps (pitch: columns that both blocks have room
 // for; FP64 rows need an even number, so that an odd count takes them in a solve, whose
 // blocks are padded, and the column-major form in a refinement and in the solve that
-// allocates nothing).  From 8 on: below, their tiles of 16 columns are mostly
-// padding.  FP32 on larger systems from 48 on: there the column-major tiles fill the GPU at
-// every level, and 3xTF32 issues three products for each of the (padded) columns.  Solves on
-// B200, column-major / row-major (ms):
-//   FP64  12^3  8: 0.32 / 0.25, 33: 0.75 / 0.33;  80^3  8: 4.33 / 3.65, 17: 5.93 / 5.06, 40:
-//         8.76 / 7.55;  100^3  256: 89.2 / 58.0
-//   FP32  24^3  8: 0.45 / 0.35, 48: 1.03 / 0.53;  44^3  8: 0.76 / 0.75, 17: 1.13 / 1.01;  52^3
-//         27-point  8: 1.46 / 1.15, 33: 2.93 / 2.07
-//         60^3  8: 1.29 / 1.45, 17: 1.91 / 2.10, 40: 2.76 / 2.74;  90^3  17: 5.98 / 6.51, 40:
-//         8.80 / 8.92, 48: 9.58 / 9.45;  100^3  64: 18.1 / 15.5
-constexpr int WIDE_MIN_NRHS = 8, WIDE_MIN_NRHS_F32 = 48, WIDE_SMALL_N = 180000;
+// allocates nothing).  FP64 from 8 on: below, their tiles of 16 columns are mostly padding.
+//
+// FP32 (3xTF32, three products for each of the padded columns) by what the column-major form
+// loses: on the levels below its dataflow launch, one warp walks a narrow cblk's rows for 16
+// columns at a time, and the level lasts as long as its longest (leaf_chain).  Where those
+// chains are short for the size of the system the column-major tiles are faster up to 24 or,
+// on larger systems, 48 columns.  The time of the row-major form over the column-major one on
+// B200 at 8, 17 and 33 columns:
+//   FP64        8^3 0.86, 0.64, 0.51;  56^3 0.92, 0.95, 0.89;  62^3 0.93, 0.97, 0.93;  80^3
+//               0.84, 0.84, 0.87;  300^2 1.00, 0.87, 0.76
+//   FP32 above the line   8^3 0.84, 0.65, 0.55;  24^3 0.77, 0.66, 0.56;  40^3 1.01, 0.99, 0.88;
+//               50^3 LU 0.80, 0.81, 0.77;  54^3 0.91, 0.90, 0.86;  64^3 LU 0.99, 1.03, 0.99;  68^3
+//               LDL^T 0.96, 0.99, 0.95;  100^3 0.94, 0.98, 1.00
+//   FP32 below it   28^3 1.17, 1.10, 0.96;  300^2 1.14, 0.97, 0.86;  56^3 1.10, 1.09, 1.05;  62^3
+//               LDL^T 1.11, 1.14, 1.06;  80^3 1.00, 1.06, 1.03;  90^3 0.99, 1.04, 1.04
+//   from 48 columns on    56^3 1.00;  62^3 1.06;  64^3 LU 0.94;  80^3 0.98;  100^3 0.94
+constexpr int WIDE_MIN_NRHS = 8;
 
 inline bool wide_wanted(const b200_solver_t *s, int nrhs) {
-    return nrhs >= (s->f32 && s->n > WIDE_SMALL_N ? WIDE_MIN_NRHS_F32 : WIDE_MIN_NRHS);
+    if (!s->f32 || nrhs < WIDE_MIN_NRHS) return nrhs >= WIDE_MIN_NRHS;
+    return nrhs >= 48 || (nrhs > 24 && s->n <= 160000) || s->n <= 10000 || s->leaf_chain >= 290 + s->n / 3000;
 }
 
 int sweeps(b200_solver_t *s, Lane *ln, double *x, double *aux, int64_t ldx, int nrhs, cudaStream_t st,

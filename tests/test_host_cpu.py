@@ -176,3 +176,27 @@ for width in (5, 12, 60):
         solve, trace = counts(s, nrhs)
         assert solve == trace, (width, nrhs, solve, trace)
 """)
+
+
+def test_rule_of_the_row_major_sweeps(run):
+    # the sweeps' launches at 7 columns are column-major; FP32 grids on both sides of the line
+    run("""
+from perf import cases as C
+
+def row_major(dims, facto, prec, nrhs):
+    s = native.Solver(C._structure(*dims, 7, facto), facto, prec)
+    s.bcsc_load(bcsc_of(sp.diags([np.full(s.n, 4.0)], [0]).tocsc(), facto))
+    s.numfact(0.0)
+    def launches(k):
+        s.solve_trace(k)
+        return len(s.trace_launches()[0])
+    return launches(nrhs) != launches(7)
+
+for dims, facto, counts in [((9, 9, 9), "potrf", {8: 1, 17: 1}), ((24, 24, 24), "potrf", {8: 1, 17: 1}),
+                            ((28, 28, 28), "potrf", {8: 0, 24: 0, 25: 1, 48: 1}),
+                            ((32, 32, 32), "getrf", {8: 1, 17: 1}), ((58, 58, 58), "potrf", {8: 0, 33: 0, 48: 1}),
+                            ((300, 300, 1), "potrf", {8: 0, 24: 0, 33: 1})]:
+    for nrhs, want in counts.items():
+        assert row_major(dims, facto, "fp32", nrhs) == bool(want), (dims, nrhs)
+    assert row_major(dims, facto, "fp64", 8), dims
+""")
