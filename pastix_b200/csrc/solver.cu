@@ -2641,9 +2641,10 @@ int b200_solve_device_noalloc(b200_solver_t *s, int64_t nrhs, double *d_b, int64
     // stream (allocated with the instance; a stream's own lane would be allocated here)
     Lane *ln = &s->main;
     CU(cudaMemsetAsync(ln->d_serr, 0, sizeof(int), st));
-    // every entry of the scratch used here is written before it is read: the first half
-    // by the permutation, the second by the forward diagonal products (for an FP32
-    // factor, the two float blocks of the sweeps by the conversion and the products)
+    // every entry of the scratch that a result depends on is written before it is read: the
+    // first half by the permutation, the second by the forward diagonal products (for an FP32
+    // factor, the two float blocks of the sweeps by the conversion and the products; the
+    // padding columns of their row-major form are read, but not what comes of them)
     int launches = 2;
     launch_permute(n, (int)nrhs, s->d_peri, d_b, ldb, xp, n, 1, st);
     RET(sweeps(s, ln, xp, aux, n, (int)nrhs, st, &launches));

@@ -42,8 +42,9 @@ def dominant(n, facto, seed):
     return A + np.diag(np.full(n, 1.2 * np.sqrt(n)))
 
 
-def backward_error(A, widths, facto, prec):
-    """|A - L U| over |L| |U| (Frobenius), and the solver, whose matrix A rounded to prec is."""
+def backward_error(A, widths, facto, prec, solves=None):
+    """|A - L U| over |L| |U| (Frobenius) of A rounded to prec; solves: list that receives the
+    relative residuals of solutions with 1, 5 and 9 right-hand sides."""
     if prec == "fp32":
         A = A.astype(np.float32).astype(np.float64)
     st = dense_structure(widths, facto)
@@ -51,6 +52,12 @@ def backward_error(A, widths, facto, prec):
     s.bcsc_load(bcsc_of(sp.csc_matrix(A), facto))
     s.numfact(1e-20)
     Lc, Uc = s.factor()
+    if solves is not None:
+        r = np.random.default_rng(7)
+        for nrhs in (1, 5, 9):  # the inverses of the diagonal blocks, through each form of the sweeps
+            xt = r.uniform(-1, 1, (st.n, nrhs))
+            x = s.solve(np.asfortranarray(A @ xt))
+            solves.append(np.linalg.norm(A @ (x - xt)) / (np.linalg.norm(A, 2) * np.linalg.norm(xt)))
     s.close()
     M = dense_factor(st, Lc)
     if facto == "potrf":
@@ -73,7 +80,11 @@ def test_widths(facto, prec, widths):
     A = spd(n, 1e2, 3) if facto == "potrf" else dominant(n, facto, 3)
     # an entry of L U is off by at most n u of its |L| |U|; random roundings of sums cut at 64
     # terms stay near u, wherever the cuts lie
-    assert backward_error(A, widths, facto, prec) <= 4 * UNIT[prec]
+    solves = []
+    assert backward_error(A, widths, facto, prec, solves) <= 4 * UNIT[prec]
+    # each sweep adds the rounding of its products, with the inverses up to their condition
+    # number (10 and less) times that, to the factor's
+    assert max(solves) <= 40 * UNIT[prec]
 
 
 # the same ratio, mean of six matrices, of substitution with sums cut at 32 columns (measured)
